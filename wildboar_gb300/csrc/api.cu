@@ -127,11 +127,14 @@ Workspace::Workspace(cudaStream_t stream)
 
 Workspace::~Workspace() { arena_->used = 0; }
 
-int Workspace::reserve(size_t bytes) {
+int Workspace::reserve(size_t bytes, size_t least) {
     if (injected(INJ_RESERVE))
         return fail(WB_ENOMEM, "cannot allocate device workspace (injected fault)");
     bytes = align256(bytes) + 4096;
-    if (bytes > arena_->cap) {
+    least = align256(least) + 4096;
+    // (a size that the device had no room for is not asked for again while the
+    // arena holds what the call needs)
+    if (bytes > arena_->cap && !(least <= arena_->cap && bytes >= arena_->denied)) {
         if (arena_->base) {
             // cudaFree waits for the device, so earlier work on this stream
             // that still reads the arena has finished
@@ -140,8 +143,14 @@ int Workspace::reserve(size_t bytes) {
             arena_->cap = 0;
             if (e != cudaSuccess) return cuda_fail(e, "cudaFree(workspace)");
         }
-        size_t cap = bytes + bytes / 4;
+        size_t cap = bytes + std::min(bytes / 4, (size_t)256 << 20);
         cudaError_t e = cudaMalloc((void **)&arena_->base, cap);
+        while (e == cudaErrorMemoryAllocation && cap > least) {
+            cudaGetLastError();
+            arena_->denied = std::min(arena_->denied, cap);
+            cap = std::max(cap / 2, least);
+            e = cudaMalloc((void **)&arena_->base, cap);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             arena_->base = nullptr;
@@ -444,7 +453,7 @@ extern "C" int wb_pairwise_distance(const wb_series *x, const wb_series *y, int6
         probe.cols.len -= 2;
     }
     need += elastic_workspace_bytes(probe);
-    WB_TRY(ws.reserve(need));
+    WB_TRY(ws.reserve(need + guided_workspace_bytes(probe), need));
 
     WB_TRY(stage(x, dim, ws, J.rows));
     if (same) J.cols = J.rows;
@@ -458,7 +467,7 @@ extern "C" int wb_pairwise_distance(const wb_series *x, const wb_series *y, int6
     if (same) {
         WB_CUDA(cudaMemsetAsync(dout, 0, out_elems * sizeof(double), s));
     }
-    WB_TRY(launch_elastic(J, ws, nullptr));
+    WB_TRY(launch_elastic(J, ws, true));
     return finish_host_copy(out, dout, out_elems * sizeof(double), out_on_device, s);
 }
 
@@ -576,7 +585,7 @@ extern "C" int wb_pairwise_distance_fp32(const wb_series *x, const wb_series *y,
         J.out_ld = yy->n;
         J.mode = same ? PM_UPPER : PM_ALL;
         if (same) WB_CUDA(cudaMemsetAsync(dout, 0, out_elems * sizeof(double), s));
-        if (all_zero) WB_TRY(launch_elastic(J, ws, nullptr));
+        if (all_zero) WB_TRY(launch_elastic(J, ws));
         else WB_TRY(launch_strip(J, ws, true));
     }
     return finish_host_copy(out, dout, out_elems * sizeof(double), out_on_device, s);
@@ -618,7 +627,7 @@ extern "C" int wb_paired_distance(const wb_series *x, const wb_series *y, int64_
                   table_bytes(metric, params, probeR, probeC, y->n, x->n, rl, cl) +
                   elastic_workspace_bytes(probe) +
                   (out_on_device ? 0 : align256((size_t)x->n * 8));
-    WB_TRY(ws.reserve(need));
+    WB_TRY(ws.reserve(need + guided_workspace_bytes(probe), need));
     WB_TRY(stage(y, dim, ws, J.rows));
     WB_TRY(stage(x, dim, ws, J.cols));
     WB_TRY(build_tables(metric, params, J, ws, false, rl, cl));
@@ -627,7 +636,7 @@ extern "C" int wb_paired_distance(const wb_series *x, const wb_series *y, int64_
     J.out = dout;
     J.out_ld = 0;
     J.mode = PM_PAIRED;
-    WB_TRY(launch_elastic(J, ws, nullptr));
+    WB_TRY(launch_elastic(J, ws, true));
     return finish_host_copy(out, dout, (size_t)x->n * sizeof(double), out_on_device, s);
 }
 
@@ -730,7 +739,7 @@ extern "C" int wb_argmin_distance(const wb_series *x, const wb_series *y, int64_
         Jb.out_ld = y->n;
         Jb.key = metric == WB_EUCLIDEAN ? nullptr : K;
         Jb.mode = PM_ALL;
-        if (!never_push && !use_ea) WB_TRY(launch_elastic(Jb, ws, nullptr));
+        if (!never_push && !use_ea) WB_TRY(launch_elastic(Jb, ws));
 
         const double *lb = lower_bound ? lower_bound + (size_t)b0 * y->n : nullptr;
         if (lower_bound && !out_on_device) {
@@ -1370,7 +1379,7 @@ extern "C" int wb_dilated_profile(const wb_series *y, const wb_series *x, int64_
         J.out = dist;
         J.out_ld = 0;
         J.mode = PM_PAIRED;
-        WB_TRY(launch_elastic(J, ws, nullptr));
+        WB_TRY(launch_elastic(J, ws));
         WB_TRY(launch_dilated_scatter(dist, n, p, np, k, L, dout, out_size, s));
         p = q;
     }

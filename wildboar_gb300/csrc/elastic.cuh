@@ -67,6 +67,9 @@ struct ElasticJob {
     int64_t out_ld = 0;                 // row stride of out (PM_ALL / PM_UPPER)
     double *key = nullptr;              // early-abandon keys (argmin), or null
     int all_zero = 0;                   // ddtw on series shorter than 3
+    // second pass of a guided evaluation (guided.cu): only the pairs whose
+    // output is kGuidedPending, *pending of them
+    const unsigned long long *pending = nullptr;
 };
 
 // Ring length (in elements) needed for a band recurrence of an (n x m)
@@ -77,7 +80,9 @@ inline int ring_len(int n, int m, int r) {
     return (int)(w < full ? w : full);
 }
 
-int launch_elastic(const ElasticJob &job, Workspace &ws, size_t *ring_bytes_query);
+// Runs the job; `guided` allows the guided evaluation (guided.cu) on what the
+// call's reservation has beyond its other needs.
+int launch_elastic(const ElasticJob &job, Workspace &ws, bool guided = false);
 // Same kernels with the per-thread rings in a caller-provided device buffer of
 // `ring_bytes` (always the global-ring variant); the grid is the largest that
 // fits.  WB_EINVAL when not even one block's rings fit.
@@ -86,7 +91,9 @@ int launch_elastic_external_ring(const ElasticJob &job, double *ring, size_t rin
 // The shared-memory ring kernels (and the tiled euclidean kernel) without any
 // workspace; WB_EUNSUPPORTED when the band ring does not fit in shared memory.
 int launch_elastic_shared_ring(const ElasticJob &job, cudaStream_t s);
+// Workspace launch_elastic needs, and what the guided evaluation adds (0: not used).
 size_t elastic_workspace_bytes(const ElasticJob &job);
+size_t guided_workspace_bytes(const ElasticJob &job);
 
 // elastic subsequence distance (one warp per (series, shapelet), one lane per
 // window); rows are the shapelet (or its slopes), columns the window.

@@ -23,6 +23,7 @@
 // two rows up (stale buffer content); the ring reproduces that value.
 
 #include "elastic_rec.cuh"
+#include "guided.cuh"
 
 namespace wb {
 
@@ -86,10 +87,12 @@ elastic_pairs_kernel(const ElasticJob J, double *gring, int P) {
     const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
     const int64_t gtid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t gthreads = (int64_t)gridDim.x * kThreads;
+    if (J.pending && *J.pending == 0) return;
 
     auto body = [&](auto ring) {
         if (J.mode == PM_PAIRED) {
             for (int64_t s = gtid; s < J.rows.count; s += gthreads) {
+                if (J.pending && !is_pending(J.out[s])) continue;
                 double key, d;
                 d = J.all_zero ? 0.0 : finish(J, run_pair<KIND>(J, ring, P, s, s, key));
                 J.out[s] = d;
@@ -106,6 +109,7 @@ elastic_pairs_kernel(const ElasticJob J, double *gring, int P) {
             } else if (rs >= J.rows.count) {
                 continue;
             }
+            if (J.pending && !is_pending(J.out[rs * J.out_ld + cs])) continue;
             double key = 0.0, d;
             if (J.all_zero) d = 0.0;
             else d = finish(J, run_pair<KIND>(J, ring, P, rs, cs, key));
@@ -287,8 +291,16 @@ static int launch_euclid_tiled(const ElasticJob &J, cudaStream_t s) {
     return WB_OK;
 }
 
-int launch_elastic(const ElasticJob &J, Workspace &ws, size_t *) {
+int launch_elastic(const ElasticJob &job, Workspace &ws, bool guided) {
+    ElasticJob J = job;
     if (J.rows.count == 0 || J.cols.count == 0) return WB_OK;
+    if (guided) {
+        // then the full recurrence over the pairs it left, in the workspace
+        // that it leaves
+        unsigned long long *pending = nullptr;
+        WB_TRY(launch_guided(J, ws, elastic_workspace_bytes(J), &pending));
+        J.pending = pending;
+    }
     if (use_strip_f64(J)) return launch_strip(J, ws, false);
     ElasticPlan pl = plan_elastic(J);
     double *gring = pl.gring ? ws.take<double>(pl.gring_bytes / sizeof(double)) : nullptr;
