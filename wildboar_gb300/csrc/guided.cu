@@ -8,10 +8,11 @@
 // monotone: only the cells of a best path matter, and any other cell may be
 // dropped (read as +inf) without changing a bit.  Per pair, one thread
 //
-//  1. sweeps the band in 32-bit fixed point (float32 costs rounded to units,
-//     exact integer sums; strips of S rows in registers, 4 columns per step)
-//     and keeps the bottom row of every strip and the cells of every S-th
-//     column;
+//  1. sweeps the band in 32-bit fixed point (exact integer sums; strips of S
+//     rows in registers, 4 columns per step) and keeps the bottom row of every
+//     strip and the cells of every S-th column (one byte per cell for S = 8,
+//     which the DRAM writes bound at about 8 ms for the shape below; S = 16
+//     halves it where S = 8 would not fit the budget);
 //  2. walks back from (n-1, m-1) over the S x S blocks between those kept rows
 //     and columns: a block's cells are recomputed from them, every predecessor
 //     whose value lies within the error bound of the cell's smallest
@@ -27,13 +28,19 @@
 // distance and lies on no best path.  Sums are exact; in float32 each of the
 // n + m additions would add an error relative to the whole sum, which at
 // length 512 keeps 1340 cells per pair instead of 835 (and 3 times as many
-// steps for a warp, which waits for its widest pair).
+// steps for a warp, which waits for its widest pair).  A cost is the high half
+// of the square of a 31-bit difference (three instructions per cell: subtract,
+// 3-input minimum, multiply-add); where the largest difference of a pair is
+// far above its distance, and for wdtw, the warp takes float32 costs rounded to
+// units instead (the conversion issues at 16 per clock and SM and takes most
+// of that sweep's time).
 //
-// Error bound.  With d = x - y of the centred, scaled float inputs, the sum of
-// a path of at most K = n + m - 1 cells differs from its exact sum on the
-// float inputs by K / 2 units and a few 2^-24 of it.  The float inputs move
-// the 2-norm of a path's differences by at most e sqrt(K) with
-// e = 2^-24 (max|x| + max|y|).  Hence for the best predecessor p of a cell on
+// Error bound.  With d = x - y of the centred, scaled, rounded inputs, the sum
+// of a path of at most K = n + m - 1 cells differs from its exact sum on these
+// inputs by K / 2 units and a few 2^-24 of it (float costs) or lies at most K
+// units below it (fixed point).  Rounding the inputs moves the 2-norm of a
+// path's differences by at most e sqrt(K), e = 2^-24 (max|x| + max|y|) for
+// float and two roundings of the shifted values for fixed-point inputs.  Hence for the best predecessor p of a cell on
 // a best path and any other predecessor q,
 //   A(p) <= A(q) + K + 16 2^-24 A_max + 4 e sqrt(K) sqrt(A_max) + 4 e^2 K,
 // A the swept values, A_max a bound of A along the path from its value at
@@ -45,6 +52,12 @@
 // band's blocks: long runs of equal values tie everywhere) or whose inputs
 // are not finite are left to the full recurrence: their output holds
 // kGuidedPending until launch_elastic's second pass over exactly those pairs.
+//
+// Measured on one GB300 (full recurrence -> guided): dtw r = 0.1, 1000 x 1000,
+// length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 8.6
+// ms; wdtw r = 1, 500 x 403, length 256: 107 -> 9.5 ms.  Of the first, the
+// sweep takes a fourth, the walk a fifth and the FP64 part half (its iterations
+// wait for the widest of 32 pairs).
 
 #include "guided.cuh"
 
@@ -57,6 +70,7 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr unsigned kCap = 1u << 30;  // saturated value, and out of band
+constexpr int kFixOne = (1 << 29) - 1;  // 1.0 in fixed point
 #define WB_GINF __int_as_float(0x7f800000)
 #define WB_GINF64 __longlong_as_double(0x7ff0000000000000LL)
 
@@ -123,13 +137,16 @@ __device__ __forceinline__ bool centre_scale(const GuidedPrep *prep, double &cen
     return true;
 }
 
-// Float copies of the centred, scaled series (one warp per series), padded so
-// that every cell past a series' end costs +inf, and their largest magnitude.
-// Row series start at element 3, which puts row 1 + S s on a 16-byte boundary.
+// Float and 30-bit fixed-point copies of the centred, scaled series (one warp
+// per series) with their extremes.  Row series start at element 3, which puts
+// row 1 + S s on a 16-byte boundary.  Past a series' end the float copies cost
+// +inf; the fixed-point ones hold 0 (cells there precede no cell of the
+// pair).
 __global__ void __launch_bounds__(256)
 guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, int64_t cs,
-                      const GuidedPrep *prep, float *xf, float *yf, float *xmax, float *ymax,
-                      const double *weights, int nw, float *wext, int woff, int wlen) {
+                      const GuidedPrep *prep, float *xf, float *yf, int *xq, int *yq,
+                      GuidedRange *xr, GuidedRange *yr, const double *weights, int nw,
+                      float *wext, int woff, int wlen) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
     const int64_t nwarp = ((int64_t)gridDim.x * 256) >> 5;
@@ -141,21 +158,31 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, in
         const SeriesSet &S = row ? rows : cols;
         const double *src = S.base + s * S.stride;
         float *dst = row ? xf + s * rs : yf + s * cs;
+        int *dsq = row ? xq + s * rs : yq + s * cs;
         const int lead = row ? 3 : 0;
         const int total = (int)(row ? rs : cs);
         const float pad = row ? WB_GINF : -WB_GINF;
         float mx = 0.0f;
+        int lo = kFixOne, hi = -kFixOne;
         for (int i = lane; i < total; i += 32) {
             const int e = i - lead;
             float v = pad;
+            int q = 0;
             if (e >= 0 && e < S.len) {
-                v = (float)((src[e] - centre) * scale);
+                const double c = (src[e] - centre) * scale;
+                v = (float)c;
+                q = __double2int_rn(c * (double)kFixOne);
                 mx = fmaxf(mx, fabsf(v));
+                lo = imin(lo, q);
+                hi = imax(hi, q);
             }
             dst[i] = v;
+            dsq[i] = q;
         }
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) (row ? xmax : ymax)[s] = mx;
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) (row ? xr : yr)[s] = GuidedRange{lo, hi, mx};
     }
     // weights by |i - j|, for i - j of either sign
     if (wext)
@@ -191,12 +218,29 @@ __device__ __forceinline__ unsigned best_of(unsigned dg, unsigned up, unsigned l
     else return __vimin3_u32(dg, up, lf);
 }
 
-// best + cost in units, saturating (the conversion saturates at 2^31 - 1)
+// best + cost in units, saturating, from a float square (the conversion
+// saturates at 2^31 - 1)
 template <int KIND>
 __device__ __forceinline__ unsigned add_cost(float sq, float w, unsigned best) {
     if constexpr (KIND == K_WDTW) sq = __fmul_rn(sq, w);
     return __viaddmin_u32(best, (unsigned)__float2int_rn(sq), kCap);
 }
+
+// best + d^2 / 2^32 (rounded down), not saturating
+__device__ __forceinline__ unsigned add_square(int d, unsigned best) {
+    unsigned r;
+    asm("mad.hi.s32 %0, %1, %1, %2;" : "=r"(r) : "r"(d), "r"(best));
+    return r;
+}
+
+// A signed power of two as a left and a right shift (one of them 0), so that
+// applying it takes two instructions and no choice.
+struct Shift {
+    int left, right;
+    __device__ __forceinline__ int of(int x) const {
+        return (int)((unsigned)x << left) >> right;
+    }
+};
 
 // bits k (k < 32) with 0 <= e - k < width: strip rows in band at a column,
 // e = c - i0 - lo
@@ -223,25 +267,62 @@ struct Band {
     }
 };
 
+// The S rows of a strip or block: scaled float pairs, or fixed point.
+template <int S, bool FIX>
+struct StripRows {
+    uint64_t x2[S / 2];
+    __device__ __forceinline__ void load(const GuidedArgs &, const float *xr, const int *,
+                                         float su, Shift) {
+        const float4 *x4 = reinterpret_cast<const float4 *>(xr);
+#pragma unroll
+        for (int k = 0; k < S / 4; k++) {
+            const float4 t = x4[k];
+            x2[2 * k] = pack2(__fmul_rn(t.x, su), __fmul_rn(t.y, su));
+            x2[2 * k + 1] = pack2(__fmul_rn(t.z, su), __fmul_rn(t.w, su));
+        }
+    }
+};
+template <int S>
+struct StripRows<S, true> {
+    int x[S];
+    __device__ __forceinline__ void load(const GuidedArgs &, const float *, const int *xq,
+                                         float, Shift sh) {
+        const int4 *x4 = reinterpret_cast<const int4 *>(xq);
+#pragma unroll
+        for (int k = 0; k < S / 4; k++) {
+            const int4 t = x4[k];
+            x[4 * k] = sh.of(t.x);
+            x[4 * k + 1] = sh.of(t.y);
+            x[4 * k + 2] = sh.of(t.z);
+            x[4 * k + 3] = sh.of(t.w);
+        }
+    }
+};
+
 // One column of a strip: Pin holds column c - 1, Pout receives column c;
-// wq[S - 1 - k] is the weight of row k.
-template <int KIND, int S, bool MASK>
+// wq[S - 1 - k] is the weight of row k.  Fixed-point values saturate only at
+// the end of a group of 4 columns: with squares of at most 2^28 (S = 8), or
+// squares and penalties of at most 2^26, the S + 3 cells of a path through a
+// group stay below 2^32.
+template <int KIND, int S, bool FIX, bool MASK>
 __device__ __forceinline__ void sweep_column(const unsigned (&Pin)[S], unsigned (&Pout)[S],
                                              unsigned bup, unsigned bdiag,
-                                             const uint64_t (&x2)[S / 2], float y,
+                                             const StripRows<S, FIX> &R, unsigned ybits,
                                              const float *wq, unsigned pen, unsigned M) {
-    const uint64_t yy = pack2(y, y);
+    const uint64_t yy = FIX ? 0 : pack2(__uint_as_float(ybits), __uint_as_float(ybits));
 #pragma unroll
     for (int k = 0; k < S; k += 2) {
         float sq[2];
-        sqdiff2(x2[k / 2], yy, sq[0], sq[1]);
+        if constexpr (!FIX) sqdiff2(R.x2[k / 2], yy, sq[0], sq[1]);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int i = k + h;
             const unsigned dg = i == 0 ? bdiag : Pin[i > 0 ? i - 1 : 0];
             const unsigned up = i == 0 ? bup : Pout[i > 0 ? i - 1 : 0];
-            const float w = KIND == K_WDTW ? wq[S - 1 - i] : 1.0f;
-            unsigned v = add_cost<KIND>(sq[h], w, best_of<KIND>(dg, up, Pin[i], pen));
+            const unsigned best = best_of<KIND>(dg, up, Pin[i], pen);
+            unsigned v;
+            if constexpr (FIX) v = add_square(R.x[i] - (int)ybits, best);
+            else v = add_cost<KIND>(sq[h], KIND == K_WDTW ? wq[S - 1 - i] : 1.0f, best);
             if (MASK) v = ((M >> i) & 1u) ? v : kCap;
             Pout[i] = v;
         }
@@ -279,35 +360,59 @@ __device__ __forceinline__ float straight_path(const GuidedArgs &A, const Band &
     return __fmul_ru(sum, 1.000001f);
 }
 
-// Step 1: the sweep; returns the value of cell (n-1, m-1) in units.  xr, yr:
-// the pair's padded float series, su: their scale; all lanes of a warp share
-// the band.
-template <int KIND, int S>
+// A pair's padded series and their scale: su for the float copies, a shift for
+// the fixed-point ones.
+struct PairData {
+    const float *xf, *yf;
+    const int *xq, *yq;
+    float su;
+    Shift shift;
+    unsigned pen;
+
+    // column values 4 g .. 4 g + 3 as the sweep takes them
+    template <bool FIX>
+    __device__ __forceinline__ uint4 raw(int g) const {
+        return reinterpret_cast<const uint4 *>(FIX ? (const void *)yq : (const void *)yf)[g];
+    }
+    template <bool FIX>
+    __device__ __forceinline__ unsigned scaled(unsigned v) const {
+        if constexpr (FIX) return (unsigned)shift.of((int)v);
+        else return __float_as_uint(__fmul_rn(__uint_as_float(v), su));
+    }
+};
+
+// Step 1: the sweep; returns the value of cell (n-1, m-1) in units.  All lanes
+// of a warp share the band.
+template <int KIND, int S, bool FIX>
 __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band &B,
-                                                 const float *__restrict__ xr,
-                                                 const float *__restrict__ yr, int64_t gt,
-                                                 float su, unsigned pen) {
+                                                 const PairData &D, int64_t gt) {
     constexpr int LG = S == 8 ? 1 : 2;  // groups of 4 columns per block, as a shift
     const int64_t nth = A.nth;
     const int G = A.groups, NB = A.blocks;
     const uint4 CAP4 = make_uint4(kCap, kCap, kCap, kCap);
-    const float4 *y4 = reinterpret_cast<const float4 *>(yr);
+    const unsigned pen = D.pen;
     unsigned result = kCap;
     // row 0: cumulative, without penalties, weight index j - 1
     {
-        const float x0 = __fmul_rn(xr[3], su);
+        const float x0 = __fmul_rn(D.xf[3], D.su);
+        const int x0q = FIX ? D.shift.of(D.xq[3]) : 0;
         const int lim = imin(B.m, B.mx);
         unsigned acc = 0;
         for (int g = 0; g <= (lim - 1) >> 2; g++) {
-            const float4 y = y4[g];
-            const float yq[4] = {y.x, y.y, y.z, y.w};
+            const uint4 y = D.raw<FIX>(g);
+            const unsigned yq[4] = {y.x, y.y, y.z, y.w};
             unsigned v[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int c = 4 * g + q;
-                const float d = __fsub_rn(x0, __fmul_rn(yq[q], su));
-                const float w = KIND == K_WDTW ? A.wext[A.woff + imax(c - 1, 0)] : 1.0f;
-                acc = add_cost<KIND>(__fmul_rn(d, d), w, acc);
+                const unsigned yb = D.scaled<FIX>(yq[q]);
+                if constexpr (FIX) {
+                    acc = umin(add_square(x0q - (int)yb, acc), kCap);
+                } else {
+                    const float d = __fsub_rn(x0, __uint_as_float(yb));
+                    const float w = KIND == K_WDTW ? A.wext[A.woff + imax(c - 1, 0)] : 1.0f;
+                    acc = add_cost<KIND>(__fmul_rn(d, d), w, acc);
+                }
                 v[q] = c < lim ? acc : kCap;
             }
             A.ckrow[(int64_t)g * nth + gt] = make_uint4(v[0], v[1], v[2], v[3]);
@@ -326,14 +431,8 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
             bstart = imax(cs, i0 + S - 1 + B.lo);
             bend = imin(s == B.ns - 1 ? imin(ce, (B.m - 1) & ~3) : ce, i0 + B.mx);
         }
-        uint64_t x2[S / 2];
-        const float4 *x4 = reinterpret_cast<const float4 *>(xr + 3 + i0);
-#pragma unroll
-        for (int k = 0; k < S / 4; k++) {
-            const float4 t = x4[k];
-            x2[2 * k] = pack2(__fmul_rn(t.x, su), __fmul_rn(t.y, su));
-            x2[2 * k + 1] = pack2(__fmul_rn(t.z, su), __fmul_rn(t.w, su));
-        }
+        StripRows<S, FIX> R;
+        R.load(A, D.xf + 3 + i0, D.xq + 3 + i0, D.su, D.shift);
         const uint4 *in = A.ckrow + ((int64_t)s * G - pg0) * nth + gt;
         uint4 *out = A.ckrow + ((int64_t)(s + 1) * G - g0) * nth + gt;
         uint4 *col = A.ckcol + ((int64_t)s * NB - (g0 >> LG)) * (S / 4) * nth + gt;
@@ -342,16 +441,16 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
 #pragma unroll
         for (int k = 0; k < S; k++) P[k] = kCap;
         unsigned bd = up4(g0 - 1).w;
-        uint4 nu = up4(g0);
-        float4 ny = y4[g0];
+        // the row above two groups ahead, the columns one
+        uint4 nu = up4(g0), nnu = up4(g0 + 1);
+        uint4 ny = D.raw<FIX>(g0);
         for (int g = g0; g <= g1; g++) {
             const uint4 u = nu;
-            const float4 y = make_float4(__fmul_rn(ny.x, su), __fmul_rn(ny.y, su),
-                                         __fmul_rn(ny.z, su), __fmul_rn(ny.w, su));
-            if (g < g1) {
-                nu = up4(g + 1);
-                ny = y4[g + 1];
-            }
+            const uint4 y = make_uint4(D.scaled<FIX>(ny.x), D.scaled<FIX>(ny.y),
+                                       D.scaled<FIX>(ny.z), D.scaled<FIX>(ny.w));
+            nu = nnu;
+            nnu = up4(g + 2);
+            if (g < g1) ny = D.raw<FIX>(g + 1);
             float w[S + 4];
             if constexpr (KIND == K_WDTW) {
                 const float4 *w4 = reinterpret_cast<const float4 *>(
@@ -367,20 +466,20 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
             }
             uint4 o;
             if (4 * g >= bstart && 4 * g + 3 < bend) {
-                sweep_column<KIND, S, false>(P, Q, u.x, bd, x2, y.x, w, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(P, Q, u.x, bd, R, y.x, w, pen, 0u);
                 o.x = Q[S - 1];
-                sweep_column<KIND, S, false>(Q, P, u.y, u.x, x2, y.y, w + 1, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(Q, P, u.y, u.x, R, y.y, w + 1, pen, 0u);
                 o.y = P[S - 1];
-                sweep_column<KIND, S, false>(P, Q, u.z, u.y, x2, y.z, w + 2, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(P, Q, u.z, u.y, R, y.z, w + 2, pen, 0u);
                 o.z = Q[S - 1];
-                sweep_column<KIND, S, false>(Q, P, u.w, u.z, x2, y.w, w + 3, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(Q, P, u.w, u.z, R, y.w, w + 3, pen, 0u);
                 o.w = P[S - 1];
             } else {
                 const int e = 4 * g - i0 - B.lo;
                 auto masked = [&](int q, const unsigned(&Pin)[S], unsigned(&Pout)[S],
-                                  unsigned bup, unsigned bdg, float yq) {
+                                  unsigned bup, unsigned bdg, unsigned yq) {
                     const unsigned M = band_rows(e + q, B.width);
-                    sweep_column<KIND, S, true>(Pin, Pout, bup, bdg, x2, yq, w + q, pen, M);
+                    sweep_column<KIND, S, FIX, true>(Pin, Pout, bup, bdg, R, yq, w + q, pen, M);
                     if (s == B.ns - 1 && 4 * g + q == B.m - 1) {
 #pragma unroll
                         for (int k = 0; k < S; k++)
@@ -396,14 +495,20 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
                 masked(3, Q, P, u.w, u.z, y.w);
                 o.w = P[S - 1];
             }
+            if constexpr (FIX) {
+#pragma unroll
+                for (int k = 0; k < S; k++) P[k] = umin(P[k], kCap);
+                o = make_uint4(umin(o.x, kCap), umin(o.y, kCap), umin(o.z, kCap), P[S - 1]);
+                result = umin(result, kCap);
+            }
             bd = u.w;
             out[(int64_t)g * nth] = o;
             if (((g + 1) & ((1 << LG) - 1)) == 0) {
                 uint4 *cd = col + (int64_t)(g >> LG) * (S / 4) * nth;
 #pragma unroll
                 for (int k = 0; k < S / 4; k++)
-                    cd[k * nth] = make_uint4(P[4 * k], P[4 * k + 1], P[4 * k + 2],
-                                             P[4 * k + 3]);
+                    __stcs(cd + k * nth, make_uint4(P[4 * k], P[4 * k + 1], P[4 * k + 2],
+                                                    P[4 * k + 3]));
             }
         }
         pg0 = g0;
@@ -420,29 +525,26 @@ __device__ __forceinline__ unsigned push_sign(unsigned bits, int v) {
 // Step 2 of one block: cells (i0 + k, c0 + q), k, q < S, from the kept row
 // above, the kept column left of it, with the excluded-predecessor bits of
 // every column (row 0 of the block in the highest of the S bits).
-template <int KIND, int S>
+template <int KIND, int S, bool FIX>
 __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, int s, int b,
-                                           const float *__restrict__ xr,
-                                           const float *__restrict__ yr, int64_t gt, float su,
-                                           unsigned pen, unsigned tol, unsigned (&xd)[S],
-                                           unsigned (&xu)[S], unsigned (&xl)[S]) {
+                                           const PairData &D, int64_t gt, unsigned tol,
+                                           unsigned (&xd)[S], unsigned (&xu)[S],
+                                           unsigned (&xl)[S]) {
     constexpr int LG = S == 8 ? 1 : 2;
     const int64_t nth = A.nth;
     const int i0 = 1 + s * S, c0 = b * S;
-    uint64_t x2[S / 2];
-    const float4 *x4 = reinterpret_cast<const float4 *>(xr + 3 + i0);
-    const float4 *y4 = reinterpret_cast<const float4 *>(yr + c0);
-    unsigned P[S], Q[S], top[S];
-    float yv[S], w[2 * S];
+    const unsigned pen = D.pen;
+    StripRows<S, FIX> R;
+    R.load(A, D.xf + 3 + i0, D.xq + 3 + i0, D.su, D.shift);
+    unsigned P[S], Q[S], top[S], yv[S];
+    float w[2 * S];
 #pragma unroll
     for (int k = 0; k < S / 4; k++) {
-        const float4 t = x4[k], u = y4[k];
-        x2[2 * k] = pack2(__fmul_rn(t.x, su), __fmul_rn(t.y, su));
-        x2[2 * k + 1] = pack2(__fmul_rn(t.z, su), __fmul_rn(t.w, su));
-        yv[4 * k] = __fmul_rn(u.x, su);
-        yv[4 * k + 1] = __fmul_rn(u.y, su);
-        yv[4 * k + 2] = __fmul_rn(u.z, su);
-        yv[4 * k + 3] = __fmul_rn(u.w, su);
+        const uint4 u = D.raw<FIX>((c0 >> 2) + k);
+        yv[4 * k] = D.scaled<FIX>(u.x);
+        yv[4 * k + 1] = D.scaled<FIX>(u.y);
+        yv[4 * k + 2] = D.scaled<FIX>(u.z);
+        yv[4 * k + 3] = D.scaled<FIX>(u.w);
     }
     // row i0 - 1, from the strip above (the row-0 slot for s = 0)
     const int pg0 = B.cs(s - 1, S) >> 2, pg1 = (B.ce(s - 1, S) - 1) >> 2;
@@ -495,12 +597,13 @@ __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, i
     }
 #pragma unroll
     for (int q = 0; q < S; q++) {
-        const uint64_t yy = pack2(yv[q], yv[q]);
+        const float yfl = __uint_as_float(yv[q]);
+        const uint64_t yy = FIX ? 0 : pack2(yfl, yfl);
         unsigned bd_ = 0, bu_ = 0, bl_ = 0;
 #pragma unroll
         for (int k = 0; k < S; k += 2) {
             float sq[2];
-            sqdiff2(x2[k / 2], yy, sq[0], sq[1]);
+            if constexpr (!FIX) sqdiff2(R.x2[k / 2], yy, sq[0], sq[1]);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int i = k + h, j = i > 0 ? i - 1 : 0;
@@ -513,8 +616,9 @@ __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, i
                 bd_ = push_sign(bd_, t - (int)dg);
                 bu_ = push_sign(bu_, tm - (int)up);
                 bl_ = push_sign(bl_, tm - (int)lf);
-                const unsigned v =
-                    add_cost<KIND>(sq[h], KIND == K_WDTW ? w[q - i + S - 1] : 1.0f, best);
+                unsigned v;
+                if constexpr (FIX) v = umin(add_square(R.x[i] - (int)yv[q], best), kCap);
+                else v = add_cost<KIND>(sq[h], KIND == K_WDTW ? w[q - i + S - 1] : 1.0f, best);
                 Q[i] = umax(v, out_of_band[q - i + S - 1]);
             }
         }
@@ -545,20 +649,271 @@ __device__ __forceinline__ unsigned fill_up(unsigned r, unsigned xu) {
     return r | ((r & up) << 1);
 }
 
+// Steps 1 and 2 of the 32 pairs of a warp: the collected blocks go to the
+// threads' lists (last block first); returns their number (-1: not collected)
+// and in `row0` the last column collected of row 0.  e: the bound of an input
+// difference's error in square roots of units.
+template <int KIND, int S, bool FIX>
+__device__ __forceinline__ int collect(const GuidedArgs &A, const Band &B, const PairData &D,
+                                       float e, bool live, int64_t gt, int &row0) {
+    constexpr int W64 = S * S / 64;  // mask words of a block
+    constexpr int EW = 2 * W64 + 1;  // list words of a block: position, mask
+    constexpr unsigned SM = (1u << S) - 1u;
+    const unsigned FULL = 0xffffffffu;
+    const int64_t nth = A.nth;
+    const unsigned au = guided_sweep<KIND, S, FIX>(A, B, D, gt);
+
+    // the bound (file header); sqrt(A_max) <= sqrt(A + K) (1 + 2^-22) + 2 e sqrt(K)
+    const float K = (float)(B.n + B.m);
+    const float ek = __fmul_ru(e, __fsqrt_ru(K));
+    const float ra =
+        __fmaf_ru(2.1f, ek, __fmul_ru(__fsqrt_ru(__fadd_ru((float)au, K)), 1.000001f));
+    const float tolf = __fadd_ru(
+        __fmaf_ru(KIND == K_ADTW ? 2.02f : 1.01f, K,
+                  FIX ? 0.0f : __fmul_ru(1.2e-6f, __fmul_ru(ra, ra))),
+        __fadd_ru(__fmul_ru(__fmul_ru(4.2f, ek), __fadd_ru(ra, ek)), 8.0f));
+    live = live && au < kCap && tolf < 2.5e8f;
+    const unsigned tol = live ? (unsigned)tolf : 0u;
+
+    int s = B.ns - 1, b = (B.m - 1) / S;
+    int slo = B.m - 1, shi = B.m - 1;  // seeds in the strip's bottom row
+    int nlo = 0x7fffffff, nhi = -1;    // seeds of the strip above
+    unsigned carry = 0;                // cells reached in the column left of the block
+    int idx = live ? 0 : -1;
+    while (__any_sync(FULL, live)) {
+        if (live) {
+            unsigned xd[S], xu[S], xl[S];
+            block_bits<KIND, S, FIX>(A, B, s, b, D, gt, tol, xd, xu, xl);
+            const int c0 = b * S;
+            const int rows = imin(S, B.n - 1 - s * S);
+            const unsigned bottom = 1u << (S - rows);
+            uint64_t mask[W64];
+#pragma unroll
+            for (int w = 0; w < W64; w++) mask[w] = 0;
+            unsigned from = carry;
+#pragma unroll
+            for (int q = S - 1; q >= 0; q--) {
+                const int c = c0 + q;
+                unsigned r = from;
+                if (c >= slo && c <= shi) r |= bottom;
+                r = fill_up<S>(r, xu[q]);
+                const unsigned dg = (r & SM & ~xd[q]) << 1;
+                if (r >> S) {
+                    nlo = imin(nlo, c);
+                    nhi = imax(nhi, c);
+                }
+                if (dg >> S) {
+                    nlo = imin(nlo, c - 1);
+                    nhi = imax(nhi, c - 1);
+                }
+                r &= SM;
+                from = ((r & ~xl[q]) | dg) & SM;
+                mask[q * S / 64] |= (uint64_t)r << (64 - S - (q * S) % 64);
+            }
+            carry = from;
+            uint32_t *ent = A.list + (int64_t)idx * EW * nth + gt;
+            ent[0] = ((uint32_t)s << 16) | (uint32_t)b;
+#pragma unroll
+            for (int w = 0; w < W64; w++) {
+                ent[(1 + 2 * w) * nth] = (uint32_t)(mask[w] >> 32);
+                ent[(2 + 2 * w) * nth] = (uint32_t)mask[w];
+            }
+            idx++;
+            if (carry != 0 || slo < c0) {
+                b--;
+            } else {
+                slo = nlo;
+                shi = nhi;
+                nlo = 0x7fffffff;
+                nhi = -1;
+                b = shi / S;
+                s--;
+                if (s < 0) {
+                    live = false;
+                    if (shi < 0) idx = -1;
+                }
+            }
+            if (live && (idx == A.list_cap || b < 0 || shi < 0)) {
+                live = false;
+                idx = -1;  // the list is full
+            }
+        }
+    }
+    row0 = shi;
+    return idx;
+}
+
+// Step 3: the FP64 recurrence over the `count` collected blocks of each lane's
+// pair (rows X, columns Y); the sum of cell (n-1, m-1), for lanes with
+// count > 0.  The lanes go through their own blocks (mask words of 64 cells):
+// a lane whose word is done takes the next one after the warp's turn of up to
+// kCellsPerTurn cells, so the code that takes a word runs once per turn for
+// the whole warp.  Longer turns idle more lanes, shorter ones take words more
+// often: turns of 2, 3, 4, 6 and 12 cells ran 1000 x 1000 pairs of length 512,
+// r = 0.1, in 49, 46, 43, 42 and 40 ms.
+// Taking a word stages its rows, columns and the cells above it in shared
+// memory (all loads in flight at once); a cell then waits for shared memory
+// and the FP64 pipe only.  (An FP64 instruction takes 71 cycles of a warp and
+// 21 of the SM whatever its active lanes, so what counts is the number of
+// iterations: going through the strips in step, with the waits for the widest
+// lane in each strip, measured 4.9 against 3.3 million cycles per 32 pairs of
+// length 512.)
+constexpr int kCellsPerTurn = 12;
+
+template <int S>
+struct Stage {
+    static constexpr int C = 64 / S;  // columns of a mask word
+    double value[S][kThreads];        // last value of every row
+    double x[S][kThreads];
+    double y[C][kThreads];
+    double top[C + 1][kThreads];      // the row above, from the column left of the word
+};
+
+template <int KIND, int S>
+__device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__restrict__ X,
+                                           const double *__restrict__ Y, int count, int row0,
+                                           int64_t gt, Stage<S> &St) {
+    constexpr int W64 = S * S / 64;
+    constexpr int EW = 2 * W64 + 1;
+    constexpr int C = 64 / S;
+    constexpr unsigned SM = (1u << S) - 1u;
+    const int64_t nth = A.nth;
+    const double INF = WB_GINF64;
+    const ElasticJob &J = A.J;
+    const int tid = threadIdx.x;
+    const int n = J.rows.len, m = J.cols.len;
+    double *brow = A.brow + gt;  // [strip parity][column]: bottom rows
+    const int64_t mp = A.brow_cols;
+    if (count > 0) {
+        const double x0 = X[0];
+        double acc = 0.0;
+        for (int c = 0; c <= row0; c++) {
+            const double v = x0 - __ldg(Y + c);
+            double cst = v * v;
+            if (KIND == K_WDTW) cst = cst * __ldg(J.weights + imax(c - 1, 0));
+            acc = c == 0 ? cst : acc + cst;
+            brow[c * nth] = acc;
+        }
+    }
+    // list entry of the leftmost block, and first and last block, of the strip
+    // above and of the current one
+    int pfirst = 0, pblock = 0, plast = -1;
+    int cfirst = 0, cblock = 0, clast = 0;
+    int cur = -1, i0 = 0, cw = 0;
+    double *below = brow;
+    uint64_t M = 0, LM = 0, todo = 0;
+    unsigned tops = 0;  // bit q: cell (i0 - 1, cw - 1 + q) is collected
+    double last = 0.0, last_old = 0.0;
+    int left = imax(count, 0) * W64;  // mask words to go
+    auto entry = [&](int e) { return A.list + (int64_t)e * EW * nth + gt; };
+    auto word = [&](int j) -> uint64_t {  // word of the j-th step from the end
+        const uint32_t *p = entry(j / W64) + (1 + 2 * (W64 - 1 - j % W64)) * nth;
+        return ((uint64_t)p[0] << 32) | p[nth];
+    };
+    // the next word, loaded while the current one is worked on
+    uint32_t nh = left > 0 ? *entry((left - 1) / W64) : 0u;
+    uint64_t nM = left > 0 ? word(left - 1) : 0u;
+    while (__any_sync(0xffffffffu, todo != 0 || left > 0)) {
+        if (todo == 0 && left > 0) {
+            left--;
+            const uint32_t h = nh;
+            unsigned lm = (unsigned)(M & SM);  // collected rows of the column to the left
+            M = nM;
+            if (left > 0) {
+                nh = *entry((left - 1) / W64);
+                nM = word(left - 1);
+            }
+            const int w = W64 - 1 - left % W64;
+            const int bs = (int)(h >> 16), bb = (int)(h & 0xffffu);
+            if (bs != cur) {
+                pfirst = cfirst;
+                pblock = cblock;
+                plast = clast;
+                cfirst = left / W64;
+                cblock = bb;
+                lm = 0;
+                i0 = 1 + bs * S;
+                below = brow + (int64_t)((bs + 1) & 1) * mp * nth;
+#pragma unroll
+                for (int k = 0; k < S; k++) St.x[k][tid] = X[imin(i0 + k, n - 1)];
+            }
+            clast = bb;
+            cw = bb * S + w * C;
+            LM = (M >> S) | ((uint64_t)lm << (64 - S));
+            todo = M;
+#pragma unroll
+            for (int q = 0; q < C; q++) St.y[q][tid] = __ldg(Y + imin(cw + q, m - 1));
+            // the cells above the word: row 0, or the bottom bits of the strip
+            // above's blocks (consecutive entries, leftmost block last)
+            tops = 0;
+            if (bs == 0) {
+#pragma unroll
+                for (int q = 0; q <= C; q++)
+                    if (cw - 1 + q >= 0 && cw - 1 + q <= row0) tops |= 1u << q;
+            } else {
+                uint32_t bits[2] = {0, 0};  // of the word's block and the one to its left
+#pragma unroll
+                for (int o = 0; o < 2; o++) {
+                    const int blk = bb - o;
+                    if (blk < pblock || blk > plast || (o == 1 && w > 0)) continue;
+                    const uint32_t *p = entry(pfirst - (blk - pblock)) + nth;
+                    // bottom row: the lowest bit of every column
+                    const int pw = o == 0 ? w : W64 - 1;
+                    const uint64_t B = ((uint64_t)p[2 * pw * nth] << 32) | p[(2 * pw + 1) * nth];
+#pragma unroll
+                    for (int q = 0; q < C; q++)
+                        bits[o] |= (uint32_t)((B >> (64 - S - q * S)) & 1u) << q;
+                    if (o == 0 && w > 0) {  // the column left of the word, same block
+                        const uint32_t *p1 = p + 2 * (w - 1) * nth;
+                        bits[1] = (p1[nth] & 1u) << (C - 1);
+                    }
+                }
+                tops = (bits[0] << 1) | (bits[1] >> (C - 1));
+            }
+            const double *above = brow + (int64_t)(bs & 1) * mp * nth;
+#pragma unroll
+            for (int q = 0; q <= C; q++)
+                if ((tops >> q) & 1u) St.top[q][tid] = above[(int64_t)(cw - 1 + q) * nth];
+            cur = bs;
+        }
+#pragma unroll 1
+        for (int turn = 0; turn < kCellsPerTurn; turn++) {
+            if (todo == 0) break;
+            const int p = __clzll((long long)todo);
+            const uint64_t bit = 0x8000000000000000ULL >> p;
+            todo ^= bit;
+            const int k = p & (S - 1), q = p / S;
+            const double d = St.x[k][tid] - St.y[q][tid];
+            double cst = d * d;
+            if (KIND == K_WDTW) cst = cst * __ldg(J.weights + abs(i0 + k - cw - q));
+            const double old = St.value[k][tid];
+            const double lf = (LM & bit) ? old : INF;
+            // above: the cell before in this column, or the row above the block
+            const bool hu = k > 0 ? (M & (bit << 1)) != 0 : (tops >> (q + 1)) & 1u;
+            const bool hd = k > 0 ? (LM & (bit << 1)) != 0 : (tops >> q) & 1u;
+            const double tu = k > 0 ? last : St.top[q + 1][tid];
+            const double td = k > 0 ? (hu ? last_old : St.value[k - 1][tid]) : St.top[q][tid];
+            double mv = nn_min(hu ? tu : INF, lf);
+            if (KIND == K_ADTW) mv = mv + J.p;
+            const double nv = nn_min(mv, hd ? td : INF) + cst;
+            St.value[k][tid] = nv;
+            last = nv;
+            last_old = old;
+            if (k == S - 1) below[(int64_t)(cw + q) * nth] = nv;
+        }
+    }
+    return last;
+}
+
 template <int KIND, int S>
 __global__ void __launch_bounds__(kThreads, S == 8 ? 4 : 3)
 guided_pairs_kernel(const GuidedArgs A) {
-    constexpr int W64 = S * S / 64;     // mask words of a block
-    constexpr int EW = 2 * W64 + 1;     // list words of a block: position, mask
-    constexpr unsigned SM = (1u << S) - 1u;
-    __shared__ double vs[S][kThreads];  // last FP64 value of every block row
+    __shared__ Stage<S> stage;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int64_t nth = A.nth;
     const int64_t gt = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const ElasticJob &J = A.J;
     const Band B(A, S);
-    const double INF = WB_GINF64;
     double centre = 0.0, scale = 1.0;
     const bool finite = centre_scale(A.prep, centre, scale);
     const float penf = KIND == K_ADTW ? __double2float_ru(J.p * scale * scale) : 0.0f;
@@ -577,199 +932,67 @@ guided_pairs_kernel(const GuidedArgs A) {
             rs = t * 32 + lane;
             cs = rs;
         }
-        bool active = rs < J.rows.count && !(J.mode == PM_UPPER && rs >= cs);
+        const bool active = rs < J.rows.count && !(J.mode == PM_UPPER && rs >= cs);
         if (!__any_sync(FULL, active)) continue;
         if (!active) {  // sweeps along on a valid pair
             rs = J.rows.count - 1;
             cs = J.mode == PM_PAIRED ? rs : cs;
         }
-        const float *xr = A.xf + rs * A.xs;
-        const float *yr = A.yf + cs * A.ys;
-        // the power of two that brings the upper bound into (2^27, 2^29] units
-        const float ub = fmaxf(straight_path<KIND>(A, B, xr, yr, penf), 1e-30f);
-        bool live = active && finite && ub < 1e30f;
-        const int half = (29 - ilogbf(ub) - 1) >> 1;
-        const float su = live ? scalbnf(1.0f, half) : 1.0f;
-        const unsigned pen =
-            KIND == K_ADTW ? (unsigned)__float2int_rn(fminf(__fmul_rn(__fmul_rn(penf, su), su),
-                                                            (float)kCap))
-                           : 0u;
-        const unsigned au = guided_sweep<KIND, S>(A, B, xr, yr, gt, su, pen);
-
-        // the bound (file header) in units; sqrt(A_max) <= sqrt(A + K) (1 + 2^-22) + 2 e sqrt(K)
-        const float e = __fmul_ru(su, __fmaf_ru(6.0e-8f, __fadd_ru(A.xmax[rs], A.ymax[cs]), 1e-37f));
-        const float ek = __fmul_ru(e, __fsqrt_ru(K));
-        const float ra = __fmaf_ru(2.1f, ek, __fmul_ru(__fsqrt_ru(__fadd_ru((float)au, K)), 1.000001f));
-        const float tolf = __fadd_ru(
-            __fmaf_ru(KIND == K_ADTW ? 2.02f : 1.01f, K, __fmul_ru(1.2e-6f, __fmul_ru(ra, ra))),
-            __fadd_ru(__fmul_ru(__fmul_ru(4.2f, ek), __fadd_ru(ra, ek)), 8.0f));
-        live = live && au < kCap && tolf < 2.5e8f;
-        const unsigned tol = live ? (unsigned)tolf : 0u;
-        const bool swept = live;
-
-        // ---- step 2: collect cells, from the last strip up
-        int s = B.ns - 1, b = (B.m - 1) / S;
-        int slo = B.m - 1, shi = B.m - 1;       // seeds in the strip's bottom row
-        int nlo = 0x7fffffff, nhi = -1;         // seeds of the strip above
-        unsigned carry = 0;                     // cells reached in the column left of the block
-        int idx = 0;
-        while (__any_sync(FULL, live)) {
-            if (live) {
-                unsigned xd[S], xu[S], xl[S];
-                block_bits<KIND, S>(A, B, s, b, xr, yr, gt, su, pen, tol, xd, xu, xl);
-                const int c0 = b * S;
-                const int rows = imin(S, B.n - 1 - s * S);
-                const unsigned bottom = 1u << (S - rows);
-                uint64_t mask[W64];
-#pragma unroll
-                for (int w = 0; w < W64; w++) mask[w] = 0;
-                unsigned from = carry;
-#pragma unroll
-                for (int q = S - 1; q >= 0; q--) {
-                    const int c = c0 + q;
-                    unsigned r = from;
-                    if (c >= slo && c <= shi) r |= bottom;
-                    r = fill_up<S>(r, xu[q]);
-                    const unsigned dg = (r & SM & ~xd[q]) << 1;
-                    if (r >> S) {
-                        nlo = imin(nlo, c);
-                        nhi = imax(nhi, c);
-                    }
-                    if (dg >> S) {
-                        nlo = imin(nlo, c - 1);
-                        nhi = imax(nhi, c - 1);
-                    }
-                    r &= SM;
-                    from = ((r & ~xl[q]) | dg) & SM;
-                    mask[q * S / 64] |= (uint64_t)r << (64 - S - (q * S) % 64);
-                }
-                carry = from;
-                uint32_t *ent = A.list + (int64_t)idx * EW * nth + gt;
-                ent[0] = ((uint32_t)s << 16) | (uint32_t)b;
-#pragma unroll
-                for (int w = 0; w < W64; w++) {
-                    ent[(1 + 2 * w) * nth] = (uint32_t)(mask[w] >> 32);
-                    ent[(2 + 2 * w) * nth] = (uint32_t)mask[w];
-                }
-                idx++;
-                if (carry != 0 || slo < c0) {
-                    b--;
-                } else {
-                    slo = nlo;
-                    shi = nhi;
-                    nlo = 0x7fffffff;
-                    nhi = -1;
-                    b = shi / S;
-                    s--;
-                    if (s < 0) {
-                        live = false;
-                        if (shi < 0) idx = -1;
-                    }
-                }
-                if (live && (idx == A.list_cap || b < 0 || shi < 0)) {
-                    live = false;
-                    idx = -1;  // the list is full
-                }
-            }
+        PairData D;
+        D.xf = A.xf + rs * A.xs;
+        D.yf = A.yf + cs * A.ys;
+        D.xq = A.xq + rs * A.xs;
+        D.yq = A.yq + cs * A.ys;
+        const GuidedRange rx = A.xr[rs], ry = A.yr[cs];
+        // upper bound of the sum (of the FP64 inputs too)
+        float e = __fmaf_ru(6.0e-8f, __fadd_ru(rx.mag, ry.mag), 1e-37f);
+        float ub = __fsqrt_ru(straight_path<KIND>(A, B, D.xf, D.yf, penf));
+        ub = __fmaf_ru(e, __fsqrt_ru(K), ub);
+        ub = fmaxf(__fmul_ru(ub, ub), 1e-30f);
+        const bool live = active && finite && ub < 1e30f;
+        const int lub = ilogbf(ub);
+        // Fixed point: units of d^2 2^(26 + 2k) (d the scaled difference), the
+        // shift k as large as the pair's largest difference (see sweep_column)
+        // and the upper bound allow; where that
+        // leaves too few units for the sums' K roundings (differences far
+        // larger than the distance), the warp sweeps with float costs.
+        bool fix = false;
+        int shift = 0;
+        float units = 0.0f;
+        if constexpr (KIND != K_WDTW) {
+            const int dmax = imax(imax(rx.hi - ry.lo, ry.hi - rx.lo), 1);
+            const int bits = S == 8 && KIND == K_DTW ? 30 : 29;
+            shift = imax(imin(bits - (32 - __clz(dmax)), (2 - lub) >> 1), -24);
+            units = live ? scalbnf(1.0f, 26 + 2 * shift) : 0.0f;
+            fix = __all_sync(FULL, !live || (ub * units >= 16384.0f * K &&
+                                             penf * units <= 67108864.0f));
         }
-        const bool ok = swept && idx > 0;
+        D.shift = Shift{imax(shift, 0), imax(-shift, 0)};
+        const int half = live ? (28 - lub) >> 1 : 0;
+        D.su = scalbnf(1.0f, half);
+        if (fix) e = __fadd_ru(scalbnf(1.0f, shift), shift < 0 ? 2.0f : 0.0f) / 65536.0f;
+        else e = __fmul_ru(e, D.su);
+        if (!fix) units = __fmul_rn(D.su, D.su);
+        D.pen = KIND == K_ADTW
+                    ? (unsigned)__float2int_rn(fminf(__fmul_rn(penf, units), (float)kCap))
+                    : 0u;
+        int row0 = -1, count;
+        if (KIND != K_WDTW && fix) count = collect<KIND, S, KIND != K_WDTW>(A, B, D, e, live, gt, row0);
+        else count = collect<KIND, S, false>(A, B, D, e, live, gt, row0);
 
-        // ---- step 3: FP64 over the collected cells, in order
         double value = 0.0;
-        if (__any_sync(FULL, ok)) {
-            const double *X = J.rows.base + rs * J.rows.stride;
-            const double *Y = J.cols.base + cs * J.cols.stride;
-            double *brow = A.brow + gt;
-            const int64_t mp = A.brow_cols;
-            const int hi0 = ok ? shi : -1;
-            if (ok) {
-                const double x0 = X[0];
-                double acc = 0.0;
-                for (int c = 0; c <= hi0; c++) {
-                    const double v = x0 - __ldg(Y + c);
-                    double cst = v * v;
-                    if (KIND == K_WDTW) cst = cst * __ldg(J.weights + imax(c - 1, 0));
-                    acc = c == 0 ? cst : acc + cst;
-                    brow[c * nth] = acc;
-                }
-            }
-            int plo = 0, phi = -1, clo = 0, chi = hi0;  // columns held by brow
-            int cur = -1;
-            unsigned lm = 0;  // collected rows of the column left of the block
-            int ei = ok ? idx - 1 : -1;
-            while (__any_sync(FULL, ei >= 0)) {
-                if (ei >= 0) {
-                    const uint32_t *ent = A.list + (int64_t)ei * EW * nth + gt;
-                    const uint32_t h = ent[0];
-                    const int bs = (int)(h >> 16), bb = (int)(h & 0xffffu);
-                    if (bs != cur) {
-                        plo = clo;
-                        phi = chi;
-                        clo = bb * S;
-                        lm = 0;
-                        cur = bs;
-                    }
-                    chi = bb * S + S - 1;
-                    const double *above = brow + (int64_t)(bs & 1) * mp * nth;
-                    double *below = brow + (int64_t)((bs + 1) & 1) * mp * nth;
-                    const int i0 = 1 + bs * S;
-#pragma unroll 1
-                    for (int w = 0; w < W64; w++) {
-                        const uint64_t M = ((uint64_t)ent[(1 + 2 * w) * nth] << 32) |
-                                           ent[(2 + 2 * w) * nth];
-                        const uint64_t LM = (M >> S) | ((uint64_t)lm << (64 - S));
-                        const int cw = bb * S + w * (64 / S);
-#pragma unroll
-                        for (int q = 0; q < 64 / S; q++)
-                            if (!((M >> (64 - S - q * S)) & 1u)) below[(int64_t)(cw + q) * nth] = INF;
-                        uint64_t todo = M;
-                        double last = 0.0, last_old = 0.0;
-                        while (todo) {
-                            const int p = __clzll((long long)todo);
-                            const uint64_t bit = 0x8000000000000000ULL >> p;
-                            todo ^= bit;
-                            const int k = p & (S - 1);
-                            const int c = cw + p / S;
-                            const double d = X[i0 + k] - __ldg(Y + c);
-                            double cst = d * d;
-                            if (KIND == K_WDTW) cst = cst * __ldg(J.weights + abs(i0 + k - c));
-                            const double old = vs[k][threadIdx.x];
-                            const double lf = (LM & bit) ? old : INF;
-                            double up, dg;
-                            if (k > 0) {
-                                const bool hu = (M & (bit << 1)) != 0;
-                                up = hu ? last : INF;
-                                dg = INF;
-                                if (LM & (bit << 1)) dg = hu ? last_old : vs[k - 1][threadIdx.x];
-                            } else {
-                                up = c >= plo && c <= phi ? above[(int64_t)c * nth] : INF;
-                                dg = c - 1 >= plo && c - 1 <= phi ? above[(int64_t)(c - 1) * nth]
-                                                                  : INF;
-                            }
-                            double mv = nn_min(up, lf);
-                            if (KIND == K_ADTW) mv = mv + J.p;
-                            const double nv = nn_min(mv, dg) + cst;
-                            vs[k][threadIdx.x] = nv;
-                            last = nv;
-                            last_old = old;
-                            if (k == S - 1) below[(int64_t)c * nth] = nv;
-                            value = nv;
-                        }
-                        lm = (unsigned)(M & SM);
-                    }
-                    ei--;
-                }
-            }
-        }
+        if (__any_sync(FULL, count > 0))
+            value = evaluate<KIND, S>(A, J.rows.base + rs * J.rows.stride,
+                                      J.cols.base + cs * J.cols.stride, count, row0, gt, stage);
         if (active) {
-            const double res = ok ? sqrt(value) : __longlong_as_double(kGuidedPending);
+            const double res = count > 0 ? sqrt(value) : __longlong_as_double(kGuidedPending);
             if (J.mode == PM_PAIRED) {
                 J.out[rs] = res;
             } else {
                 J.out[rs * J.out_ld + cs] = res;
                 if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = res;
             }
-            if (!ok) atomicAdd(&A.prep->pending, 1ull);
+            if (count <= 0) atomicAdd(&A.prep->pending, 1ull);
         }
     }
 }
@@ -783,7 +1006,7 @@ struct Plan {
     int groups = 0, blocks = 0, list_cap = 0, brow_cols = 0;
     int64_t xs = 0, ys = 0;
     int woff = 0, wlen = 0;
-    size_t shared_bytes = 0;  // float copies, magnitudes, weights, prep
+    size_t shared_bytes = 0;  // copies of the series, their extremes, weights, prep
     size_t thread_bytes = 0;  // per resident thread
 };
 
@@ -831,8 +1054,10 @@ Plan plan_guided(const ElasticJob &J, size_t avail) {
         const int EW = S * S / 32 + 1;
         p.thread_bytes = (size_t)(ns + 1) * p.groups * 16 + (size_t)ns * p.blocks * S * 4 +
                          (size_t)p.list_cap * EW * 4 + (size_t)2 * p.brow_cols * 8;
-        p.shared_bytes = align256(J.rows.count * p.xs * 4) + align256(J.cols.count * p.ys * 4) +
-                         align256(J.rows.count * 4) + align256(J.cols.count * 4) +
+        p.shared_bytes = 2 * align256(J.rows.count * p.xs * 4) +
+                         2 * align256(J.cols.count * p.ys * 4) +
+                         align256(J.rows.count * sizeof(GuidedRange)) +
+                         align256(J.cols.count * sizeof(GuidedRange)) +
                          align256((size_t)imax(p.wlen, 1) * 4) + align256(sizeof(GuidedPrep)) +
                          4 * 256;
         int nb;
@@ -895,8 +1120,10 @@ int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
     WB_TAKE(prep, GuidedPrep, ws, 1);
     WB_TAKE(xf, float, ws, J.rows.count * p.xs);
     WB_TAKE(yf, float, ws, J.cols.count * p.ys);
-    WB_TAKE(xmax, float, ws, J.rows.count);
-    WB_TAKE(ymax, float, ws, J.cols.count);
+    WB_TAKE(xq, int, ws, J.rows.count * p.xs);
+    WB_TAKE(yq, int, ws, J.cols.count * p.ys);
+    WB_TAKE(xr, GuidedRange, ws, J.rows.count);
+    WB_TAKE(yr, GuidedRange, ws, J.cols.count);
     WB_TAKE(wext, float, ws, imax(p.wlen, 1));
     WB_TAKE(ckrow, uint4, ws, (size_t)(ns + 1) * p.groups * nth);
     WB_TAKE(ckcol, uint4, ws, (size_t)ns * p.blocks * (p.S / 4) * nth);
@@ -905,8 +1132,10 @@ int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
     A.prep = prep;
     A.xf = xf;
     A.yf = yf;
-    A.xmax = xmax;
-    A.ymax = ymax;
+    A.xq = xq;
+    A.yq = yq;
+    A.xr = xr;
+    A.yr = yr;
     A.wext = wext;
     A.ckrow = ckrow;
     A.ckcol = ckcol;
@@ -924,7 +1153,7 @@ int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
     const int64_t series = J.rows.count + J.cols.count;
     const int nw = J.kind == K_WDTW ? imax(J.rows.len, J.cols.len) : 0;
     guided_convert_kernel<<<(int)std::min(cap, (series + 7) / 8), 256, 0, s>>>(
-        J.rows, J.cols, p.xs, p.ys, prep, xf, yf, xmax, ymax, J.weights, nw,
+        J.rows, J.cols, p.xs, p.ys, prep, xf, yf, xq, yq, xr, yr, J.weights, nw,
         p.wlen ? wext : nullptr, p.woff, p.wlen);
     WB_LAUNCH_CHECK("guided_convert_kernel");
     switch (J.kind) {

@@ -19,11 +19,18 @@ struct GuidedPrep {
     unsigned long long pending;  // pairs left to the full recurrence
 };
 
+// Extremes of a series: fixed point, and the largest float magnitude.
+struct GuidedRange {
+    int lo, hi;
+    float mag;
+};
+
 struct GuidedArgs {
     ElasticJob J;
     const float *xf = nullptr, *yf = nullptr;  // centred, scaled, padded float series
+    const int *xq = nullptr, *yq = nullptr;    // the same in fixed point
     int64_t xs = 0, ys = 0;                    // their strides
-    const float *xmax = nullptr, *ymax = nullptr;
+    const GuidedRange *xr = nullptr, *yr = nullptr;
     const float *wext = nullptr;  // wdtw: weight of i - j at woff + (j - i)
     int woff = 0;
     GuidedPrep *prep = nullptr;
