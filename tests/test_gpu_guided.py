@@ -60,6 +60,8 @@ def _data(kind, rng, n, length):
         return w + 1e9
     if kind == "tiny":
         return w * 1e-200
+    if kind == "subnormal":  # whose squares are subnormal
+        return w * 1e-160
     if kind == "huge":
         return w * 1e150
     if kind == "outlier":
@@ -78,6 +80,7 @@ def test_pairwise_shapes(metric, params, lx, ly):
 
 
 @pytest.mark.parametrize("kind", ["noise", "integers", "binary", "constant", "offset", "tiny",
+                                  "subnormal",
                                   "huge", "outlier", "near"])
 @pytest.mark.parametrize("metric,params", METRICS, ids=IDS)
 def test_pairwise_data(metric, params, kind):

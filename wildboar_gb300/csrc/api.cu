@@ -18,6 +18,7 @@
 
 #include "dtw32.cuh"
 #include "elastic.cuh"
+#include "guided.cuh"
 #include "subseq.cuh"
 
 namespace wb {
@@ -690,6 +691,8 @@ extern "C" int wb_argmin_distance(const wb_series *x, const wb_series *y, int64_
     ea.all_zero = derivative(metric) && std::min(xl, yl) < 3;
     const bool use_ea = !argmin_ea_disabled() && argmin_ea_supported(ea);
     const size_t ea_ring_bytes = use_ea ? argmin_ea_ring_bytes(ea) : 0;
+    // dtw family: float32 bounds and guided evaluations in front of them
+    const bool use_guided = use_ea && argmin_guided_supported(ea);
     constexpr int kMaxChunks = 64;  // doubling chunks of at most 2^31 candidates
     auto schedule = [&](int64_t nq) {
         std::vector<int64_t> chunks;
@@ -713,7 +716,8 @@ extern "C" int wb_argmin_distance(const wb_series *x, const wb_series *y, int64_
         (lower_bound && !out_on_device ? align256(bpairs * 8) : 0) +
         (use_ea ? 2 * align256((size_t)batch * 8) + align256(kMaxChunks * 8) + ea_ring_bytes
                 : 0);
-    WB_TRY(ws.reserve(fixed + per_batch));
+    const size_t need = fixed + per_batch;
+    WB_TRY(ws.reserve(need + (use_guided ? argmin_guided_bytes(ea) : 0), need));
     WB_TRY(stage(x, dim, ws, J.rows));
     WB_TRY(stage(y, dim, ws, J.cols));
     WB_TRY(build_tables(metric, params, J, ws, false, xl, yl));
@@ -775,6 +779,32 @@ extern "C" int wb_argmin_distance(const wb_series *x, const wb_series *y, int64_
                 return fail(WB_ENOMEM, "workspace reservation exceeded");
             WB_CUDA(cudaMemsetAsync(counters, 0, kMaxChunks * 8, s));
             WB_TRY(launch_fill(A.state_dist, HUGE_VAL, nb, s));
+            GuidedArgmin guided;
+            bool guided_ok = false;
+            if (use_guided) WB_TRY(guided.prepare(Jb, ws, 0, guided_ok));
+            if (guided_ok) {
+                const std::vector<int64_t> at = argmin_guided_chunks(nb, y->n, k);
+                A.key = nullptr;  // abandoning never decides for these metrics
+                for (size_t c = 0; c + 1 < at.size(); c++) {
+                    EaChunk C;
+                    C.j0 = at[c];
+                    C.nc = at[c + 1] - at[c];
+                    C.nq = nb;
+                    C.ny = y->n;
+                    C.cur_dist = A.state_dist;
+                    C.lower_bound = lb;
+                    ElasticJob Jp = Jb;
+                    WB_TRY(guided.launch_chunk((int)c, C, s, &Jp.pending));
+                    WB_TRY(launch_argmin_ea(Jp, metric, xl, yl, C.j0, C.nc, y->n, A.state_dist,
+                                            lb, counters + c, ea_ring, s));
+                    A.j0 = at[c];
+                    A.j1 = at[c + 1];
+                    A.resume = c > 0;
+                    A.finish = c + 2 == at.size();
+                    WB_TRY(launch_argmin_replay(A, s));
+                }
+                continue;
+            }
             for (size_t c = 0; c + 1 < chunks.size(); c++) {
                 const int64_t a = chunks[c], b = chunks[c + 1];
                 WB_TRY(launch_argmin_ea(Jb, metric, xl, yl, a, b - a, y->n, A.state_dist, lb,

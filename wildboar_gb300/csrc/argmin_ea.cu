@@ -36,6 +36,7 @@
 
 #include "argmin.cuh"
 #include "elastic_rec.cuh"
+#include "guided.cuh"
 
 namespace wb {
 
@@ -45,6 +46,7 @@ constexpr int kEaThreads = 128;
 template <int KIND>
 __global__ void __launch_bounds__(kEaThreads)
 argmin_ea_kernel(const ElasticJob J, const EaChunk C, int P) {
+    if (J.pending && *J.pending == 0) return;
     const RingS ring{(int)threadIdx.x, kEaThreads};
     const int n = J.rows.len, m = J.cols.len, r = J.band;
     const int mx = imax(0, m - n) + r;
@@ -64,6 +66,10 @@ argmin_ea_kernel(const ElasticJob J, const EaChunk C, int P) {
             qi = p / C.nc;
             cj = C.j0 + (p - qi * C.nc);
             const double d = C.cur_dist[qi];
+            if (J.pending && !is_pending(J.out[qi * C.ny + cj])) {
+                p = (int64_t)atomicAdd(C.counter, 1ULL);
+                continue;
+            }
             if (C.lower_bound && C.lower_bound[qi * C.ny + cj] >= d) {
                 // the replay skips it: lb >= D_a >= every later k-th distance
                 J.out[qi * C.ny + cj] = INF;
@@ -139,6 +145,7 @@ argmin_ea_kernel(const ElasticJob J, const EaChunk C, int P) {
 template <int KIND, int S>
 __global__ void __launch_bounds__(kEaThreads)
 argmin_ea_strip_kernel(const ElasticJob J, const EaChunk C, double *ring_base, int64_t ring_ld) {
+    if (J.pending && *J.pending == 0) return;
     const int64_t gtid = (int64_t)blockIdx.x * kEaThreads + threadIdx.x;
     double *ring = ring_base + gtid * ring_ld;
     const int n = J.rows.len, m = J.cols.len, r = J.band;
@@ -160,6 +167,10 @@ argmin_ea_strip_kernel(const ElasticJob J, const EaChunk C, double *ring_base, i
             qi = p / C.nc;
             cj = C.j0 + (p - qi * C.nc);
             const double d = C.cur_dist[qi];
+            if (J.pending && !is_pending(J.out[qi * C.ny + cj])) {
+                p = (int64_t)atomicAdd(C.counter, 1ULL);
+                continue;
+            }
             if (C.lower_bound && C.lower_bound[qi * C.ny + cj] >= d) {
                 J.out[qi * C.ny + cj] = INF;
                 J.key[qi * C.ny + cj] = INF;

@@ -71,24 +71,11 @@ namespace {
 constexpr int kThreads = 128;
 constexpr unsigned kCap = 1u << 30;  // saturated value, and out of band
 constexpr int kFixOne = (1 << 29) - 1;  // 1.0 in fixed point
-#define WB_GINF __int_as_float(0x7f800000)
-#define WB_GINF64 __longlong_as_double(0x7ff0000000000000LL)
-
-// order-preserving integer code of a double (for atomicMin / atomicMax);
-// NaN counts as infinite
-__device__ __forceinline__ long long order_code(double v) {
-    const long long b = __double_as_longlong(v);
-    return b < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)b) : b;
-}
-__device__ __forceinline__ double order_value(long long c) {
-    return __longlong_as_double(
-        c < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)c) : c);
-}
 
 // Smallest and largest value of both series sets.
 __global__ void __launch_bounds__(256)
 guided_range_kernel(const SeriesSet a, const SeriesSet b, GuidedPrep *prep) {
-    double lo = WB_GINF64, hi = -WB_GINF64;
+    double lo = WB_DBL_INF, hi = -WB_DBL_INF;
     for (int set = 0; set < 2; set++) {
         const SeriesSet &S = set ? b : a;
         if (set && b.base == a.base) break;
@@ -97,7 +84,7 @@ guided_range_kernel(const SeriesSet a, const SeriesSet b, GuidedPrep *prep) {
              t += (int64_t)gridDim.x * 256) {
             const int64_t s = t / S.len;
             double v = S.base[s * S.stride + (t - s * S.len)];
-            if (isnan(v)) v = WB_GINF64;
+            if (isnan(v)) v = WB_DBL_INF;
             lo = v < lo ? v : lo;
             hi = v > hi ? v : hi;
         }
@@ -125,18 +112,6 @@ guided_range_kernel(const SeriesSet a, const SeriesSet b, GuidedPrep *prep) {
     }
 }
 
-// centre and power-of-two scale that map [lo, hi] into [-1, 1]
-__device__ __forceinline__ bool centre_scale(const GuidedPrep *prep, double &centre,
-                                             double &scale) {
-    const double lo = order_value(prep->lo), hi = order_value(prep->hi);
-    const double half = hi * 0.5 - lo * 0.5;
-    if (!(isfinite(lo) && isfinite(hi) && isfinite(half))) return false;
-    centre = lo * 0.5 + hi * 0.5;
-    const int e = half > 0.0 ? ilogb(half) + 1 : 0;
-    scale = scalbn(1.0, e < -1000 ? 1000 : -e);
-    return true;
-}
-
 // Float and 30-bit fixed-point copies of the centred, scaled series (one warp
 // per series) with their extremes.  Row series start at element 3, which puts
 // row 1 + S s on a 16-byte boundary.  Past a series' end the float copies cost
@@ -161,7 +136,7 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, in
         int *dsq = row ? xq + s * rs : yq + s * cs;
         const int lead = row ? 3 : 0;
         const int total = (int)(row ? rs : cs);
-        const float pad = row ? WB_GINF : -WB_GINF;
+        const float pad = row ? WB_FLT_INF : -WB_FLT_INF;
         float mx = 0.0f;
         int lo = kFixOne, hi = -kFixOne;
         for (int i = lane; i < total; i += 32) {
@@ -196,12 +171,6 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, in
 }
 
 // --------------------------------------------------------------------------
-
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-    uint64_t p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
-    return p;
-}
 
 // (a - b)^2 of both halves (each rounded as the scalar operations would be)
 __device__ __forceinline__ void sqdiff2(uint64_t a, uint64_t b, float &d0, float &d1) {
@@ -239,31 +208,6 @@ struct Shift {
     int left, right;
     __device__ __forceinline__ int of(int x) const {
         return (int)((unsigned)x << left) >> right;
-    }
-};
-
-// bits k (k < 32) with 0 <= e - k < width: strip rows in band at a column,
-// e = c - i0 - lo
-__device__ __forceinline__ unsigned band_rows(int e, int width) {
-    const unsigned upper = e < 0 ? 0u : (e >= 31 ? 0xffffffffu : (0xffffffffu >> (31 - e)));
-    const int lb = e - width + 1;
-    const unsigned lower = lb <= 0 ? 0u : (lb >= 32 ? 0xffffffffu : ((1u << lb) - 1u));
-    return upper & ~lower;
-}
-
-// the band of every pair (all pairs of a job share it)
-struct Band {
-    int n, m, r, mx, mn, lo, width, ns;
-    __device__ __forceinline__ Band(const GuidedArgs &A, int S)
-        : n(A.J.rows.len), m(A.J.cols.len), r(A.J.band), mx(imax(0, m - n) + r),
-          mn(imax(0, n - m)), lo(-(mn + r - 1)), width(mx - lo), ns((n - 1 + S - 1) / S) {}
-    // columns [cs, ce) of strip s (rows 1 + S s ...); s = -1: row 0
-    __device__ __forceinline__ int cs(int s, int S) const {
-        return imax(0, 1 + s * S - mn - r + 1);
-    }
-    __device__ __forceinline__ int ce(int s, int S) const {
-        const int last = s < 0 ? 0 : imin(n - 1, s * S + S);
-        return imin(m, last + mx);
     }
 };
 
@@ -778,7 +722,7 @@ __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__
     constexpr int C = 64 / S;
     constexpr unsigned SM = (1u << S) - 1u;
     const int64_t nth = A.nth;
-    const double INF = WB_GINF64;
+    const double INF = WB_DBL_INF;
     const ElasticJob &J = A.J;
     const int tid = threadIdx.x;
     const int n = J.rows.len, m = J.cols.len;
@@ -913,12 +857,15 @@ guided_pairs_kernel(const GuidedArgs A) {
     const int lane = threadIdx.x & 31;
     const int64_t gt = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const ElasticJob &J = A.J;
-    const Band B(A, S);
+    const Band B(J, S);
     double centre = 0.0, scale = 1.0;
     const bool finite = centre_scale(A.prep, centre, scale);
     const float penf = KIND == K_ADTW ? __double2float_ru(J.p * scale * scale) : 0.0f;
     const int64_t chunks = (J.rows.count + 31) >> 5;
-    const int64_t ntiles = J.mode == PM_PAIRED ? chunks : chunks * J.cols.count;
+    const bool listed = A.items != nullptr || A.n_all > 0;
+    const int64_t nlist = A.items ? (int64_t)*A.n_items : A.n_all;
+    const int64_t ntiles = listed ? (nlist + 31) >> 5
+                                  : (J.mode == PM_PAIRED ? chunks : chunks * J.cols.count);
     const float K = (float)(B.n + B.m);
 
     for (;;) {
@@ -932,9 +879,16 @@ guided_pairs_kernel(const GuidedArgs A) {
             rs = t * 32 + lane;
             cs = rs;
         }
-        const bool active = rs < J.rows.count && !(J.mode == PM_UPPER && rs >= cs);
+        bool active = rs < J.rows.count && !(J.mode == PM_UPPER && rs >= cs);
+        if (listed) {
+            const int64_t at = t * 32 + lane;
+            active = at < nlist;
+            const int64_t p = active ? (A.items ? (int64_t)A.items[at] : at) : 0;
+            cs = A.col0 + p / J.rows.count;
+            rs = p % J.rows.count;
+        }
         if (!__any_sync(FULL, active)) continue;
-        if (!active) {  // sweeps along on a valid pair
+        if (!active && !listed) {  // sweeps along on a valid pair
             rs = J.rows.count - 1;
             cs = J.mode == PM_PAIRED ? rs : cs;
         }
@@ -1025,11 +979,12 @@ int64_t round_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 // per-thread memory budget of the kept rows and columns of all resident pairs
 constexpr size_t kGuidedBudget = (size_t)8 << 30;
 
-Plan plan_guided(const ElasticJob &J, size_t avail) {
+// max_pairs > 0: for lists of at most so many pairs
+Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
     Plan p;
     const int n = J.rows.len, m = J.cols.len, r = J.band;
     if (J.kind != K_DTW && J.kind != K_WDTW && J.kind != K_ADTW) return p;
-    if (J.key || J.all_zero || J.pending) return p;
+    if ((J.key && max_pairs == 0) || J.all_zero || J.pending) return p;
     const char *e = getenv("WB_GPU_ELASTIC");
     if (e && (strcmp(e, "ring") == 0 || strcmp(e, "strip") == 0)) return p;
     const int mx = imax(0, m - n) + r, mn = imax(0, n - m);
@@ -1037,8 +992,9 @@ Plan plan_guided(const ElasticJob &J, size_t avail) {
     if (imin(n, m) < 24 || imin(width, m) < 12) return p;
     if ((int64_t)n + m > 1 << 15) return p;  // positions are 16 bits
     const DeviceInfo &dev = device_info();
-    const int64_t work = (J.mode == PM_PAIRED ? (J.rows.count + 31) / 32
-                                              : (J.rows.count + 31) / 32 * J.cols.count) * 32;
+    int64_t work = (J.mode == PM_PAIRED ? (J.rows.count + 31) / 32
+                                        : (J.rows.count + 31) / 32 * J.cols.count) * 32;
+    if (max_pairs > 0) work = std::min(work, max_pairs);
     const int64_t want = (work + kThreads - 1) / kThreads;
     for (int S = 8; S <= 16; S += 8) {
         const int ns = (n - 1 + S - 1) / S;
@@ -1080,34 +1036,38 @@ Plan plan_guided(const ElasticJob &J, size_t avail) {
 }
 
 template <int KIND>
-int run_kernel(const GuidedArgs &A, int S, int grid, cudaStream_t s) {
-    timer_begin("guided_pairs_kernel", s);
-    if (S == 8) guided_pairs_kernel<KIND, 8><<<grid, kThreads, 0, s>>>(A);
-    else guided_pairs_kernel<KIND, 16><<<grid, kThreads, 0, s>>>(A);
-    timer_end(s);
+int run_kernel(const GuidedContext &C, cudaStream_t s) {
+    if (C.S == 8) guided_pairs_kernel<KIND, 8><<<C.grid, kThreads, 0, s>>>(C.args);
+    else guided_pairs_kernel<KIND, 16><<<C.grid, kThreads, 0, s>>>(C.args);
     WB_LAUNCH_CHECK("guided_pairs_kernel");
     return WB_OK;
 }
 
 }  // namespace
 
-size_t guided_workspace_bytes(const ElasticJob &J) {
-    const Plan p = plan_guided(J, SIZE_MAX);
-    if (!p.use) return 0;
-    return p.shared_bytes + 2 * 4096 + p.thread_bytes * (size_t)p.grid * kThreads;
+static size_t plan_bytes(const Plan &p) {
+    return p.use ? p.shared_bytes + 2 * 4096 + p.thread_bytes * (size_t)p.grid * kThreads : 0;
 }
 
-int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
-                  unsigned long long **pending) {
-    *pending = nullptr;
+size_t guided_workspace_bytes(const ElasticJob &J) { return plan_bytes(plan_guided(J, SIZE_MAX)); }
+
+size_t guided_list_bytes(const ElasticJob &J, int64_t max_pairs) {
+    return plan_bytes(plan_guided(J, SIZE_MAX, max_pairs));
+}
+
+int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max_pairs,
+                   GuidedContext &C) {
     leave += 4096;  // and the alignment of the pieces
     const size_t avail = ws.remaining();
-    const Plan p = plan_guided(J, avail > leave ? avail - leave : 0);
+    const Plan p = plan_guided(J, avail > leave ? avail - leave : 0, max_pairs);
+    C.args.prep = nullptr;
     if (!p.use) return WB_OK;
     cudaStream_t s = ws.stream();
     const int ns = (J.rows.len - 1 + p.S - 1) / p.S;
     const int64_t nth = (int64_t)p.grid * kThreads;
-    GuidedArgs A;
+    C.S = p.S;
+    C.grid = p.grid;
+    GuidedArgs &A = C.args;
     A.J = J;
     A.nth = nth;
     A.groups = p.groups;
@@ -1141,10 +1101,9 @@ int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
     A.ckcol = ckcol;
     A.list = list;
     A.brow = brow;
-    // lo = the largest code, hi = the smallest, the counters zero
+    // lo = a very large code, hi = a very small one
     WB_CUDA(cudaMemsetAsync(&prep->lo, 0x7f, sizeof(prep->lo), s));
     WB_CUDA(cudaMemsetAsync(&prep->hi, 0x80, sizeof(prep->hi), s));
-    WB_CUDA(cudaMemsetAsync(&prep->queue, 0, 2 * sizeof(prep->queue), s));
     const int64_t cap = (int64_t)device_info().sm_count * 4;
     const int64_t values = J.rows.count * J.rows.len + J.cols.count * J.cols.len;
     guided_range_kernel<<<(int)std::min(cap, (values + 1023) / 1024), 256, 0, s>>>(
@@ -1156,12 +1115,29 @@ int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
         J.rows, J.cols, p.xs, p.ys, prep, xf, yf, xq, yq, xr, yr, J.weights, nw,
         p.wlen ? wext : nullptr, p.woff, p.wlen);
     WB_LAUNCH_CHECK("guided_convert_kernel");
-    switch (J.kind) {
-        case K_DTW: WB_TRY(run_kernel<K_DTW>(A, p.S, p.grid, s)); break;
-        case K_WDTW: WB_TRY(run_kernel<K_WDTW>(A, p.S, p.grid, s)); break;
-        default: WB_TRY(run_kernel<K_ADTW>(A, p.S, p.grid, s)); break;
+    return WB_OK;
+}
+
+int guided_run(const GuidedContext &C, cudaStream_t s) {
+    GuidedPrep *prep = C.args.prep;
+    WB_CUDA(cudaMemsetAsync(&prep->queue, 0, sizeof(prep->queue) + sizeof(prep->pending), s));
+    switch (C.args.J.kind) {
+        case K_DTW: return run_kernel<K_DTW>(C, s);
+        case K_WDTW: return run_kernel<K_WDTW>(C, s);
+        default: return run_kernel<K_ADTW>(C, s);
     }
-    *pending = &prep->pending;
+}
+
+int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
+                  unsigned long long **pending) {
+    *pending = nullptr;
+    GuidedContext C;
+    WB_TRY(guided_prepare(J, ws, leave, 0, C));
+    if (!C.args.prep) return WB_OK;
+    timer_begin("guided_pairs_kernel", ws.stream());
+    WB_TRY(guided_run(C, ws.stream()));
+    timer_end(ws.stream());
+    *pending = &C.args.prep->pending;
     return WB_OK;
 }
 

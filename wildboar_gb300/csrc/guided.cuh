@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 
 #include "elastic.cuh"
 
@@ -34,6 +35,12 @@ struct GuidedArgs {
     const float *wext = nullptr;  // wdtw: weight of i - j at woff + (j - i)
     int woff = 0;
     GuidedPrep *prep = nullptr;
+    // Instead of the job's mode: items p, the pair of row p % rows.count and
+    // column col0 + p / rows.count -- the `n_items` (device) ones of `items`,
+    // or without it all p < n_all.
+    const uint32_t *items = nullptr;
+    const unsigned *n_items = nullptr;
+    int64_t n_all = 0, col0 = 0;
     // per resident thread, interleaved [...][thread]
     int64_t nth = 0;
     uint4 *ckrow = nullptr;   // [strip + 1][group of 4 columns] bottom rows
@@ -43,6 +50,19 @@ struct GuidedArgs {
     int groups = 0, blocks = 0, list_cap = 0, brow_cols = 0;
 };
 
+// The guided evaluation in two steps, for a caller that runs it over several
+// lists of pairs: buffers and float / fixed-point series of the job (the grid
+// holds at most max_pairs pairs), then a run per list.  ctx.args.prep is null
+// when the job cannot be guided.
+struct GuidedContext {
+    GuidedArgs args;
+    int S = 8, grid = 0;
+};
+size_t guided_list_bytes(const ElasticJob &job, int64_t max_pairs);
+int guided_prepare(const ElasticJob &job, Workspace &ws, size_t leave, int64_t max_pairs,
+                   GuidedContext &ctx);
+int guided_run(const GuidedContext &ctx, cudaStream_t s);
+
 // Evaluates the job on what is left of the workspace beyond `leave` bytes;
 // *pending is null when
 // the job is not guided (or too little is left), else the device counter of
@@ -50,7 +70,86 @@ struct GuidedArgs {
 int launch_guided(const ElasticJob &job, Workspace &ws, size_t leave,
                   unsigned long long **pending);
 
+// argmin_distance of the dtw family over float32 bounds and guided
+// evaluations (argmin_guided.cu).
+bool argmin_guided_supported(const ElasticJob &job);
+size_t argmin_guided_bytes(const ElasticJob &job);
+// chunk boundaries of `ny` candidates for `nq` queries, from 0 to ny
+std::vector<int64_t> argmin_guided_chunks(int64_t nq, int64_t ny, int64_t k);
+class GuidedArgmin {
+  public:
+    int prepare(const ElasticJob &job, Workspace &ws, size_t leave, bool &ok);
+    int launch_chunk(int index, const EaChunk &chunk, cudaStream_t s,
+                     const unsigned long long **pending);
+
+  private:
+    struct Impl;
+    std::shared_ptr<Impl> impl_;
+};
+
 #ifdef __CUDACC__
+#define WB_FLT_INF __int_as_float(0x7f800000)
+#define WB_DBL_INF __longlong_as_double(0x7ff0000000000000LL)
+#define WB_DBL_MAX 1.7976931348623157e308
+
+// order-preserving integer code of a double (for atomicMin / atomicMax);
+// NaN counts as infinite
+__device__ __forceinline__ long long order_code(double v) {
+    const long long b = __double_as_longlong(v);
+    return b < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)b) : b;
+}
+__device__ __forceinline__ double order_value(long long c) {
+    return __longlong_as_double(
+        c < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)c) : c);
+}
+
+// Centre and power-of-two scale that map [lo, hi] into [-1, 1]; false where the
+// values are not finite or too small.
+__device__ __forceinline__ bool centre_scale(const GuidedPrep *prep, double &centre,
+                                             double &scale) {
+    const double lo = order_value(prep->lo), hi = order_value(prep->hi);
+    const double half = hi * 0.5 - lo * 0.5;
+    if (!(isfinite(lo) && isfinite(hi) && isfinite(half))) return false;
+    centre = lo * 0.5 + hi * 0.5;
+    const int e = half > 0.0 ? ilogb(half) + 1 : 0;
+    // (FP64 sums of squares of smaller values would round at the subnormal
+    // step, which the bounds do not cover)
+    if (e < -400) return false;
+    scale = scalbn(1.0, -e);
+    return true;
+}
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
+    return p;
+}
+
+// bits k (k < 32) with 0 <= e - k < width: strip rows in band at a column,
+// e = c - i0 - lo
+__device__ __forceinline__ unsigned band_rows(int e, int width) {
+    const unsigned upper = e < 0 ? 0u : (e >= 31 ? 0xffffffffu : (0xffffffffu >> (31 - e)));
+    const int lb = e - width + 1;
+    const unsigned lower = lb <= 0 ? 0u : (lb >= 32 ? 0xffffffffu : ((1u << lb) - 1u));
+    return upper & ~lower;
+}
+
+// the band of every pair (all pairs of a job share it)
+struct Band {
+    int n, m, r, mx, mn, lo, width, ns;
+    __device__ __forceinline__ Band(const ElasticJob &J, int S)
+        : n(J.rows.len), m(J.cols.len), r(J.band), mx(imax(0, m - n) + r),
+          mn(imax(0, n - m)), lo(-(mn + r - 1)), width(mx - lo), ns((n - 1 + S - 1) / S) {}
+    // columns [cs, ce) of strip s (rows 1 + S s ...); s = -1: row 0
+    __device__ __forceinline__ int cs(int s, int S) const {
+        return imax(0, 1 + s * S - mn - r + 1);
+    }
+    __device__ __forceinline__ int ce(int s, int S) const {
+        const int last = s < 0 ? 0 : imin(n - 1, s * S + S);
+        return imin(m, last + mx);
+    }
+};
+
 __device__ __forceinline__ bool is_pending(double v) {
     return __double_as_longlong(v) == kGuidedPending;
 }
