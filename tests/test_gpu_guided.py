@@ -1,5 +1,5 @@
-"""Guided FP64 evaluation (float32 sweep, FP64 on the cells it cannot rule
-out) against the full recurrence: the same bits for every metric it takes,
+"""Guided FP64 evaluation (32-bit sweep, FP64 on the cells it cannot rule out)
+and bit-parallel edr / lcss against the full recurrence: the same bits for every metric it takes,
 over its strip and block edges, bands, modes and data that stress its error
 bound (ties, constant stretches, near duplicates, offsets, tiny and huge
 values)."""
@@ -18,14 +18,17 @@ if not torch.cuda.is_available():  # pragma: no cover
 
 from wildboar_gb300.distance import paired_distance, pairwise_distance  # noqa: E402
 
+# edr / lcss take the bit-parallel form (full band), whose strips have 32 rows
 METRICS = [
+    ("edr", {}), ("edr", {"epsilon": 1.0}), ("edr", {"epsilon": 0.3}),
+    ("lcss", {}), ("lcss", {"epsilon": 0.4}),
     ("dtw", {"r": 0.1}), ("dtw", {"r": 0.37}), ("dtw", {"r": 1.0}),
     ("ddtw", {"r": 0.3}), ("wdtw", {"r": 1.0}), ("wdtw", {"r": 0.2, "g": 0.3}),
     ("wddtw", {"r": 1.0}), ("adtw", {"r": 0.2}), ("adtw", {"r": 1.0, "p": 0.05}),
     ("adtw", {"r": 0.5, "p": 0.0}),
 ]
 IDS = ["%s-%d" % (m, i) for i, (m, _) in enumerate(METRICS)]
-SHAPES = [(64, 64), (65, 65), (57, 130), (131, 60), (256, 249), (25, 400), (400, 26)]
+SHAPES = [(1, 5), (33, 1), (31, 33), (32, 32), (64, 64), (65, 65), (57, 130), (131, 60), (256, 249), (25, 400), (400, 26)]
 
 
 def _full(fn):

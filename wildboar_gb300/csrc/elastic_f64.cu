@@ -298,7 +298,9 @@ int launch_elastic(const ElasticJob &job, Workspace &ws, bool guided) {
         // then the full recurrence over the pairs it left, in the workspace
         // that it leaves
         unsigned long long *pending = nullptr;
-        WB_TRY(launch_guided(J, ws, elastic_workspace_bytes(J), &pending));
+        const size_t full = elastic_workspace_bytes(J);
+        if (bit_edit_supported(J)) WB_TRY(launch_bit_edit(J, ws, full, &pending));
+        else WB_TRY(launch_guided(J, ws, full, &pending));
         J.pending = pending;
     }
     if (use_strip_f64(J)) return launch_strip(J, ws, false);

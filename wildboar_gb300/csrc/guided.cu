@@ -118,10 +118,8 @@ guided_range_kernel(const SeriesSet a, const SeriesSet b, GuidedPrep *prep) {
 // +inf; the fixed-point ones hold 0 (cells there precede no cell of the
 // pair).
 __global__ void __launch_bounds__(256)
-guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, int64_t cs,
-                      const GuidedPrep *prep, float *xf, float *yf, int *xq, int *yq,
-                      GuidedRange *xr, GuidedRange *yr, const double *weights, int nw,
-                      float *wext, int woff, int wlen) {
+guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSeries D,
+                      const GuidedPrep *prep, const double *weights, int nw) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
     const int64_t nwarp = ((int64_t)gridDim.x * 256) >> 5;
@@ -132,10 +130,12 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, in
         const int64_t s = row ? t : t - rows.count;
         const SeriesSet &S = row ? rows : cols;
         const double *src = S.base + s * S.stride;
-        float *dst = row ? xf + s * rs : yf + s * cs;
-        int *dsq = row ? xq + s * rs : yq + s * cs;
+        const int64_t at = s * (row ? D.xs : D.ys);
+        float *dst = (row ? D.xf : D.yf) + at;
+        int *dsq = row ? D.xq : D.yq;
+        if (dsq) dsq += at;
         const int lead = row ? 3 : 0;
-        const int total = (int)(row ? rs : cs);
+        const int total = (int)(row ? D.xs : D.ys);
         const float pad = row ? WB_FLT_INF : -WB_FLT_INF;
         float mx = 0.0f;
         int lo = kFixOne, hi = -kFixOne;
@@ -152,21 +152,20 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, int64_t rs, in
                 hi = imax(hi, q);
             }
             dst[i] = v;
-            dsq[i] = q;
+            if (dsq) dsq[i] = q;
         }
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         lo = __reduce_min_sync(0xffffffffu, lo);
         hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane == 0) (row ? xr : yr)[s] = GuidedRange{lo, hi, mx};
+        if (lane == 0) (row ? D.xr : D.yr)[s] = GuidedRange{lo, hi, mx};
     }
-    // weights by |i - j|, for i - j of either sign
-    if (wext)
-        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < wlen;
+    // weights by |i - j|, for i - j of either sign (a zero weight would turn an
+    // infinite cost into NaN; 1e-38 is far below the bound's absolute term)
+    if (D.wext)
+        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < D.wlen;
              i += (int64_t)gridDim.x * 256) {
-            const int d = abs((int)i - woff);
-            // (a zero weight would turn an infinite cost into NaN; 1e-38 is far
-            // below the bound's absolute term)
-            wext[i] = fmaxf((float)weights[d < nw ? d : nw - 1], FLT_MIN);
+            const int d = abs((int)i - D.woff);
+            D.wext[i] = fmaxf((float)weights[d < nw ? d : nw - 1], FLT_MIN);
         }
 }
 
@@ -1049,10 +1048,29 @@ static size_t plan_bytes(const Plan &p) {
     return p.use ? p.shared_bytes + 2 * 4096 + p.thread_bytes * (size_t)p.grid * kThreads : 0;
 }
 
-size_t guided_workspace_bytes(const ElasticJob &J) { return plan_bytes(plan_guided(J, SIZE_MAX)); }
+size_t guided_workspace_bytes(const ElasticJob &J) {
+    if (bit_edit_supported(J)) return bit_edit_bytes(J);
+    return plan_bytes(plan_guided(J, SIZE_MAX));
+}
 
 size_t guided_list_bytes(const ElasticJob &J, int64_t max_pairs) {
     return plan_bytes(plan_guided(J, SIZE_MAX, max_pairs));
+}
+
+int guided_series(const ElasticJob &J, const GuidedSeries &S, GuidedPrep *prep, cudaStream_t s) {
+    // lo = a very large code, hi = a very small one
+    WB_CUDA(cudaMemsetAsync(&prep->lo, 0x7f, sizeof(prep->lo), s));
+    WB_CUDA(cudaMemsetAsync(&prep->hi, 0x80, sizeof(prep->hi), s));
+    const int64_t cap = (int64_t)device_info().sm_count * 4;
+    const int64_t values = J.rows.count * J.rows.len + J.cols.count * J.cols.len;
+    guided_range_kernel<<<(int)std::min(cap, (values + 1023) / 1024), 256, 0, s>>>(
+        J.rows, J.cols, prep);
+    WB_LAUNCH_CHECK("guided_range_kernel");
+    const int64_t series = J.rows.count + J.cols.count;
+    guided_convert_kernel<<<(int)std::min(cap, (series + 7) / 8), 256, 0, s>>>(
+        J.rows, J.cols, S, prep, J.weights, S.wext ? imax(J.rows.len, J.cols.len) : 0);
+    WB_LAUNCH_CHECK("guided_convert_kernel");
+    return WB_OK;
 }
 
 int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max_pairs,
@@ -1101,20 +1119,21 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     A.ckcol = ckcol;
     A.list = list;
     A.brow = brow;
-    // lo = a very large code, hi = a very small one
-    WB_CUDA(cudaMemsetAsync(&prep->lo, 0x7f, sizeof(prep->lo), s));
-    WB_CUDA(cudaMemsetAsync(&prep->hi, 0x80, sizeof(prep->hi), s));
-    const int64_t cap = (int64_t)device_info().sm_count * 4;
-    const int64_t values = J.rows.count * J.rows.len + J.cols.count * J.cols.len;
-    guided_range_kernel<<<(int)std::min(cap, (values + 1023) / 1024), 256, 0, s>>>(
-        J.rows, J.cols, prep);
-    WB_LAUNCH_CHECK("guided_range_kernel");
-    const int64_t series = J.rows.count + J.cols.count;
-    const int nw = J.kind == K_WDTW ? imax(J.rows.len, J.cols.len) : 0;
-    guided_convert_kernel<<<(int)std::min(cap, (series + 7) / 8), 256, 0, s>>>(
-        J.rows, J.cols, p.xs, p.ys, prep, xf, yf, xq, yq, xr, yr, J.weights, nw,
-        p.wlen ? wext : nullptr, p.woff, p.wlen);
-    WB_LAUNCH_CHECK("guided_convert_kernel");
+    GuidedSeries S;
+    S.xf = xf;
+    S.yf = yf;
+    S.xq = xq;
+    S.yq = yq;
+    S.xs = p.xs;
+    S.ys = p.ys;
+    S.xr = xr;
+    S.yr = yr;
+    if (p.wlen) {
+        S.wext = wext;
+        S.woff = p.woff;
+        S.wlen = p.wlen;
+    }
+    WB_TRY(guided_series(J, S, prep, s));
     return WB_OK;
 }
 

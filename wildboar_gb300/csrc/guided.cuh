@@ -50,6 +50,25 @@ struct GuidedArgs {
     int groups = 0, blocks = 0, list_cap = 0, brow_cols = 0;
 };
 
+// Centred, scaled, padded copies of a job's series (guided.cu): floats and,
+// where set, fixed point, the extremes of every series, extended weights.
+struct GuidedSeries {
+    float *xf = nullptr, *yf = nullptr;
+    int *xq = nullptr, *yq = nullptr;
+    int64_t xs = 0, ys = 0;  // strides; row series start at element 3
+    GuidedRange *xr = nullptr, *yr = nullptr;
+    float *wext = nullptr;
+    int woff = 0, wlen = 0;
+};
+int guided_series(const ElasticJob &job, const GuidedSeries &out, GuidedPrep *prep,
+                  cudaStream_t s);
+
+// edr / lcss over the full band, bit-parallel (bit_edit.cu); like launch_guided.
+bool bit_edit_supported(const ElasticJob &job);
+size_t bit_edit_bytes(const ElasticJob &job);
+int launch_bit_edit(const ElasticJob &job, Workspace &ws, size_t leave,
+                    unsigned long long **pending);
+
 // The guided evaluation in two steps, for a caller that runs it over several
 // lists of pairs: buffers and float / fixed-point series of the job (the grid
 // holds at most max_pairs pairs), then a run per list.  ctx.args.prep is null
