@@ -20,6 +20,7 @@
 #include "elastic.cuh"
 #include "guided.cuh"
 #include "subseq.cuh"
+#include "subseq_filter.cuh"
 
 namespace wb {
 
@@ -906,7 +907,9 @@ static int subseq_elastic(const double *shapelets, const int64_t *offsets,
                   (metric == WB_ERP ? align256((size_t)x->n * T * 8) + align256(x->n * 8) : 0) +
                   (metric == WB_TWE ? align256((size_t)max_orig * 8 + 8) : 0) +
                   (out_on_device ? 0 : 2 * align256(n_out * 8));
-    WB_TRY(ws.reserve(need));
+    const bool filter = !profile && subseq_filter_supported(J, kind, max_band);
+    const size_t filter_bytes = filter ? subseq_filter_bytes(J, total) : 0;
+    WB_TRY(ws.reserve(need + filter_bytes, need));
     WB_TAKE(gring, double, ws, ring / sizeof(double));
     SeriesSet X;
     WB_TRY(stage(x, dim, ws, X));
@@ -991,6 +994,8 @@ static int subseq_elastic(const double *shapelets, const int64_t *offsets,
     }
     J.out_dist = od;
     J.out_idx = oi;
+    if (filter && ws.remaining() >= filter_bytes)
+        WB_TRY(launch_subseq_filter(J, total, gring, P, grid, ws, s));
     WB_TRY(launch_elastic_subseq(J, kind, gring, P, grid, s));
     if (!out_on_device) {
         WB_CUDA(cudaMemcpyAsync(out_dist, od, n_out * 8, cudaMemcpyDeviceToHost, s));

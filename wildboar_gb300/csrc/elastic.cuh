@@ -122,6 +122,10 @@ struct SubseqElasticJob {
     double *prof_key = nullptr;
     int64_t prof_ld = 0;
     int std_as_given = 0;  // a zero shapelet std gives epsilon 0 (distance profile)
+    // second pass after the float32 filter (subseq_filter.cu): only the pairs
+    // with kept[pair] <= 0, *redo of them
+    const int *kept = nullptr;
+    const unsigned long long *redo = nullptr;
 };
 size_t elastic_subseq_ring_bytes(const SubseqElasticJob &J, int max_len, int max_band,
                                  int *P_out, int *grid_out);

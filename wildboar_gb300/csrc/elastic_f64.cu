@@ -346,6 +346,7 @@ elastic_subseq_kernel(const SubseqElasticJob J, double *gring, int P) {
     const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
     const int64_t gtid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t gthreads = (int64_t)gridDim.x * kThreads;
+    if (J.redo && *J.redo == 0) return;
     RingG ring{gring + gtid, gthreads};
     const double INF = WB_INF;
     const int64_t ntask = J.paired ? J.x.count : J.x.count * J.m;
@@ -353,6 +354,7 @@ elastic_subseq_kernel(const SubseqElasticJob J, double *gring, int P) {
         const int64_t si = J.paired ? task : task / J.m;
         const int64_t sh = J.paired ? task : task - si * J.m;
         const int64_t oidx = J.paired ? task : si * J.m + sh;
+        if (J.kept && J.kept[oidx] > 0) continue;
         const int Lorig = (int)J.len[sh];
         const int L = J.slopes ? Lorig - 2 : Lorig;  // length of the compared rows
         if (J.slopes && Lorig < 3) {
