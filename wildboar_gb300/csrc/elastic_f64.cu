@@ -87,12 +87,13 @@ elastic_pairs_kernel(const ElasticJob J, double *gring, int P) {
     const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
     const int64_t gtid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t gthreads = (int64_t)gridDim.x * kThreads;
-    if (J.pending && *J.pending == 0) return;
+    constexpr bool PASS2 = guided_kind(KIND);
+    if (PASS2 && J.pending && *J.pending == 0) return;
 
     auto body = [&](auto ring) {
         if (J.mode == PM_PAIRED) {
             for (int64_t s = gtid; s < J.rows.count; s += gthreads) {
-                if (J.pending && !is_pending(J.out[s])) continue;
+                if (PASS2 && J.pending && !is_pending(J.out[s])) continue;
                 double key, d;
                 d = J.all_zero ? 0.0 : finish(J, run_pair<KIND>(J, ring, P, s, s, key));
                 J.out[s] = d;
@@ -109,7 +110,7 @@ elastic_pairs_kernel(const ElasticJob J, double *gring, int P) {
             } else if (rs >= J.rows.count) {
                 continue;
             }
-            if (J.pending && !is_pending(J.out[rs * J.out_ld + cs])) continue;
+            if (PASS2 && J.pending && !is_pending(J.out[rs * J.out_ld + cs])) continue;
             double key = 0.0, d;
             if (J.all_zero) d = 0.0;
             else d = finish(J, run_pair<KIND>(J, ring, P, rs, cs, key));

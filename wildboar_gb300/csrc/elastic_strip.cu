@@ -532,7 +532,8 @@ __global__ void __launch_bounds__(kStripThreads)
     const int64_t nwarps = nth >> 5;
     typename A::R *ring = ring_base + gtid;
     const int n = J.rows.len, m = J.cols.len;
-    if (J.pending && *J.pending == 0) return;
+    constexpr bool PASS2 = guided_kind(KIND);
+    if (PASS2 && J.pending && *J.pending == 0) return;
 
     auto run = [&](int64_t rs, int64_t cs) -> double {
         if (J.all_zero) return 0.0;
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(kStripThreads)
 
     if (J.mode == PM_PAIRED) {
         for (int64_t s = gtid; s < J.rows.count; s += nth)
-            if (!J.pending || is_pending(J.out[s])) J.out[s] = run(s, s);
+            if (!PASS2 || !J.pending || is_pending(J.out[s])) J.out[s] = run(s, s);
         return;
     }
     const int64_t chunks = (J.rows.count + 31) >> 5;
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(kStripThreads)
         } else if (rs >= J.rows.count) {
             continue;
         }
-        if (J.pending && !is_pending(J.out[rs * J.out_ld + cs])) continue;
+        if (PASS2 && J.pending && !is_pending(J.out[rs * J.out_ld + cs])) continue;
         const double d = run(rs, cs);
         J.out[rs * J.out_ld + cs] = d;
         if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = d;

@@ -33,14 +33,17 @@
 // 3-input minimum, multiply-add); where the largest difference of a pair is
 // far above its distance, and for wdtw, the warp takes float32 costs rounded to
 // units instead (the conversion issues at 16 per clock and SM and takes most
-// of that sweep's time).
+// of that sweep's time, which hides the low parts of the inputs: without them
+// the inputs' rounding, unweighted, kept 467 instead of 155 blocks per pair for
+// wdtw at length 569, 17.3 instead of 6.3 ms for 143 x 6 pairs).
 //
 // Error bound.  With d = x - y of the centred, scaled, rounded inputs, the sum
 // of a path of at most K = n + m - 1 cells differs from its exact sum on these
 // inputs by K / 2 units and a few 2^-24 of it (float costs) or lies at most K
 // units below it (fixed point).  Rounding the inputs moves the 2-norm of a
-// path's differences by at most e sqrt(K), e = 2^-24 (max|x| + max|y|) for
-// float and two roundings of the shifted values for fixed-point inputs.  Hence for the best predecessor p of a cell on
+// path's differences by at most e sqrt(K), e = 2^-47 (max|x| + max|y|) for
+// float inputs with their low parts and two roundings of the shifted values for
+// fixed-point ones.  Hence for the best predecessor p of a cell on
 // a best path and any other predecessor q,
 //   A(p) <= A(q) + K + 16 2^-24 A_max + 4 e sqrt(K) sqrt(A_max) + 4 e^2 K,
 // A the swept values, A_max a bound of A along the path from its value at
@@ -112,8 +115,8 @@ guided_range_kernel(const SeriesSet a, const SeriesSet b, GuidedPrep *prep) {
     }
 }
 
-// Float and 30-bit fixed-point copies of the centred, scaled series (one warp
-// per series) with their extremes.  Row series start at element 3, which puts
+// Float (value and rest) and 30-bit fixed-point copies of the centred, scaled
+// series (one warp per series) with their extremes.  Row series start at element 3, which puts
 // row 1 + S s on a 16-byte boundary.  Past a series' end the float copies cost
 // +inf; the fixed-point ones hold 0 (cells there precede no cell of the
 // pair).
@@ -134,6 +137,8 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
         float *dst = (row ? D.xf : D.yf) + at;
         int *dsq = row ? D.xq : D.yq;
         if (dsq) dsq += at;
+        float *low = row ? D.xl : D.yl;
+        if (low) low += at;
         const int lead = row ? 3 : 0;
         const int total = (int)(row ? D.xs : D.ys);
         const float pad = row ? WB_FLT_INF : -WB_FLT_INF;
@@ -141,11 +146,12 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
         int lo = kFixOne, hi = -kFixOne;
         for (int i = lane; i < total; i += 32) {
             const int e = i - lead;
-            float v = pad;
+            float v = pad, rest = 0.0f;
             int q = 0;
             if (e >= 0 && e < S.len) {
                 const double c = (src[e] - centre) * scale;
                 v = (float)c;
+                rest = (float)(c - (double)v);
                 q = __double2int_rn(c * (double)kFixOne);
                 mx = fmaxf(mx, fabsf(v));
                 lo = imin(lo, q);
@@ -153,6 +159,7 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
             }
             dst[i] = v;
             if (dsq) dsq[i] = q;
+            if (low) low[i] = rest;
         }
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         lo = __reduce_min_sync(0xffffffffu, lo);
@@ -171,12 +178,13 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
 
 // --------------------------------------------------------------------------
 
-// (a - b)^2 of both halves (each rounded as the scalar operations would be)
-__device__ __forceinline__ void sqdiff2(uint64_t a, uint64_t b, float &d0, float &d1) {
-    asm("{\n\t.reg .b64 p;\n\tsub.rn.f32x2 p, %2, %3;\n\tmul.rn.f32x2 p, p, p;\n\t"
-        "mov.b64 {%0, %1}, p;\n\t}"
+// ((a - b) + (al - bl))^2 of both halves
+__device__ __forceinline__ void sqdiff2(uint64_t a, uint64_t al, uint64_t b, uint64_t bl,
+                                        float &d0, float &d1) {
+    asm("{\n\t.reg .b64 p, q;\n\tsub.rn.f32x2 p, %2, %4;\n\tsub.rn.f32x2 q, %3, %5;\n\t"
+        "add.rn.f32x2 p, p, q;\n\tmul.rn.f32x2 p, p, p;\n\tmov.b64 {%0, %1}, p;\n\t}"
         : "=f"(d0), "=f"(d1)
-        : "l"(a), "l"(b));
+        : "l"(a), "l"(al), "l"(b), "l"(bl));
 }
 
 // smallest predecessor (with the move's penalty) of a cell
@@ -210,34 +218,73 @@ struct Shift {
     }
 };
 
-// The S rows of a strip or block: scaled float pairs, or fixed point.
+// A pair's padded series and their scale: su for the float copies, a shift for
+// the fixed-point ones.
+struct PairData {
+    const float *xf, *yf, *xl, *yl;
+    const int *xq, *yq;
+    float su;
+    Shift shift;
+    unsigned pen;
+};
+
+// The S rows of a strip or block from row i0: scaled float pairs with their
+// low parts, or fixed point.
 template <int S, bool FIX>
 struct StripRows {
-    uint64_t x2[S / 2];
-    __device__ __forceinline__ void load(const GuidedArgs &, const float *xr, const int *,
-                                         float su, Shift) {
-        const float4 *x4 = reinterpret_cast<const float4 *>(xr);
+    uint64_t x2[S / 2], l2[S / 2];
+    __device__ __forceinline__ void load(const PairData &D, int i0) {
+        const float4 *x4 = reinterpret_cast<const float4 *>(D.xf + 3 + i0);
+        const float4 *l4 = reinterpret_cast<const float4 *>(D.xl + 3 + i0);
 #pragma unroll
         for (int k = 0; k < S / 4; k++) {
-            const float4 t = x4[k];
-            x2[2 * k] = pack2(__fmul_rn(t.x, su), __fmul_rn(t.y, su));
-            x2[2 * k + 1] = pack2(__fmul_rn(t.z, su), __fmul_rn(t.w, su));
+            const float4 t = x4[k], u = l4[k];
+            x2[2 * k] = pack2(__fmul_rn(t.x, D.su), __fmul_rn(t.y, D.su));
+            x2[2 * k + 1] = pack2(__fmul_rn(t.z, D.su), __fmul_rn(t.w, D.su));
+            l2[2 * k] = pack2(__fmul_rn(u.x, D.su), __fmul_rn(u.y, D.su));
+            l2[2 * k + 1] = pack2(__fmul_rn(u.z, D.su), __fmul_rn(u.w, D.su));
         }
     }
 };
 template <int S>
 struct StripRows<S, true> {
     int x[S];
-    __device__ __forceinline__ void load(const GuidedArgs &, const float *, const int *xq,
-                                         float, Shift sh) {
-        const int4 *x4 = reinterpret_cast<const int4 *>(xq);
+    __device__ __forceinline__ void load(const PairData &D, int i0) {
+        const int4 *x4 = reinterpret_cast<const int4 *>(D.xq + 3 + i0);
 #pragma unroll
         for (int k = 0; k < S / 4; k++) {
             const int4 t = x4[k];
-            x[4 * k] = sh.of(t.x);
-            x[4 * k + 1] = sh.of(t.y);
-            x[4 * k + 2] = sh.of(t.z);
-            x[4 * k + 3] = sh.of(t.w);
+            x[4 * k] = D.shift.of(t.x);
+            x[4 * k + 1] = D.shift.of(t.y);
+            x[4 * k + 2] = D.shift.of(t.z);
+            x[4 * k + 3] = D.shift.of(t.w);
+        }
+    }
+};
+
+// Columns 4 g .. 4 g + 3, as loaded and scaled.
+template <bool FIX>
+struct Columns {
+    uint4 v, l;
+    __device__ __forceinline__ void load(const PairData &D, int g) {
+        v = reinterpret_cast<const uint4 *>(FIX ? (const void *)D.yq : (const void *)D.yf)[g];
+        if constexpr (!FIX) l = reinterpret_cast<const uint4 *>(D.yl)[g];
+    }
+    __device__ __forceinline__ unsigned one(const PairData &D, unsigned t) const {
+        if constexpr (FIX) return (unsigned)D.shift.of((int)t);
+        else return __float_as_uint(__fmul_rn(__uint_as_float(t), D.su));
+    }
+    __device__ __forceinline__ void scaled(const PairData &D, unsigned (&y)[4],
+                                           unsigned (&yl)[4]) const {
+        y[0] = one(D, v.x);
+        y[1] = one(D, v.y);
+        y[2] = one(D, v.z);
+        y[3] = one(D, v.w);
+        if constexpr (!FIX) {
+            yl[0] = one(D, l.x);
+            yl[1] = one(D, l.y);
+            yl[2] = one(D, l.z);
+            yl[3] = one(D, l.w);
         }
     }
 };
@@ -251,12 +298,13 @@ template <int KIND, int S, bool FIX, bool MASK>
 __device__ __forceinline__ void sweep_column(const unsigned (&Pin)[S], unsigned (&Pout)[S],
                                              unsigned bup, unsigned bdiag,
                                              const StripRows<S, FIX> &R, unsigned ybits,
-                                             const float *wq, unsigned pen, unsigned M) {
-    const uint64_t yy = FIX ? 0 : pack2(__uint_as_float(ybits), __uint_as_float(ybits));
+                                             unsigned lbits, const float *wq, unsigned pen, unsigned M) {
+    const float yf = __uint_as_float(ybits), lf = __uint_as_float(lbits);
+    const uint64_t yy = FIX ? 0 : pack2(yf, yf), ll = FIX ? 0 : pack2(lf, lf);
 #pragma unroll
     for (int k = 0; k < S; k += 2) {
         float sq[2];
-        if constexpr (!FIX) sqdiff2(R.x2[k / 2], yy, sq[0], sq[1]);
+        if constexpr (!FIX) sqdiff2(R.x2[k / 2], R.l2[k / 2], yy, ll, sq[0], sq[1]);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int i = k + h;
@@ -303,27 +351,6 @@ __device__ __forceinline__ float straight_path(const GuidedArgs &A, const Band &
     return __fmul_ru(sum, 1.000001f);
 }
 
-// A pair's padded series and their scale: su for the float copies, a shift for
-// the fixed-point ones.
-struct PairData {
-    const float *xf, *yf;
-    const int *xq, *yq;
-    float su;
-    Shift shift;
-    unsigned pen;
-
-    // column values 4 g .. 4 g + 3 as the sweep takes them
-    template <bool FIX>
-    __device__ __forceinline__ uint4 raw(int g) const {
-        return reinterpret_cast<const uint4 *>(FIX ? (const void *)yq : (const void *)yf)[g];
-    }
-    template <bool FIX>
-    __device__ __forceinline__ unsigned scaled(unsigned v) const {
-        if constexpr (FIX) return (unsigned)shift.of((int)v);
-        else return __float_as_uint(__fmul_rn(__uint_as_float(v), su));
-    }
-};
-
 // Step 1: the sweep; returns the value of cell (n-1, m-1) in units.  All lanes
 // of a warp share the band.
 template <int KIND, int S, bool FIX>
@@ -337,22 +364,23 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
     unsigned result = kCap;
     // row 0: cumulative, without penalties, weight index j - 1
     {
-        const float x0 = __fmul_rn(D.xf[3], D.su);
+        const float x0 = __fmul_rn(D.xf[3], D.su), x0l = __fmul_rn(D.xl[3], D.su);
         const int x0q = FIX ? D.shift.of(D.xq[3]) : 0;
         const int lim = imin(B.m, B.mx);
         unsigned acc = 0;
         for (int g = 0; g <= (lim - 1) >> 2; g++) {
-            const uint4 y = D.raw<FIX>(g);
-            const unsigned yq[4] = {y.x, y.y, y.z, y.w};
-            unsigned v[4];
+            Columns<FIX> Y;
+            Y.load(D, g);
+            unsigned y[4], yl[4], v[4];
+            Y.scaled(D, y, yl);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int c = 4 * g + q;
-                const unsigned yb = D.scaled<FIX>(yq[q]);
                 if constexpr (FIX) {
-                    acc = umin(add_square(x0q - (int)yb, acc), kCap);
+                    acc = umin(add_square(x0q - (int)y[q], acc), kCap);
                 } else {
-                    const float d = __fsub_rn(x0, __uint_as_float(yb));
+                    const float d = __fadd_rn(__fsub_rn(x0, __uint_as_float(y[q])),
+                                              __fsub_rn(x0l, __uint_as_float(yl[q])));
                     const float w = KIND == K_WDTW ? A.wext[A.woff + imax(c - 1, 0)] : 1.0f;
                     acc = add_cost<KIND>(__fmul_rn(d, d), w, acc);
                 }
@@ -375,7 +403,7 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
             bend = imin(s == B.ns - 1 ? imin(ce, (B.m - 1) & ~3) : ce, i0 + B.mx);
         }
         StripRows<S, FIX> R;
-        R.load(A, D.xf + 3 + i0, D.xq + 3 + i0, D.su, D.shift);
+        R.load(D, i0);
         const uint4 *in = A.ckrow + ((int64_t)s * G - pg0) * nth + gt;
         uint4 *out = A.ckrow + ((int64_t)(s + 1) * G - g0) * nth + gt;
         uint4 *col = A.ckcol + ((int64_t)s * NB - (g0 >> LG)) * (S / 4) * nth + gt;
@@ -386,14 +414,15 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
         unsigned bd = up4(g0 - 1).w;
         // the row above two groups ahead, the columns one
         uint4 nu = up4(g0), nnu = up4(g0 + 1);
-        uint4 ny = D.raw<FIX>(g0);
+        Columns<FIX> Y;
+        Y.load(D, g0);
         for (int g = g0; g <= g1; g++) {
             const uint4 u = nu;
-            const uint4 y = make_uint4(D.scaled<FIX>(ny.x), D.scaled<FIX>(ny.y),
-                                       D.scaled<FIX>(ny.z), D.scaled<FIX>(ny.w));
+            unsigned y[4], yl[4];
+            Y.scaled(D, y, yl);
             nu = nnu;
             nnu = up4(g + 2);
-            if (g < g1) ny = D.raw<FIX>(g + 1);
+            if (g < g1) Y.load(D, g + 1);
             float w[S + 4];
             if constexpr (KIND == K_WDTW) {
                 const float4 *w4 = reinterpret_cast<const float4 *>(
@@ -409,33 +438,34 @@ __device__ __forceinline__ unsigned guided_sweep(const GuidedArgs &A, const Band
             }
             uint4 o;
             if (4 * g >= bstart && 4 * g + 3 < bend) {
-                sweep_column<KIND, S, FIX, false>(P, Q, u.x, bd, R, y.x, w, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(P, Q, u.x, bd, R, y[0], yl[0], w, pen, 0u);
                 o.x = Q[S - 1];
-                sweep_column<KIND, S, FIX, false>(Q, P, u.y, u.x, R, y.y, w + 1, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(Q, P, u.y, u.x, R, y[1], yl[1], w + 1, pen, 0u);
                 o.y = P[S - 1];
-                sweep_column<KIND, S, FIX, false>(P, Q, u.z, u.y, R, y.z, w + 2, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(P, Q, u.z, u.y, R, y[2], yl[2], w + 2, pen, 0u);
                 o.z = Q[S - 1];
-                sweep_column<KIND, S, FIX, false>(Q, P, u.w, u.z, R, y.w, w + 3, pen, 0u);
+                sweep_column<KIND, S, FIX, false>(Q, P, u.w, u.z, R, y[3], yl[3], w + 3, pen, 0u);
                 o.w = P[S - 1];
             } else {
                 const int e = 4 * g - i0 - B.lo;
                 auto masked = [&](int q, const unsigned(&Pin)[S], unsigned(&Pout)[S],
-                                  unsigned bup, unsigned bdg, unsigned yq) {
+                                  unsigned bup, unsigned bdg) {
                     const unsigned M = band_rows(e + q, B.width);
-                    sweep_column<KIND, S, FIX, true>(Pin, Pout, bup, bdg, R, yq, w + q, pen, M);
+                    sweep_column<KIND, S, FIX, true>(Pin, Pout, bup, bdg, R, y[q], yl[q], w + q,
+                                                     pen, M);
                     if (s == B.ns - 1 && 4 * g + q == B.m - 1) {
 #pragma unroll
                         for (int k = 0; k < S; k++)
                             if (k < rows) result = Pout[k];
                     }
                 };
-                masked(0, P, Q, u.x, bd, y.x);
+                masked(0, P, Q, u.x, bd);
                 o.x = Q[S - 1];
-                masked(1, Q, P, u.y, u.x, y.y);
+                masked(1, Q, P, u.y, u.x);
                 o.y = P[S - 1];
-                masked(2, P, Q, u.z, u.y, y.z);
+                masked(2, P, Q, u.z, u.y);
                 o.z = Q[S - 1];
-                masked(3, Q, P, u.w, u.z, y.w);
+                masked(3, Q, P, u.w, u.z);
                 o.w = P[S - 1];
             }
             if constexpr (FIX) {
@@ -476,18 +506,22 @@ __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, i
     constexpr int LG = S == 8 ? 1 : 2;
     const int64_t nth = A.nth;
     const int i0 = 1 + s * S, c0 = b * S;
-    const unsigned pen = D.pen;
     StripRows<S, FIX> R;
-    R.load(A, D.xf + 3 + i0, D.xq + 3 + i0, D.su, D.shift);
-    unsigned P[S], Q[S], top[S], yv[S];
+    R.load(D, i0);
+    const unsigned pen = D.pen;
+    unsigned P[S], Q[S], top[S], y[S], yl[S];
     float w[2 * S];
 #pragma unroll
     for (int k = 0; k < S / 4; k++) {
-        const uint4 u = D.raw<FIX>((c0 >> 2) + k);
-        yv[4 * k] = D.scaled<FIX>(u.x);
-        yv[4 * k + 1] = D.scaled<FIX>(u.y);
-        yv[4 * k + 2] = D.scaled<FIX>(u.z);
-        yv[4 * k + 3] = D.scaled<FIX>(u.w);
+        Columns<FIX> Y;
+        Y.load(D, (c0 >> 2) + k);
+        unsigned t[4], u[4];
+        Y.scaled(D, t, u);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            y[4 * k + q] = t[q];
+            if (!FIX) yl[4 * k + q] = u[q];
+        }
     }
     // row i0 - 1, from the strip above (the row-0 slot for s = 0)
     const int pg0 = B.cs(s - 1, S) >> 2, pg1 = (B.ce(s - 1, S) - 1) >> 2;
@@ -540,13 +574,13 @@ __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, i
     }
 #pragma unroll
     for (int q = 0; q < S; q++) {
-        const float yfl = __uint_as_float(yv[q]);
-        const uint64_t yy = FIX ? 0 : pack2(yfl, yfl);
+        const float yf = __uint_as_float(y[q]), lf_ = FIX ? 0.0f : __uint_as_float(yl[q]);
+        const uint64_t yy = FIX ? 0 : pack2(yf, yf), ll = FIX ? 0 : pack2(lf_, lf_);
         unsigned bd_ = 0, bu_ = 0, bl_ = 0;
 #pragma unroll
         for (int k = 0; k < S; k += 2) {
             float sq[2];
-            if constexpr (!FIX) sqdiff2(R.x2[k / 2], yy, sq[0], sq[1]);
+            if constexpr (!FIX) sqdiff2(R.x2[k / 2], R.l2[k / 2], yy, ll, sq[0], sq[1]);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int i = k + h, j = i > 0 ? i - 1 : 0;
@@ -560,7 +594,7 @@ __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, i
                 bu_ = push_sign(bu_, tm - (int)up);
                 bl_ = push_sign(bl_, tm - (int)lf);
                 unsigned v;
-                if constexpr (FIX) v = umin(add_square(R.x[i] - (int)yv[q], best), kCap);
+                if constexpr (FIX) v = umin(add_square(R.x[i] - (int)y[q], best), kCap);
                 else v = add_cost<KIND>(sq[h], KIND == K_WDTW ? w[q - i + S - 1] : 1.0f, best);
                 Q[i] = umax(v, out_of_band[q - i + S - 1]);
             }
@@ -894,6 +928,8 @@ guided_pairs_kernel(const GuidedArgs A) {
         PairData D;
         D.xf = A.xf + rs * A.xs;
         D.yf = A.yf + cs * A.ys;
+        D.xl = A.xl + rs * A.xs;
+        D.yl = A.yl + cs * A.ys;
         D.xq = A.xq + rs * A.xs;
         D.yq = A.yq + cs * A.ys;
         const GuidedRange rx = A.xr[rs], ry = A.yr[cs];
@@ -924,7 +960,9 @@ guided_pairs_kernel(const GuidedArgs A) {
         const int half = live ? (28 - lub) >> 1 : 0;
         D.su = scalbnf(1.0f, half);
         if (fix) e = __fadd_ru(scalbnf(1.0f, shift), shift < 0 ? 2.0f : 0.0f) / 65536.0f;
-        else e = __fmul_ru(e, D.su);
+        // (float differences with their low parts: relative errors apart,
+        // which the bound counts, they are off by 2^-47 of the values)
+        else e = __fmul_ru(__fmul_ru(e, 1.3e-7f), D.su);
         if (!fix) units = __fmul_rn(D.su, D.su);
         D.pen = KIND == K_ADTW
                     ? (unsigned)__float2int_rn(fminf(__fmul_rn(penf, units), (float)kCap))
@@ -1009,8 +1047,8 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
         const int EW = S * S / 32 + 1;
         p.thread_bytes = (size_t)(ns + 1) * p.groups * 16 + (size_t)ns * p.blocks * S * 4 +
                          (size_t)p.list_cap * EW * 4 + (size_t)2 * p.brow_cols * 8;
-        p.shared_bytes = 2 * align256(J.rows.count * p.xs * 4) +
-                         2 * align256(J.cols.count * p.ys * 4) +
+        p.shared_bytes = 3 * align256(J.rows.count * p.xs * 4) +
+                         3 * align256(J.cols.count * p.ys * 4) +
                          align256(J.rows.count * sizeof(GuidedRange)) +
                          align256(J.cols.count * sizeof(GuidedRange)) +
                          align256((size_t)imax(p.wlen, 1) * 4) + align256(sizeof(GuidedPrep)) +
@@ -1098,6 +1136,8 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     WB_TAKE(prep, GuidedPrep, ws, 1);
     WB_TAKE(xf, float, ws, J.rows.count * p.xs);
     WB_TAKE(yf, float, ws, J.cols.count * p.ys);
+    WB_TAKE(xl, float, ws, J.rows.count * p.xs);
+    WB_TAKE(yl, float, ws, J.cols.count * p.ys);
     WB_TAKE(xq, int, ws, J.rows.count * p.xs);
     WB_TAKE(yq, int, ws, J.cols.count * p.ys);
     WB_TAKE(xr, GuidedRange, ws, J.rows.count);
@@ -1110,6 +1150,8 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     A.prep = prep;
     A.xf = xf;
     A.yf = yf;
+    A.xl = xl;
+    A.yl = yl;
     A.xq = xq;
     A.yq = yq;
     A.xr = xr;
@@ -1122,6 +1164,8 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     GuidedSeries S;
     S.xf = xf;
     S.yf = yf;
+    S.xl = xl;
+    S.yl = yl;
     S.xq = xq;
     S.yq = yq;
     S.xs = p.xs;

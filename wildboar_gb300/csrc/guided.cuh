@@ -14,6 +14,11 @@ namespace wb {
 // produces).
 constexpr long long kGuidedPending = 0x7ff8d7a05e1e57edLL;
 
+// Kinds with a first pass that can leave pairs pending.
+constexpr bool guided_kind(int kind) {
+    return kind == K_DTW || kind == K_WDTW || kind == K_ADTW || kind == K_EDR || kind == K_LCSS;
+}
+
 struct GuidedPrep {
     long long lo, hi;            // order codes of the smallest / largest input
     unsigned long long queue;    // next tile of 32 pairs
@@ -29,6 +34,7 @@ struct GuidedRange {
 struct GuidedArgs {
     ElasticJob J;
     const float *xf = nullptr, *yf = nullptr;  // centred, scaled, padded float series
+    const float *xl = nullptr, *yl = nullptr;  // their rests
     const int *xq = nullptr, *yq = nullptr;    // the same in fixed point
     int64_t xs = 0, ys = 0;                    // their strides
     const GuidedRange *xr = nullptr, *yr = nullptr;
@@ -54,6 +60,7 @@ struct GuidedArgs {
 // where set, fixed point, the extremes of every series, extended weights.
 struct GuidedSeries {
     float *xf = nullptr, *yf = nullptr;
+    float *xl = nullptr, *yl = nullptr;  // the floats' rests
     int *xq = nullptr, *yq = nullptr;
     int64_t xs = 0, ys = 0;  // strides; row series start at element 3
     GuidedRange *xr = nullptr, *yr = nullptr;
