@@ -1181,7 +1181,9 @@ static int subseq_entry(const double *shapelets, const int64_t *offsets, const i
     J.x.count = x->n;
     J.x.len = (int)x->n_timestep;
     need += subseq_workspace_bytes(J, scaled);
-    WB_TRY(ws.reserve(need));
+    const size_t filter_bytes =
+        !profile && subseq_dot_supported(J) ? subseq_dot_bytes(J, scaled) : 0;
+    WB_TRY(ws.reserve(need + filter_bytes, need));
     WB_TRY(stage(x, dim, ws, J.x));
     if (stop_sq) {
         WB_TAKE(dstop, double, ws, m);
@@ -1257,7 +1259,8 @@ static int subseq_entry(const double *shapelets, const int64_t *offsets, const i
     J.out_dist = out_on_device ? out_dist : ws.take<double>(n_out);
     J.out_idx = out_on_device ? out_idx : ws.take<int64_t>(n_out);
     if (!J.out_dist || !J.out_idx) return fail(WB_ENOMEM, "workspace reservation exceeded");
-    WB_TRY(launch_subseq(J, scaled, ws));
+    SubseqHost host{order, hlen, group_of, {}};
+    WB_TRY(launch_subseq(J, scaled, ws, host));
     if (!out_on_device) {
         WB_CUDA(cudaMemcpyAsync(out_dist, J.out_dist, n_out * 8, cudaMemcpyDeviceToHost, s));
         WB_CUDA(cudaMemcpyAsync(out_idx, J.out_idx, n_out * 8, cudaMemcpyDeviceToHost, s));

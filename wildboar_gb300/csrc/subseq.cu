@@ -144,6 +144,7 @@ subseq_scan_kernel(const SubseqJob J, const double *norm, const double *mean_tab
     unsigned int *tmax = reinterpret_cast<unsigned int *>(Tf + nt + (nt & 1));
     const bool filt = !SCALED && J.shp_f32 != nullptr;
     __shared__ int wqueue[kSubWarps][64];
+    if (J.redo && *J.redo == 0) return;
     for (int64_t b = blockIdx.x; b < J.x.count * chunks; b += gridDim.x) {
         const int64_t si = b / chunks;
         const int64_t c0 = (b - si * chunks) * J.chunk;
@@ -165,6 +166,7 @@ subseq_scan_kernel(const SubseqJob J, const double *norm, const double *mean_tab
         const float MT = filt ? __uint_as_float(*tmax) : 0.0f;
         for (int64_t sh = c0 + wid; sh < c1; sh += kSubWarps) {
             const int64_t idx = J.order ? J.order[sh] : sh;
+            if (J.kept && J.kept[si * J.m + idx] > 0) continue;
             const int L = (int)J.lengths[idx];
             const double *S = (SCALED ? norm : J.shapelets) + J.offsets[idx];
             const int nwin = nt - L + 1;
@@ -283,6 +285,7 @@ subseq_scaled_tiled_kernel(const SubseqJob J, const double *norm, const double *
     float *Zf = reinterpret_cast<float *>(Z + (size_t)J.max_len * 32);  // [max_len][32]
     unsigned int *zmax = reinterpret_cast<unsigned int *>(Zf + (size_t)J.max_len * 32);
     const bool filt = J.shp_f32 != nullptr;
+    if (J.redo && *J.redo == 0) return;
     for (int64_t b = blockIdx.x; b < J.x.count * J.n_chunks; b += gridDim.x) {
         const int64_t si = b / J.n_chunks;
         const int64_t ch = b - si * J.n_chunks;
@@ -321,6 +324,7 @@ subseq_scaled_tiled_kernel(const SubseqJob J, const double *norm, const double *
             const int w = base + lane;
             for (int q = wid; q < cnt; q += kSubWarps) {
                 const int64_t idx = J.order[first + q];
+                if (J.kept && J.kept[si * J.m + idx] > 0) continue;
                 const double *S = norm + J.offsets[idx];
                 const double bq = best[q];
                 double dist = INF;
@@ -372,6 +376,7 @@ subseq_scaled_tiled_kernel(const SubseqJob J, const double *norm, const double *
         __syncthreads();
         for (int q = threadIdx.x; q < cnt; q += kSubThreads) {
             const int64_t idx = J.order[first + q];
+            if (J.kept && J.kept[si * J.m + idx] > 0) continue;
             J.out_dist[si * J.m + idx] = sqrt(best[q]);
             J.out_idx[si * J.m + idx] = bidx[q];
         }
@@ -528,10 +533,14 @@ static int sub_grid(int64_t n, int block) {
     return (int)(g < 1 ? 1 : g);
 }
 
+// FP32 copies of the (normalised) shapelets and their max |value|
+static size_t scan_bytes(const SubseqJob &J) {
+    return align256((size_t)J.total_values * sizeof(float)) +
+           align256((size_t)J.m * sizeof(double)) + 1024;
+}
+
 size_t subseq_workspace_bytes(const SubseqJob &J, bool scaled) {
-    // FP32 copies of the (normalised) shapelets and their max |value|
-    const size_t filt = align256((size_t)J.total_values * sizeof(float)) +
-                        align256((size_t)J.m * sizeof(double));
+    const size_t filt = scan_bytes(J);
     if (!scaled) return filt;
     const size_t rows = J.paired ? (size_t)J.x.count : (size_t)J.n_groups * J.x.count;
     size_t tab = rows * J.win_stride * sizeof(double);
@@ -551,8 +560,9 @@ static int make_f32_copies(const SubseqJob &J, const double *src, Workspace &ws,
     return WB_OK;
 }
 
-int launch_subseq(const SubseqJob &J, bool scaled, Workspace &ws) {
+int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &host) {
     cudaStream_t s = ws.stream();
+    SubseqJob J = job;
     if (J.m == 0 || J.x.count == 0) return WB_OK;
     const int64_t chunks = (J.m + J.chunk - 1) / J.chunk;
     const int64_t blocks = J.x.count * chunks;
@@ -567,10 +577,16 @@ int launch_subseq(const SubseqJob &J, bool scaled, Workspace &ws) {
         double *norm = ws.take<double>((size_t)J.total_values);
         if (!mean_tab || !std_tab || !norm)
             return fail(WB_ENOMEM, "workspace reservation exceeded");
-        window_stats_kernel<<<sub_grid((int64_t)rows, 128), 128, 0, s>>>(J, mean_tab, std_tab);
-        WB_LAUNCH_CHECK("window_stats_kernel");
         shapelet_norm_kernel<<<(int)(J.m < 65535 ? J.m : 65535), 128, 0, s>>>(J, norm);
         WB_LAUNCH_CHECK("shapelet_norm_kernel");
+        if (subseq_dot_supported(J) &&
+            ws.remaining() >= subseq_dot_bytes(J, true) + scan_bytes(J)) {
+            WB_TRY(launch_subseq_dot(J, true, norm, mean_tab, std_tab, host.order, host.lengths,
+                                     host.group_of, host.uploads, ws));
+        } else {
+            window_stats_kernel<<<sub_grid((int64_t)rows, 128), 128, 0, s>>>(J, mean_tab, std_tab);
+            WB_LAUNCH_CHECK("window_stats_kernel");
+        }
         if (J.paired) {
             timer_begin("subseq_paired_kernel<scaled>", s);
             subseq_paired_kernel<true><<<sub_grid(J.x.count * 32, kSubThreads), kSubThreads, 0,
@@ -607,6 +623,10 @@ int launch_subseq(const SubseqJob &J, bool scaled, Workspace &ws) {
         timer_end(s);
         WB_LAUNCH_CHECK("subseq_paired_kernel");
     } else {
+        if (subseq_dot_supported(J) &&
+            ws.remaining() >= subseq_dot_bytes(J, false) + scan_bytes(J))
+            WB_TRY(launch_subseq_dot(J, false, nullptr, nullptr, nullptr, host.order, host.lengths,
+                                     host.group_of, host.uploads, ws));
         SubseqJob Jf = J;
         WB_TRY(make_f32_copies(J, J.shapelets, ws, Jf));
         // T (doubles), its float copy and the max |t| word

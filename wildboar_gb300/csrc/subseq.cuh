@@ -1,6 +1,9 @@
 // subseq.cuh -- job description of the subsequence scan kernels.
 #pragma once
 
+#include <memory>
+#include <vector>
+
 #include "elastic.cuh"
 
 namespace wb {
@@ -38,6 +41,10 @@ struct SubseqJob {
     // FP32 pre-filter of the minimum scans (set by launch_subseq)
     const float *shp_f32 = nullptr;      // packed shapelets (z-normalised when scaled)
     const float *shp_absmax = nullptr;   // (m,) max |value| of each shapelet, rounded up
+    // after the dot-product filter (subseq_dot.cu): the scan takes only pairs
+    // with kept[pair] <= 0, *redo of them
+    const int *kept = nullptr;
+    const unsigned long long *redo = nullptr;
     double *out_dist = nullptr;          // (x.count, m)
     int64_t *out_idx = nullptr;          // (x.count, m)
 };
@@ -48,7 +55,29 @@ size_t subseq_workspace_bytes(const SubseqJob &J, bool scaled);
 constexpr int kScaledTileMaxLen = 384;
 // shapelets of one length sharing the z-normalised window tiles of a block
 constexpr int kScaledTileChunk = 256;
-int launch_subseq(const SubseqJob &J, bool scaled, Workspace &ws);
+// Host arrays that asynchronous uploads read; to be kept until the stream is
+// synchronised.
+struct DotPlan;
+struct DotUploads {
+    std::shared_ptr<DotPlan> plan;
+};
+// What launch_subseq takes from the host besides the job, for the filter.
+struct SubseqHost {
+    const std::vector<int64_t> &order, &lengths;
+    const std::vector<int32_t> &group_of;
+    DotUploads uploads;
+};
+int launch_subseq(const SubseqJob &J, bool scaled, Workspace &ws, SubseqHost &host);
+
+// Dot-product filter of the minimum scans (subseq_dot.cu): settles most pairs
+// and sets J.kept / J.redo for the scan of the others.  Scaled: `norm` holds
+// the normalised shapelets; ex / ex2 receive the windows' running sums and, if
+// pairs are left, their means and standard deviations.
+bool subseq_dot_supported(const SubseqJob &J);
+size_t subseq_dot_bytes(const SubseqJob &J, bool scaled);
+int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex, double *ex2,
+                      const std::vector<int64_t> &order, const std::vector<int64_t> &hlen,
+                      const std::vector<int32_t> &group_of, DotUploads &keep, Workspace &ws);
 // paired jobs: every window's full sum at raw[pair * ld + window]
 int launch_subseq_profile(const SubseqJob &J, bool scaled, Workspace &ws, double *raw,
                           int64_t ld);
