@@ -439,17 +439,27 @@ def _is_arraylike(x):
 _GROUPED_STATS_OK = None
 
 
+def _row_stats(A):
+    """np.mean / np.std of the rows of a float64 array, by the steps of
+    numpy's _mean and _var without their per-call overhead."""
+    n = A.shape[1]
+    mean = np.add.reduce(A, axis=1) / n
+    D = A - mean[:, None]
+    np.multiply(D, D, out=D)
+    return mean, np.sqrt(np.add.reduce(D, axis=1) / n)
+
+
 def _grouped_stats_ok():
-    """Whether np.mean / np.std over the rows of a stacked (count, L) array
-    give, bit for bit, the values of one call per row (numpy reduces every
-    contiguous row with the same pairwise sum); checked once per process."""
+    """Whether _row_stats over the rows of a stacked (count, L) array gives,
+    bit for bit, the values of one np.mean / np.std call per row (numpy reduces
+    every contiguous row with the same pairwise sum); checked once per process."""
     global _GROUPED_STATS_OK
     if _GROUPED_STATS_OK is None:
         rng = np.random.default_rng(12345)
         ok = True
         for L in (1, 7, 8, 9, 16, 33, 100, 128, 129, 300, 513, 1024, 4097):
             A = rng.standard_normal((5, L)) * 1e3 + 7.0
-            m, sd = np.mean(A, axis=1), np.std(A, axis=1)
+            m, sd = _row_stats(A)
             for i in range(5):
                 ok &= bool(np.mean(A[i]).view(np.uint64) == m[i].view(np.uint64))
                 ok &= bool(np.std(A[i]).view(np.uint64) == sd[i].view(np.uint64))
@@ -463,31 +473,33 @@ def _shapelet_stats(shapelets, lens, packed=None, offs=None):
     gathered from the packed float64 copy when it is given)."""
     n = len(shapelets)
     # other dtypes reduce in their own precision: keep one call per shapelet
-    all_f64 = all(getattr(s, "dtype", None) == np.float64 for s in shapelets)
+    f64 = np.dtype(np.float64)
+    all_f64 = all(getattr(s, "dtype", None) == f64 for s in shapelets)
     if n < 64 or not all_f64 or not _grouped_stats_ok():
         means = np.array([np.mean(s) for s in shapelets], dtype=np.float64)
         stds = np.array([np.std(s) for s in shapelets], dtype=np.float64)
         return means, stds
     means = np.empty(n)
     stds = np.empty(n)
-    for L in np.unique(lens):
-        rows = np.flatnonzero(lens == L)
+    order = np.argsort(lens, kind="stable")
+    bounds = np.flatnonzero(np.diff(lens[order])) + 1
+    for rows in np.split(order, bounds):
+        L = lens[rows[0]]
         if packed is not None:
-            A = packed[offs[rows][:, None] + np.arange(L)[None, :]]
+            A = packed[offs[rows][:, None] + np.arange(L)]
         else:
             A = np.stack([np.ravel(shapelets[i]) for i in rows])
-        means[rows] = np.mean(A, axis=1)
-        stds[rows] = np.std(A, axis=1)
+        means[rows], stds[rows] = _row_stats(A)
     return means, stds
 
 
 def _pack_shapelets(shapelets, scaled):
-    lens = np.array([s.shape[0] for s in shapelets], dtype=np.int64)
+    lens = np.fromiter(map(len, shapelets), dtype=np.int64, count=len(shapelets))
     offs = np.zeros(len(shapelets), dtype=np.int64)
     if len(shapelets) > 1:
         offs[1:] = np.cumsum(lens)[:-1]
-    packed = np.ascontiguousarray(np.concatenate([np.ravel(s) for s in shapelets]),
-                                  dtype=np.float64)
+    flat = shapelets if all(s.ndim == 1 for s in shapelets) else [np.ravel(s) for s in shapelets]
+    packed = np.ascontiguousarray(np.concatenate(flat), dtype=np.float64)
     if scaled:
         # ScaledSubsequenceMetric.from_array: distance/_cdistance.pyx:453-467
         means, stds = _shapelet_stats(shapelets, lens, packed, offs)
@@ -540,10 +552,11 @@ def pairwise_subsequence_distance(y, x, *, dim=0, metric="euclidean", metric_par
     """
     y = _validate_subsequence(y)
     X = _as_input(x)
+    n_timestep = X.shape[-1]
     for s in y:
-        if s.shape[0] > X.shape[-1]:
+        if s.shape[0] > n_timestep:
             raise ValueError(
-                "Invalid subsequnce shape (%d > %d)" % (s.shape[0], X.shape[-1])
+                "Invalid subsequnce shape (%d > %d)" % (s.shape[0], n_timestep)
             )
     Metric_ = check_subsequence_metric(metric, scale=scale)
     metric_params = metric_params or {}
@@ -569,10 +582,11 @@ def paired_subsequence_distance(y, x, *, dim=0, metric="euclidean", metric_param
     n_dims = X.shape[1]
     if not 0 >= dim < n_dims:
         raise ValueError("The parameter dim must be 0 <= dim < n_dims")
+    n_timestep = X.shape[-1]
     for s in y:
-        if s.shape[0] > X.shape[-1]:
+        if s.shape[0] > n_timestep:
             raise ValueError(
-                "Invalid subsequnce shape (%d > %d)" % (s.shape[0], X.shape[-1])
+                "Invalid subsequnce shape (%d > %d)" % (s.shape[0], n_timestep)
             )
     Metric_ = check_subsequence_metric(metric, scale=scale)
     n_samples = X.shape[0] if X.ndim > 1 else 1
