@@ -203,90 +203,107 @@ size_t elastic_workspace_bytes(const ElasticJob &J) {
 }
 
 // --------------------------------------------------------------------------
-// Euclidean pairwise distance, tiled: a block computes a 64 x 64 tile of
-// (row series i, column series j) pairs, 4 x 4 per thread, staging 32 values
-// of each of the 64 + 64 series in shared memory per step.  Every pair's sum
-// still runs k = 0 .. L-1 in order with the reference's operations (v = y_k -
+// Euclidean pairwise distance, tiled: a block computes a TILE x TILE tile of
+// (row series i, column series j) pairs, PER x PER pairs per thread, staging 32
+// values of each of the 2 TILE series in shared memory per step.  Every pair's
+// sum runs k = 0 .. L-1 in order with the reference's operations (v = y_k -
 // x_k, dist = dist + v * v; euclidean_distance with one window,
-// distance/_metric.pyx:654-682), so results are bit-identical; the tiling
-// only replaces the per-lane strided row reads of the thread-per-pair kernel
-// (whose speed depended on the L1 carve-out) by shared-memory reuse.
-constexpr int kEuT = 64, kEuK = 32;
+// distance/_metric.pyx:654-682), so results are bit-identical whatever the
+// tile.
+//
+// Bound: the FP64 pipe (3 operations per value; an FP64 instruction takes 21
+// cycles of an SM, so even one pair per thread reads shared memory far below
+// its rate) and how evenly the tiles fill the SMs.  One block per tile, so the
+// scheduler balances them.  Tiles of 32 (2 x 2 pairs per thread) where they
+// give every SM several blocks, else 16, else 8 with 64 threads, where the
+// chain of 3 dependent operations per value (71 cycles each) is the bound:
+// 2000 x 1500 series of 700 15.2 -> 12.7 ms (tiles of 64 left 5 or 6 to an SM),
+// 97 x 60 of 866 3.42 -> 0.39 ms (two tiles of 64).
+constexpr int kEuK = 32;
 
-__global__ void __launch_bounds__(256) euclid_tiled_kernel(const ElasticJob J) {
-    __shared__ double xs[kEuK][kEuT + 1];
-    __shared__ double ys[kEuK][kEuT + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+template <int TILE, int PER>
+__global__ void __launch_bounds__((TILE / PER) * (TILE / PER))
+euclid_tiled_kernel(const ElasticJob J) {
+    constexpr int SIDE = TILE / PER, THREADS = SIDE * SIDE;
+    __shared__ double xs[kEuK][TILE + 1];
+    __shared__ double ys[kEuK][TILE + 1];
+    const int tx = threadIdx.x % SIDE, ty = threadIdx.x / SIDE;
     const int L = J.rows.len;
-    const int64_t tiles_c = (J.cols.count + kEuT - 1) / kEuT;
-    const int64_t tiles_r = (J.rows.count + kEuT - 1) / kEuT;
-    for (int64_t t = blockIdx.x; t < tiles_r * tiles_c; t += gridDim.x) {
-        const int64_t tr = t / tiles_c, tc = t - (t / tiles_c) * tiles_c;
-        if (J.mode == PM_UPPER && tr > tc) continue;  // the mirror tile fills it
-        const int64_t r0 = tr * kEuT, c0 = tc * kEuT;
-        double acc[4][4];
+    const int64_t tiles_c = (J.cols.count + TILE - 1) / TILE;
+    const int64_t tr = blockIdx.x / tiles_c, tc = blockIdx.x - tr * tiles_c;
+    if (J.mode == PM_UPPER && tr > tc) return;  // the mirror tile fills it
+    const int64_t r0 = tr * TILE, c0 = tc * TILE;
+    double acc[PER][PER];
 #pragma unroll
-        for (int a = 0; a < 4; a++)
+    for (int a = 0; a < PER; a++)
 #pragma unroll
-            for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-        for (int k0 = 0; k0 < L; k0 += kEuK) {
-            __syncthreads();
-            for (int e = threadIdx.x; e < kEuK * kEuT; e += 256) {
-                const int s = e / kEuK, k = e - (e / kEuK) * kEuK;
-                const int64_t ri = r0 + s, ci = c0 + s;
-                double xv = 0.0, yv = 0.0;
-                if (k0 + k < L) {
-                    if (ri < J.rows.count) xv = J.rows.base[ri * J.rows.stride + k0 + k];
-                    if (ci < J.cols.count) yv = J.cols.base[ci * J.cols.stride + k0 + k];
-                }
-                xs[k][s] = xv;
-                ys[k][s] = yv;
+        for (int b = 0; b < PER; b++) acc[a][b] = 0.0;
+    for (int k0 = 0; k0 < L; k0 += kEuK) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < kEuK * TILE; e += THREADS) {
+            const int s = e / kEuK, k = e - (e / kEuK) * kEuK;
+            const int64_t ri = r0 + s, ci = c0 + s;
+            double xv = 0.0, yv = 0.0;
+            if (k0 + k < L) {
+                if (ri < J.rows.count) xv = J.rows.base[ri * J.rows.stride + k0 + k];
+                if (ci < J.cols.count) yv = J.cols.base[ci * J.cols.stride + k0 + k];
             }
-            __syncthreads();
-            const int kn = L - k0 < kEuK ? L - k0 : kEuK;
-            for (int k = 0; k < kn; k++) {
-                double xv[4], yv[4];
-#pragma unroll
-                for (int a = 0; a < 4; a++) xv[a] = xs[k][ty + 16 * a];
-#pragma unroll
-                for (int b = 0; b < 4; b++) yv[b] = ys[k][tx + 16 * b];
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        double v = yv[b];
-                        v = v - xv[a];
-                        acc[a][b] = acc[a][b] + v * v;
-                    }
-            }
+            xs[k][s] = xv;
+            ys[k][s] = yv;
         }
+        __syncthreads();
+        const int kn = L - k0 < kEuK ? L - k0 : kEuK;
+#pragma unroll 4
+        for (int k = 0; k < kn; k++) {
+            double xv[PER], yv[PER];
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
-            const int64_t i = r0 + ty + 16 * a;
-            if (i >= J.rows.count) continue;
+            for (int a = 0; a < PER; a++) xv[a] = xs[k][ty + SIDE * a];
 #pragma unroll
-            for (int b = 0; b < 4; b++) {
-                const int64_t j = c0 + tx + 16 * b;
-                if (j >= J.cols.count) continue;
-                if (J.mode == PM_UPPER) {
-                    if (i >= j) continue;
-                    const double d = J.all_zero ? 0.0 : sqrt(acc[a][b]);
-                    J.out[i * J.out_ld + j] = d;
-                    J.out[j * J.out_ld + i] = d;
-                } else {
-                    J.out[i * J.out_ld + j] = J.all_zero ? 0.0 : sqrt(acc[a][b]);
+            for (int b = 0; b < PER; b++) yv[b] = ys[k][tx + SIDE * b];
+#pragma unroll
+            for (int a = 0; a < PER; a++)
+#pragma unroll
+                for (int b = 0; b < PER; b++) {
+                    double v = yv[b];
+                    v = v - xv[a];
+                    acc[a][b] = acc[a][b] + v * v;
                 }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < PER; a++) {
+        const int64_t i = r0 + ty + SIDE * a;
+        if (i >= J.rows.count) continue;
+#pragma unroll
+        for (int b = 0; b < PER; b++) {
+            const int64_t j = c0 + tx + SIDE * b;
+            if (j >= J.cols.count) continue;
+            if (J.mode == PM_UPPER) {
+                if (i >= j) continue;
+                const double d = J.all_zero ? 0.0 : sqrt(acc[a][b]);
+                J.out[i * J.out_ld + j] = d;
+                J.out[j * J.out_ld + i] = d;
+            } else {
+                J.out[i * J.out_ld + j] = J.all_zero ? 0.0 : sqrt(acc[a][b]);
             }
         }
     }
 }
 
 static int launch_euclid_tiled(const ElasticJob &J, cudaStream_t s) {
-    const int64_t tiles = ((J.rows.count + kEuT - 1) / kEuT) * ((J.cols.count + kEuT - 1) / kEuT);
-    const int64_t cap = (int64_t)device_info().sm_count * 8;
-    const int grid = (int)(tiles < cap ? tiles : cap);
+    auto tiles = [&](int64_t t) {
+        return ((J.rows.count + t - 1) / t) * ((J.cols.count + t - 1) / t);
+    };
+    const int64_t sms = device_info().sm_count;
+    if (tiles(32) > 0x7fffffffLL)
+        return fail(WB_EINVAL, "too many pairs for one call");
     timer_begin("euclid_tiled_kernel", s);
-    euclid_tiled_kernel<<<grid, 256, 0, s>>>(J);
+    if (tiles(32) >= 8 * sms)
+        euclid_tiled_kernel<32, 2><<<(unsigned)tiles(32), 256, 0, s>>>(J);
+    else if (tiles(16) >= 2 * sms)
+        euclid_tiled_kernel<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(J);
+    else
+        euclid_tiled_kernel<8, 1><<<(unsigned)tiles(8), 64, 0, s>>>(J);
     timer_end(s);
     WB_LAUNCH_CHECK("euclid_tiled_kernel");
     return WB_OK;
