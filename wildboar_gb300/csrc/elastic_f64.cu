@@ -189,7 +189,8 @@ static ElasticPlan plan_elastic(const ElasticJob &J) {
 // cells of each strip's ragged band edges; measured on GB300 (dtw, L = 512)
 // the ring kernel wins for shared-memory rings (r = 0.1: 171 vs 152 GCUPS)
 // and the strip kernel for global rings (r = 1: 167 vs 128 GCUPS; lcss 168 vs
-// 134, erp 127 vs 115, msm 64 vs 58), except twe (53 vs 57).
+// 134, erp 127 vs 115, msm 64 vs 58), except twe (53 vs 57).  erp, msm and twe
+// over the full band come here only where elastic_wave.cu has no workspace.
 static bool use_strip_f64(const ElasticJob &J) {
     if (!strip_supported(J)) return false;
     if (strip_forced()) return true;
@@ -313,6 +314,7 @@ int launch_elastic(const ElasticJob &job, Workspace &ws, bool guided) {
     ElasticJob J = job;
     if (J.rows.count == 0 || J.cols.count == 0) return WB_OK;
     if (guided) {
+        if (wave_supported(J) && ws.remaining() >= wave_bytes(J)) return launch_wave(J, ws);
         // then the full recurrence over the pairs it left, in the workspace
         // that it leaves
         unsigned long long *pending = nullptr;

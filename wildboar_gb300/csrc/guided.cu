@@ -1088,6 +1088,10 @@ static size_t plan_bytes(const Plan &p) {
 
 size_t guided_workspace_bytes(const ElasticJob &J) {
     if (bit_edit_supported(J)) return bit_edit_bytes(J);
+    if (wave_supported(J)) {
+        const size_t own = wave_bytes(J), other = elastic_workspace_bytes(J);
+        return own > other ? own - other : 0;
+    }
     return plan_bytes(plan_guided(J, SIZE_MAX));
 }
 

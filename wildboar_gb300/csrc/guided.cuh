@@ -76,6 +76,12 @@ size_t bit_edit_bytes(const ElasticJob &job);
 int launch_bit_edit(const ElasticJob &job, Workspace &ws, size_t leave,
                     unsigned long long **pending);
 
+// erp, msm and twe over the full band (elastic_wave.cu), the whole job in place
+// of the ring or strip kernel.
+bool wave_supported(const ElasticJob &job);
+size_t wave_bytes(const ElasticJob &job);
+int launch_wave(const ElasticJob &job, Workspace &ws);
+
 // The guided evaluation in two steps, for a caller that runs it over several
 // lists of pairs: buffers and float / fixed-point series of the job (the grid
 // holds at most max_pairs pairs), then a run per list.  ctx.args.prep is null
