@@ -224,7 +224,8 @@ typedef struct wb_dtw32 {
     const float *weights;      /* wdtw weights (length >= max length) or NULL */
     int32_t strip;             /* rows per register strip: 4, 8, 16, 24, 32 (0 = 16) */
     int32_t block;             /* threads per block (0 = 128) */
-    int32_t grid;              /* persistent grid (0 = occupancy x SMs) */
+    int32_t grid;              /* persistent grid (0 = occupancy x SMs; few dtw items then
+                                  take several lanes each, whatever strip and block) */
 } wb_dtw32;
 
 /* dtw distance of every item: out[t] = sqrt(cost), out_cost[t] = cost (or NULL) */

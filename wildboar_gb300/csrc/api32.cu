@@ -84,6 +84,7 @@ int dtw32_plan(const wb_dtw32 *q, bool backward, Dtw32Job &J, size_t &bytes) {
     J.weights = q->weights;
     J.grid = grid;
     J.block = block;
+    if (!backward && q->grid <= 0) dtw32_wave_plan(J);
     const int64_t nth = (int64_t)grid * block;
     size_t ring_bytes = align256((size_t)J.ring_cols * nth * sizeof(float2));
     size_t dir_bytes = 0;

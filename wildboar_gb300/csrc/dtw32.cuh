@@ -45,6 +45,8 @@ struct Dtw32Job {
     int seg_strips = 1;           // strips per segment (backward)
     unsigned long long *queue = nullptr;  // work counter (persistent kernel)
     int grid = 0, block = 0;
+    int wave = 0;                 // > 0: blocks of the lanes-per-item forward
+    int wave_rows = 0;            // its rows per strip
 };
 
 // Kept directions of a differentiable call (see dtw32.cu): one region of
@@ -64,6 +66,7 @@ int dtw32_keep_walk(const Dtw32Job &J, const DirKeep &D, const double *dist, cud
 int dtw32_keep_blocks_per_sm(bool walk, bool weighted);
 int dtw32_backward(const Dtw32Job &J, cudaStream_t s);
 int dtw32_blocks_per_sm(int strip, bool weighted, bool backward, int block);
+void dtw32_wave_plan(Dtw32Job &J);
 int launch_grid_to_matrix(const double *in, int64_t nx, int64_t ny, int upper, double *out,
                           cudaStream_t s);
 int dtw32_plan(const wb_dtw32 *q, bool backward, Dtw32Job &J, size_t &bytes);

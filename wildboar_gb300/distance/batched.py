@@ -194,7 +194,10 @@ class Autotuner:
         out = torch.empty(sx.numel(), dtype=torch.float64, device=x.device)
         for strip, block in [(s_, b_) for s_ in STRIPS for b_ in BLOCKS]:
             kw = dict(r=r, x_lengths=x_lengths, y_lengths=y_lengths, item_x=sx,
-                      item_y=sy, weights=weights, strip=strip, block=block)
+                      item_y=sy, weights=weights, strip=strip, block=block,
+                      # one thread per item, which the tile is for: a small
+                      # sample would take lanes per item
+                      grid=-(-sx.numel() // block))
             dtw32(x, y, out=out, **kw)  # warm-up (workspace growth)
             torch.cuda.synchronize()
             t0 = time.perf_counter()
