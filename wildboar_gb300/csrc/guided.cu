@@ -57,10 +57,11 @@
 // kGuidedPending until launch_elastic's second pass over exactly those pairs.
 //
 // Measured on one GB300 (full recurrence -> guided): dtw r = 0.1, 1000 x 1000,
-// length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 8.6
-// ms; wdtw r = 1, 500 x 403, length 256: 107 -> 9.5 ms.  Of the first, the
-// sweep takes a fourth, the walk a fifth and the FP64 part half (its iterations
-// wait for the widest of 32 pairs).
+// length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.3
+// ms; wdtw r = 1, 500 x 403, length 256: 107 -> 9.0 ms.  Of the first, the
+// sweep takes a third, the walk a fourth and the FP64 part two fifths (2100
+// iterations for the 890 cells of a pair: lanes wait for the turn's longest
+// word).
 
 #include "guided.cuh"
 
@@ -139,6 +140,8 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
         if (dsq) dsq += at;
         float *low = row ? D.xl : D.yl;
         if (low) low += at;
+        double *as = row ? D.xd : D.yd;
+        if (as) as += at;
         const int lead = row ? 3 : 0;
         const int total = (int)(row ? D.xs : D.ys);
         const float pad = row ? WB_FLT_INF : -WB_FLT_INF;
@@ -148,8 +151,10 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
             const int e = i - lead;
             float v = pad, rest = 0.0f;
             int q = 0;
+            double given = 0.0;
             if (e >= 0 && e < S.len) {
-                const double c = (src[e] - centre) * scale;
+                given = src[e];
+                const double c = (given - centre) * scale;
                 v = (float)c;
                 rest = (float)(c - (double)v);
                 q = __double2int_rn(c * (double)kFixOne);
@@ -160,6 +165,7 @@ guided_convert_kernel(const SeriesSet rows, const SeriesSet cols, const GuidedSe
             dst[i] = v;
             if (dsq) dsq[i] = q;
             if (low) low[i] = rest;
+            if (as) as[i] = given;
         }
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         lo = __reduce_min_sync(0xffffffffu, lo);
@@ -634,10 +640,8 @@ template <int KIND, int S, bool FIX>
 __device__ __forceinline__ int collect(const GuidedArgs &A, const Band &B, const PairData &D,
                                        float e, bool live, int64_t gt, int &row0) {
     constexpr int W64 = S * S / 64;  // mask words of a block
-    constexpr int EW = 2 * W64 + 1;  // list words of a block: position, mask
     constexpr unsigned SM = (1u << S) - 1u;
     const unsigned FULL = 0xffffffffu;
-    const int64_t nth = A.nth;
     const unsigned au = guided_sweep<KIND, S, FIX>(A, B, D, gt);
 
     // the bound (file header); sqrt(A_max) <= sqrt(A + K) (1 + 2^-22) + 2 e sqrt(K)
@@ -688,13 +692,13 @@ __device__ __forceinline__ int collect(const GuidedArgs &A, const Band &B, const
                 mask[q * S / 64] |= (uint64_t)r << (64 - S - (q * S) % 64);
             }
             carry = from;
-            uint32_t *ent = A.list + (int64_t)idx * EW * nth + gt;
-            ent[0] = ((uint32_t)s << 16) | (uint32_t)b;
+            // (the last word first, like the blocks)
+            uint4 *ent = A.list + (gt * A.list_cap + idx) * W64;
+            const uint32_t pos = ((uint32_t)s << 16) | (uint32_t)b;
 #pragma unroll
-            for (int w = 0; w < W64; w++) {
-                ent[(1 + 2 * w) * nth] = (uint32_t)(mask[w] >> 32);
-                ent[(2 + 2 * w) * nth] = (uint32_t)mask[w];
-            }
+            for (int w = 0; w < W64; w++)
+                ent[W64 - 1 - w] =
+                    make_uint4(pos, (uint32_t)(mask[w] >> 32), (uint32_t)mask[w], 0u);
             idx++;
             if (carry != 0 || slo < c0) {
                 b--;
@@ -726,11 +730,14 @@ __device__ __forceinline__ int collect(const GuidedArgs &A, const Band &B, const
 // a lane whose word is done takes the next one after the warp's turn of up to
 // kCellsPerTurn cells, so the code that takes a word runs once per turn for
 // the whole warp.  Longer turns idle more lanes, shorter ones take words more
-// often: turns of 2, 3, 4, 6 and 12 cells ran 1000 x 1000 pairs of length 512,
-// r = 0.1, in 49, 46, 43, 42 and 40 ms.
+// often: turns of 4, 6, 8 and 12 cells ran 1000 x 1000 pairs of length 512, r =
+// 0.1 (other random walks), in 38.5, 38.2, 37.2 and 36.9 ms.
 // Taking a word stages its rows, columns and the cells above it in shared
 // memory (all loads in flight at once); a cell then waits for shared memory
-// and the FP64 pipe only.  (An FP64 instruction takes 71 cycles of a warp and
+// and the FP64 pipe only.  A lane's lists, bottom rows and series lie one after
+// the other and are read 16 bytes at a time: with every value of a lane in a
+// sector of its own (interleaved by thread) taking a word was 55 % of this
+// step's time, now 37 %, and that call took 40.4 instead of 36.9 ms.  (An FP64 instruction takes 71 cycles of a warp and
 // 21 of the SM whatever its active lanes, so what counts is the number of
 // iterations: going through the strips in step, with the waits for the widest
 // lane in each strip, measured 4.9 against 3.3 million cycles per 32 pairs of
@@ -746,21 +753,34 @@ struct Stage {
     double top[C + 1][kThreads];      // the row above, from the column left of the word
 };
 
+// Bits of a word's bottom row, column q in bit q.
+template <int S>
+__device__ __forceinline__ unsigned bottom_bits(uint64_t word) {
+    constexpr int C = 64 / S;
+    if constexpr (S == 8) {
+        // bit 8 i to bit 56 + i: the products of distinct bits do not collide
+        const uint64_t g = (word & 0x0101010101010101ull) * 0x0102040810204080ull;
+        return __brev((unsigned)(g >> 56)) >> 24;
+    }
+    unsigned bits = 0;
+#pragma unroll
+    for (int q = 0; q < C; q++) bits |= (unsigned)((word >> (64 - S - q * S)) & 1u) << q;
+    return bits;
+}
+
 template <int KIND, int S>
 __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__restrict__ X,
                                            const double *__restrict__ Y, int count, int row0,
                                            int64_t gt, Stage<S> &St) {
     constexpr int W64 = S * S / 64;
-    constexpr int EW = 2 * W64 + 1;
     constexpr int C = 64 / S;
     constexpr unsigned SM = (1u << S) - 1u;
-    const int64_t nth = A.nth;
+    constexpr unsigned TM = (1u << (C + 1)) - 1u;
     const double INF = WB_DBL_INF;
     const ElasticJob &J = A.J;
     const int tid = threadIdx.x;
-    const int n = J.rows.len, m = J.cols.len;
-    double *brow = A.brow + gt;  // [strip parity][column]: bottom rows
-    const int64_t mp = A.brow_cols;
+    double *brow = A.brow + gt * 2 * A.brow_cols;  // [strip parity][column]: bottom rows
+    const uint4 *list = A.list + gt * A.list_cap * W64;
     if (count > 0) {
         const double x0 = X[0];
         double acc = 0.0;
@@ -769,88 +789,92 @@ __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__
             double cst = v * v;
             if (KIND == K_WDTW) cst = cst * __ldg(J.weights + imax(c - 1, 0));
             acc = c == 0 ? cst : acc + cst;
-            brow[c * nth] = acc;
+            brow[c] = acc;
         }
     }
-    // list entry of the leftmost block, and first and last block, of the strip
-    // above and of the current one
-    int pfirst = 0, pblock = 0, plast = -1;
-    int cfirst = 0, cblock = 0, clast = 0;
+    // Of the strip above and of the current one: the words' columns, the first
+    // word, and the collected cells of the bottom row (of 64 columns; the masks
+    // are read again for wider strips).
+    int pcol = 0, pend = 0, pfirst = 0;
+    int ccol = 0, cend = 0, cfirst = 0;
+    uint64_t pbits = 0, cbits = 0;
     int cur = -1, i0 = 0, cw = 0;
     double *below = brow;
     uint64_t M = 0, LM = 0, todo = 0;
     unsigned tops = 0;  // bit q: cell (i0 - 1, cw - 1 + q) is collected
     double last = 0.0, last_old = 0.0;
     int left = imax(count, 0) * W64;  // mask words to go
-    auto entry = [&](int e) { return A.list + (int64_t)e * EW * nth + gt; };
-    auto word = [&](int j) -> uint64_t {  // word of the j-th step from the end
-        const uint32_t *p = entry(j / W64) + (1 + 2 * (W64 - 1 - j % W64)) * nth;
-        return ((uint64_t)p[0] << 32) | p[nth];
-    };
     // the next word, loaded while the current one is worked on
-    uint32_t nh = left > 0 ? *entry((left - 1) / W64) : 0u;
-    uint64_t nM = left > 0 ? word(left - 1) : 0u;
+    uint4 next = left > 0 ? list[left - 1] : make_uint4(0u, 0u, 0u, 0u);
     while (__any_sync(0xffffffffu, todo != 0 || left > 0)) {
         if (todo == 0 && left > 0) {
             left--;
-            const uint32_t h = nh;
-            unsigned lm = (unsigned)(M & SM);  // collected rows of the column to the left
-            M = nM;
-            if (left > 0) {
-                nh = *entry((left - 1) / W64);
-                nM = word(left - 1);
-            }
+            const uint4 E = next;
+            if (left > 0) next = list[left - 1];
             const int w = W64 - 1 - left % W64;
-            const int bs = (int)(h >> 16), bb = (int)(h & 0xffffu);
+            const int bs = (int)(E.x >> 16), bb = (int)(E.x & 0xffffu);
+            unsigned lm = (unsigned)(M & SM);  // collected rows of the column to the left
+            M = ((uint64_t)E.y << 32) | E.z;
+            cw = bb * S + w * C;
+#pragma unroll
+            for (int q = 0; q < C; q += 2) {
+                const double2 v = __ldg(reinterpret_cast<const double2 *>(Y + cw + q));
+                St.y[q][tid] = v.x;
+                St.y[q + 1][tid] = v.y;
+            }
             if (bs != cur) {
+                pcol = ccol;
+                pend = cend;
                 pfirst = cfirst;
-                pblock = cblock;
-                plast = clast;
-                cfirst = left / W64;
-                cblock = bb;
+                pbits = cbits;
+                ccol = cw;
+                cfirst = left;
+                cbits = 0;
                 lm = 0;
                 i0 = 1 + bs * S;
-                below = brow + (int64_t)((bs + 1) & 1) * mp * nth;
+                below = brow + ((bs + 1) & 1) * A.brow_cols;
 #pragma unroll
-                for (int k = 0; k < S; k++) St.x[k][tid] = X[imin(i0 + k, n - 1)];
+                for (int k = 0; k < S; k += 2) {
+                    const double2 v = __ldg(reinterpret_cast<const double2 *>(X + i0 + k));
+                    St.x[k][tid] = v.x;
+                    St.x[k + 1][tid] = v.y;
+                }
             }
-            clast = bb;
-            cw = bb * S + w * C;
+            cend = cw + C;
+            if (cw - ccol < 64) cbits |= (uint64_t)bottom_bits<S>(M) << (cw - ccol);
             LM = (M >> S) | ((uint64_t)lm << (64 - S));
             todo = M;
-#pragma unroll
-            for (int q = 0; q < C; q++) St.y[q][tid] = __ldg(Y + imin(cw + q, m - 1));
-            // the cells above the word: row 0, or the bottom bits of the strip
-            // above's blocks (consecutive entries, leftmost block last)
-            tops = 0;
+            // the cells above the word: row 0, or the bottom row of the strip
+            // above
             if (bs == 0) {
-#pragma unroll
-                for (int q = 0; q <= C; q++)
-                    if (cw - 1 + q >= 0 && cw - 1 + q <= row0) tops |= 1u << q;
+                const int cells = row0 - cw + 2;
+                tops = cells <= 0 ? 0u : cells > C ? TM : (1u << cells) - 1u;
+                if (cw == 0) tops &= ~1u;
+            } else if (pend - pcol <= 64) {
+                const int sh = cw - 1 - pcol;
+                tops = sh >= 64 || sh < -C ? 0u
+                                           : (unsigned)(sh >= 0 ? pbits >> sh : pbits << -sh) & TM;
             } else {
-                uint32_t bits[2] = {0, 0};  // of the word's block and the one to its left
+                tops = 0;
 #pragma unroll
-                for (int o = 0; o < 2; o++) {
-                    const int blk = bb - o;
-                    if (blk < pblock || blk > plast || (o == 1 && w > 0)) continue;
-                    const uint32_t *p = entry(pfirst - (blk - pblock)) + nth;
-                    // bottom row: the lowest bit of every column
-                    const int pw = o == 0 ? w : W64 - 1;
-                    const uint64_t B = ((uint64_t)p[2 * pw * nth] << 32) | p[(2 * pw + 1) * nth];
-#pragma unroll
-                    for (int q = 0; q < C; q++)
-                        bits[o] |= (uint32_t)((B >> (64 - S - q * S)) & 1u) << q;
-                    if (o == 0 && w > 0) {  // the column left of the word, same block
-                        const uint32_t *p1 = p + 2 * (w - 1) * nth;
-                        bits[1] = (p1[nth] & 1u) << (C - 1);
-                    }
+                for (int o = 0; o < 2; o++) {  // the word's columns, those to the left
+                    const int col = cw - o * C;
+                    if (col < pcol || col >= pend) continue;
+                    const uint4 v = list[pfirst - (col - pcol) / C];
+                    const unsigned bits = bottom_bits<S>(((uint64_t)v.y << 32) | v.z);
+                    tops |= o == 0 ? bits << 1 : bits >> (C - 1);
                 }
-                tops = (bits[0] << 1) | (bits[1] >> (C - 1));
             }
-            const double *above = brow + (int64_t)(bs & 1) * mp * nth;
+            const double *above = brow + (bs & 1) * A.brow_cols + cw;
+            if (tops > 1u) {
 #pragma unroll
-            for (int q = 0; q <= C; q++)
-                if ((tops >> q) & 1u) St.top[q][tid] = above[(int64_t)(cw - 1 + q) * nth];
+                for (int q = 0; q < C; q += 2) {
+                    const double2 v = *reinterpret_cast<const double2 *>(above + q);
+                    St.top[q + 1][tid] = v.x;
+                    St.top[q + 2][tid] = v.y;
+                }
+            }
+            if (tops & 1u) St.top[0][tid] = above[-1];
             cur = bs;
         }
 #pragma unroll 1
@@ -876,7 +900,7 @@ __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__
             St.value[k][tid] = nv;
             last = nv;
             last_old = old;
-            if (k == S - 1) below[(int64_t)(cw + q) * nth] = nv;
+            if (k == S - 1) below[cw + q] = nv;
         }
     }
     return last;
@@ -973,8 +997,8 @@ guided_pairs_kernel(const GuidedArgs A) {
 
         double value = 0.0;
         if (__any_sync(FULL, count > 0))
-            value = evaluate<KIND, S>(A, J.rows.base + rs * J.rows.stride,
-                                      J.cols.base + cs * J.cols.stride, count, row0, gt, stage);
+            value = evaluate<KIND, S>(A, A.xd + rs * A.xs + 3, A.yd + cs * A.ys, count, row0, gt,
+                                      stage);
         if (active) {
             const double res = count > 0 ? sqrt(value) : __longlong_as_double(kGuidedPending);
             if (J.mode == PM_PAIRED) {
@@ -1044,11 +1068,11 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
         p.ys = round_up(m, 16);
         p.woff = (int)round_up(n + 2 * S, 4);
         p.wlen = J.kind == K_WDTW ? (int)round_up(p.woff + m + 2 * S, 4) : 0;
-        const int EW = S * S / 32 + 1;
         p.thread_bytes = (size_t)(ns + 1) * p.groups * 16 + (size_t)ns * p.blocks * S * 4 +
-                         (size_t)p.list_cap * EW * 4 + (size_t)2 * p.brow_cols * 8;
+                         (size_t)p.list_cap * (S * S / 64) * 16 + (size_t)2 * p.brow_cols * 8;
         p.shared_bytes = 3 * align256(J.rows.count * p.xs * 4) +
                          3 * align256(J.cols.count * p.ys * 4) +
+                         align256(J.rows.count * p.xs * 8) + align256(J.cols.count * p.ys * 8) +
                          align256(J.rows.count * sizeof(GuidedRange)) +
                          align256(J.cols.count * sizeof(GuidedRange)) +
                          align256((size_t)imax(p.wlen, 1) * 4) + align256(sizeof(GuidedPrep)) +
@@ -1144,12 +1168,14 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     WB_TAKE(yl, float, ws, J.cols.count * p.ys);
     WB_TAKE(xq, int, ws, J.rows.count * p.xs);
     WB_TAKE(yq, int, ws, J.cols.count * p.ys);
+    WB_TAKE(xd, double, ws, J.rows.count * p.xs);
+    WB_TAKE(yd, double, ws, J.cols.count * p.ys);
     WB_TAKE(xr, GuidedRange, ws, J.rows.count);
     WB_TAKE(yr, GuidedRange, ws, J.cols.count);
     WB_TAKE(wext, float, ws, imax(p.wlen, 1));
     WB_TAKE(ckrow, uint4, ws, (size_t)(ns + 1) * p.groups * nth);
     WB_TAKE(ckcol, uint4, ws, (size_t)ns * p.blocks * (p.S / 4) * nth);
-    WB_TAKE(list, uint32_t, ws, (size_t)p.list_cap * (p.S * p.S / 32 + 1) * nth);
+    WB_TAKE(list, uint4, ws, (size_t)p.list_cap * (p.S * p.S / 64) * nth);
     WB_TAKE(brow, double, ws, (size_t)2 * p.brow_cols * nth);
     A.prep = prep;
     A.xf = xf;
@@ -1158,6 +1184,8 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     A.yl = yl;
     A.xq = xq;
     A.yq = yq;
+    A.xd = xd;
+    A.yd = yd;
     A.xr = xr;
     A.yr = yr;
     A.wext = wext;
@@ -1172,6 +1200,8 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     S.yl = yl;
     S.xq = xq;
     S.yq = yq;
+    S.xd = xd;
+    S.yd = yd;
     S.xs = p.xs;
     S.ys = p.ys;
     S.xr = xr;

@@ -36,6 +36,7 @@ struct GuidedArgs {
     const float *xf = nullptr, *yf = nullptr;  // centred, scaled, padded float series
     const float *xl = nullptr, *yl = nullptr;  // their rests
     const int *xq = nullptr, *yq = nullptr;    // the same in fixed point
+    const double *xd = nullptr, *yd = nullptr;  // the series as given
     int64_t xs = 0, ys = 0;                    // their strides
     const GuidedRange *xr = nullptr, *yr = nullptr;
     const float *wext = nullptr;  // wdtw: weight of i - j at woff + (j - i)
@@ -51,8 +52,9 @@ struct GuidedArgs {
     int64_t nth = 0;
     uint4 *ckrow = nullptr;   // [strip + 1][group of 4 columns] bottom rows
     uint4 *ckcol = nullptr;   // [strip][block][S / 4] last columns of the blocks
-    uint32_t *list = nullptr;  // [entry][word] collected blocks
-    double *brow = nullptr;    // [2][column] FP64 bottom rows of two strips
+    // per resident thread, one after the other
+    uint4 *list = nullptr;    // [block][word] collected blocks: position, mask (high, low)
+    double *brow = nullptr;   // [2][column] FP64 bottom rows of two strips
     int groups = 0, blocks = 0, list_cap = 0, brow_cols = 0;
 };
 
@@ -62,6 +64,7 @@ struct GuidedSeries {
     float *xf = nullptr, *yf = nullptr;
     float *xl = nullptr, *yl = nullptr;  // the floats' rests
     int *xq = nullptr, *yq = nullptr;
+    double *xd = nullptr, *yd = nullptr;  // the values as given, padded with 0
     int64_t xs = 0, ys = 0;  // strides; row series start at element 3
     GuidedRange *xr = nullptr, *yr = nullptr;
     float *wext = nullptr;
