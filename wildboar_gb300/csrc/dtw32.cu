@@ -35,6 +35,7 @@
 
 #include "dtw32.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace wb {
@@ -349,323 +350,6 @@ __global__ void __launch_bounds__(256) dtw32_forward_kernel(const Dtw32Job J) {
             J.out[t] = res;
         }
     }
-}
-
-// ---------------------------------------------------------------------------
-// Forward of few items (dtw): the strips of an item on several lanes.
-//
-// With one thread per item a batch of some thousand items leaves most warp
-// slots empty, and the call takes as long as its longest item on a warp by
-// itself.  Here G = 8, 16 or 32 lanes share an item: lane g sweeps strips g, g +
-// G, .. of S rows, a pair of columns per step, one pair behind lane g - 1,
-// whose bottom cells it takes by shuffle; lane 0 takes them from a row in
-// global memory that lane G - 1 wrote in the round before.  A lane keeps to its
-// strip's columns; round q + 1 starts `delta` steps after round q, the least
-// after which every lane is done with its strip and lane 0's row is written.
-// The cells' operations are fwd_column's, so the results have the same bits.
-//
-// Bound: instruction issue, 15 a cell (11 for the cell and its band mask; pairs
-// of columns, as one column per step took 17 to 20), at 2.6 of 4 per cycle: the
-// strips' registers leave 2 to 4 warps per scheduler.  4 items at a time, in
-// the order of the batch (largest first); one at a time measured slower.  One
-// GB300, 12288 items of 32 to 2048 values, r = 0.1 (6.0e9 cells): 20.4 -> 4.7 ms.
-
-constexpr int kWaveItems = 4;    // items a warp takes at a time (32 / the least G)
-constexpr int kWaveBlock = 128;
-
-// An item with the shorter series on the rows (its own geometry has mn = 0).
-// Strips of S rows, columns in pairs: strip s runs over pairs [cs(s), ce(s)).
-template <int S>
-struct WaveGeom {
-    const float *X, *Y;
-    int n, m, r, mx, strips;
-    __device__ int cs(int s) const { return imax(0, 1 + s * S - r + 1) >> 1; }
-    __device__ int ce(int s) const { return (imin(m, imin(n, 1 + (s + 1) * S) - 1 + mx) + 1) >> 1; }
-    // steps from a round to the next: lane 0 reads a pair of the row one step
-    // before it uses it, after lane G - 1's step; and ce(s) - cs(s + G) <=
-    // min(m, mx + r + S - 2 - G S) / 2 + 1
-    __device__ int delta(int G) const {
-        return imax(G + 2, (imin(m, mx + r + S - 2 - G * S) >> 1) + 1);
-    }
-    __device__ int steps(int G) const {
-        return strips < 1 ? 0
-                          : (strips - 1) / G * delta(G) + ((strips - 1) & (G - 1)) + ((m + 1) >> 1);
-    }
-};
-
-template <int S>
-__device__ __forceinline__ WaveGeom<S> wave_item(const Dtw32Job &J, int64_t t, int64_t end) {
-    WaveGeom<S> w{};
-    if (t >= end) return w;
-    const Item it = load_item(J, t);
-    if (it.n < 1 || it.m < 1 || it.n >= J.ring_cols || it.m >= J.ring_cols) return w;
-    const bool swap = it.n > it.m;
-    w.X = swap ? it.Y : it.X;
-    w.Y = swap ? it.X : it.Y;
-    w.n = swap ? it.m : it.n;
-    w.m = swap ? it.n : it.m;
-    w.r = it.r;
-    w.mx = w.m - w.n + w.r;
-    w.strips = (w.n - 1 + S - 1) / S;
-    return w;
-}
-
-// band_bits with the shifts' clamp at 32
-__device__ __forceinline__ unsigned wave_bits(int e, int width) {
-    unsigned upper, lower;
-    asm("shr.u32 %0, 0xffffffff, %1;" : "=r"(upper) : "r"(imax(31 - e, 0)));
-    asm("shl.b32 %0, 0xffffffff, %1;" : "=r"(lower) : "r"(imax(e - width + 1, 0)));
-    return upper & lower;
-}
-
-__device__ __forceinline__ HL hl_shfl_up(HL v, int G) {
-    return HL{__shfl_up_sync(0xffffffffu, v.h, 1, G), __shfl_up_sync(0xffffffffu, v.l, 1, G)};
-}
-
-// fwd_column with the band mask.  Its three selections are additions of -0 (nz,
-// which the compiler does not know) under a predicate: they run on the FMA pipe
-// and leave the ALU pipe the minimum and the comparisons.
-template <int S>
-__device__ __forceinline__ void wave_column(const HL (&Pin)[S], HL (&Pout)[S], HL bup, HL bdiag,
-                                            float yc, const uint64_t (&xr2)[S / 2], unsigned M,
-                                            float nz, float inf) {
-    float cpair[2];
-    const uint64_t yp = pack2(yc, yc);
-#pragma unroll
-    for (int k = 0; k < S; k++) {
-        if ((k & 1) == 0) sqdiff2p(xr2[k / 2], yp, cpair[0], cpair[1]);
-        const HL dg = k == 0 ? bdiag : Pin[k - 1];
-        const HL up = k == 0 ? bup : Pout[k - 1];
-        const HL lf = Pin[k];
-        float cst = cpair[k & 1];
-        asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.eq.u32 p, t, 0;"
-            " @p add.rn.f32 %0, %3, %4;}"
-            : "+f"(cst)
-            : "r"(M), "r"(1u << k), "f"(inf), "f"(nz));
-        float bh, bl = dg.l;
-        asm("min.f32 %0, %1, %2, %3;" : "=f"(bh) : "f"(dg.h), "f"(up.h), "f"(lf.h));
-        asm("{.reg .pred p; setp.eq.f32 p, %1, %2; @p add.rn.f32 %0, %3, %4;}"
-            : "+f"(bl) : "f"(up.h), "f"(bh), "f"(up.l), "f"(nz));
-        asm("{.reg .pred p; setp.eq.f32 p, %1, %2; @p add.rn.f32 %0, %3, %4;}"
-            : "+f"(bl) : "f"(lf.h), "f"(bh), "f"(lf.l), "f"(nz));
-        const float sh = __fadd_rn(bh, cst);
-        const float err = __fsub_rn(cst, __fsub_rn(sh, bh));
-        Pout[k] = HL{sh, __fadd_rn(bl, err)};
-    }
-}
-
-template <int S, int NB>
-__global__ void __launch_bounds__(kWaveBlock, NB)
-    dtw32_wave_kernel(const Dtw32Job J, float nz, float inf) {
-    const unsigned FULL = 0xffffffffu;
-    constexpr int NEVER = 0x7fffffff;
-    const float qnan = __int_as_float(0x7fc00000);
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * kWaveBlock + threadIdx.x) >> 5;
-    const int64_t slots = (int64_t)gridDim.x * (kWaveBlock / 32) * kWaveItems;
-    for (;;) {
-        unsigned long long first = 0;
-        if (lane == 0) first = atomicAdd(J.queue, 1ull);
-        const int64_t turn = (int64_t)__shfl_sync(FULL, first, 0);
-        const int64_t base = turn * kWaveItems;
-        if (base >= J.n_items) break;
-        const int64_t end = J.n_items < base + kWaveItems ? J.n_items : base + kWaveItems;
-        // lanes per item: the least passes x steps
-        int G = 32;
-        {
-            const WaveGeom<S> w = wave_item<S>(J, base + (lane & (kWaveItems - 1)), end);
-            int best = NEVER;
-            for (int q = 8; q <= 32; q *= 2) {
-                const int cost = __reduce_max_sync(FULL, w.steps(q)) * (q / 8);
-                if (cost < best) {
-                    best = cost;
-                    G = q;
-                }
-            }
-        }
-        const int g = lane & (G - 1), group = lane / G, per_warp = 32 / G;
-        float4 *ring = reinterpret_cast<float4 *>(J.ring) + warp * kWaveItems + group;
-        for (int64_t b0 = base; b0 < end; b0 += per_warp) {
-            const int64_t t = b0 + group;
-            const WaveGeom<S> w = wave_item<S>(J, t, end);
-            const int n = w.n, m = w.m, strips = w.strips;
-            const int lim = imin(m, w.mx);  // columns of row 0
-            const int lo = -(w.r - 1), width = w.mx - lo;
-            const int delta = w.delta(G);
-            const int steps = __reduce_max_sync(FULL, w.steps(G));
-            const float *const Y = w.Y;
-            HL result = hl_inf(), acc = hl_inf(), bdiag = hl_inf(), before = hl_inf();
-            float4 rq = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const float x0 = n > 0 ? w.X[0] : 0.0f;
-            // cell (0, c) of row 0, c ascending
-            auto row0 = [&](int c, float y) {
-                const float v = __fsub_rn(x0, y);
-                const float cc = __fmul_rn(v, v);
-                acc = c == 0 ? HL{cc, 0.0f} : add_c(acc, cc);
-            };
-            if (n == 1 && g == 0) {
-                for (int c = 0; c < lim; c++) row0(c, Y[c]);
-                result = acc;
-            }
-            // the lane's strip: rows from i0, pairs [cs, ce), those of the row
-            // above [pcs, pce); p runs through it, below cs before its start
-            int s = g, p = -g, i0 = 1 + g * S;
-            int cs = NEVER, ce = NEVER, pcs = 0, pce = (lim + 1) >> 1, pres = -1;
-            bool store = false;
-            auto enter = [&]() {
-                const bool any = s < strips;
-                cs = any ? w.cs(s) : NEVER;
-                ce = any ? w.ce(s) : NEVER;
-                if (any && s > 0) {
-                    pcs = w.cs(s - 1);
-                    pce = w.ce(s - 1);
-                }
-                pres = s == strips - 1 ? (m - 1) >> 1 : -1;
-                store = g == G - 1 && s + 1 < strips;
-                i0 = 1 + s * S;
-            };
-            enter();
-            float xn[S], yq0 = 0.0f, yq1 = 0.0f;
-            auto load_y = [&](int q) {
-                if ((unsigned)(2 * q) < (unsigned)m) yq0 = Y[2 * q];
-                if ((unsigned)(2 * q + 1) < (unsigned)m) yq1 = Y[2 * q + 1];
-            };
-#pragma unroll
-            for (int k = 0; k < S; k++) xn[k] = i0 + k < n ? w.X[i0 + k] : qnan;
-            load_y(p);
-            HL P[S], Q[S];
-            float xr[S];
-            uint64_t xr2[S / 2];
-#pragma unroll
-            for (int k = 0; k < S; k++) P[k] = Q[k] = hl_inf(), xr[k] = qnan;
-#pragma unroll
-            for (int k = 0; k < S / 2; k++) xr2[k] = 0ull;
-            for (int step = 0; step < steps; step++) {
-                HL up0 = hl_shfl_up(Q[S - 1], G), up1 = hl_shfl_up(P[S - 1], G);
-                const float y0 = yq0, y1 = yq1;
-                const int p1 = p + 1;
-                load_y(p1);
-                if (g == 0) {
-                    if (s > 0) {
-                        up0 = HL{rq.x, rq.y};
-                        up1 = HL{rq.z, rq.w};
-                        if (p1 >= pcs && p1 < pce) rq = ring[(int64_t)p1 * slots];
-                    } else if (p < pce) {
-                        row0(2 * p, y0);
-                        up0 = acc;
-                        up1 = hl_inf();
-                        if (2 * p + 1 < lim) {
-                            row0(1, y1);
-                            up1 = acc;
-                        }
-                    }
-                }
-                if (p >= cs) {
-                    if (p == cs) {
-                        bdiag = hl_inf();
-                        if (cs > pcs && cs <= pce) {
-                            bdiag = before;
-                            if (g == 0) {
-                                const float4 v = ring[(int64_t)(cs - 1) * slots];
-                                bdiag = HL{v.z, v.w};
-                            }
-                        }
-#pragma unroll
-                        for (int k = 0; k < S; k++) {
-                            P[k] = hl_inf();
-                            xr[k] = xn[k];
-                            const int i = i0 + G * S + k;
-                            xn[k] = i < n ? w.X[i] : qnan;
-                        }
-#pragma unroll
-                        for (int k = 0; k < S / 2; k++)
-                            xr2[k] = pack2(xr[2 * k], xr[2 * k + 1]);
-                    }
-                    HL a0 = up0, a1 = up1;
-                    if (p >= pce) a0 = a1 = hl_inf();
-                    const int e = 2 * p - i0 - lo;
-                    wave_column<S>(P, Q, a0, bdiag, y0, xr2, wave_bits(e, width), nz, inf);
-                    const unsigned M1 = 2 * p + 1 < m ? wave_bits(e + 1, width) : 0u;
-                    wave_column<S>(Q, P, a1, a0, y1, xr2, M1, nz, inf);
-                    bdiag = a1;
-                    if (store)
-                        ring[(int64_t)p * slots] =
-                            make_float4(Q[S - 1].h, Q[S - 1].l, P[S - 1].h, P[S - 1].l);
-                    if (p == pres) {
-#pragma unroll
-                        for (int k = 0; k < S; k++)
-                            if (i0 + k < n) result = (m & 1) ? Q[k] : P[k];
-                    }
-                }
-                before = up1;
-                p = p1;
-                if (p >= ce) {  // the lane's next strip
-                    s += G;
-                    p -= delta;
-                    enter();
-                    load_y(p);
-                    if (g == 0 && s < strips && p >= pcs && p < pce)
-                        rq = ring[(int64_t)p * slots];
-                }
-                __syncwarp();
-            }
-            // the lane of the last strip (lane 0 where row 0 is the only one)
-            const int owner = strips > 0 ? (strips - 1) & (G - 1) : 0;
-            if (t < end && g == owner) {
-                double res = __longlong_as_double(0x7ff8000000000000LL);  // NaN: empty series
-                if (n > 0) {
-                    const double cost = (double)result.h + (double)result.l;
-                    if (J.out_cost) J.out_cost[t] = cost;
-                    res = sqrt(cost);
-                } else if (J.out_cost) {
-                    J.out_cost[t] = res;
-                }
-                J.out[t] = res;
-            }
-            __syncwarp();
-        }
-    }
-}
-
-// Rows of a strip and blocks of the lanes-per-item forward for a planned job
-// (grid and block of one thread per item), or no such form.  Measured on one
-// GB300 (ms; one thread per item against the strips below):
-//   ragged to 2048, r = 0.1, 12288 items   20.4   8: 7.1  16: 5.0  24: 4.7
-//   ragged to 2048, r = 0.05, 24576        22.2      8.9      7.3      7.4
-//   ragged to 1024, r = 0.1, 12288          5.1      2.0      1.40     1.44
-//   ragged to 512, r = 0.1, 24576           1.7      0.77     0.83     1.06
-//   ragged to 500, r = 0.2, 1000            1.69     0.40     0.30     0.27
-//   ragged to 200, r = 0.05, 24576          0.31     0.23     0.32     0.42
-//   256 each, r = 0.1, 8000                 0.29     0.18     0.24     0.31
-//   256 each, r = 0.1, 32000                0.39     0.51     0.68     0.98
-//   1024 each, r = 0.1, 20000               3.7      2.9      2.6      2.6
-//   1024 each, r = 0.1, 120000             12.0     15.8     13.2     14.1
-//   64 each, r = 0.1, 10000                 0.072    0.077    0.091    0.117
-// so: up to 6 warps' worth of items per SM, fewer for short series.
-void dtw32_wave_plan(Dtw32Job &J) {
-    J.wave = 0;
-    if (J.weights) return;
-    const int64_t sms = device_info().sm_count;
-    const int rows = imin(J.x_len, J.y_len);
-    if (J.n_items > 32 * 6 * sms || (rows < 128 && J.n_items > 32 * sms)) return;
-    const int64_t turns = (J.n_items + kWaveItems - 1) / kWaveItems;
-    int per_sm;
-    if (rows < 192 || (rows < 768 && turns > 16 * sms)) {
-        J.wave_rows = 8;
-        per_sm = 4;
-    } else if (rows < 1536) {
-        J.wave_rows = 16;
-        per_sm = 3;
-    } else {
-        J.wave_rows = 24;
-        per_sm = 2;
-    }
-    // its rows take no more of the ring than one thread per item does
-    const int64_t warps = kWaveBlock / 32;
-    const int64_t fit = (int64_t)J.grid * J.block / (kWaveItems * warps);
-    int64_t g = (turns + warps - 1) / warps;
-    if (g > per_sm * sms) g = per_sm * sms;
-    J.wave = (int)(g < fit ? g : fit);
 }
 
 // ---------------------------------------------------------------------------
@@ -1295,15 +979,17 @@ __global__ void __launch_bounds__(kBwdBlock) dtw32_keep_walk_kernel(const Dtw32J
     const int lane = threadIdx.x & 31;
     const float *__restrict__ w = J.weights;
     for (;;) {
-        const int64_t base = take_items(J.queue, lane);
+        unsigned long long first = 0;
+        if (lane == 0) first = atomicAdd(J.queue, (unsigned long long)J.wave_items);
+        const int64_t base = (int64_t)__shfl_sync(0xffffffffu, first, 0);
         if (base >= J.n_items) break;
-        const int64_t t = base + lane;
+        const int64_t t = lane < J.wave_items ? base + lane : J.n_items;
         BwdItem B;
         double g = 0.0;
         bwd_setup(J, t, B, g);
         int *tab_cs, *tab_base;
         uint32_t *words;
-        keep_region(D, base, tab_cs, tab_base, words);
+        keep_region(D, t & ~(int64_t)31, tab_cs, tab_base, words);
         int i = B.n - 1, j = B.m - 1;
         float gr = 0.0f, gcol = 0.0f, sc = 0.0f;
         bool done = B.n < 1;
@@ -1313,16 +999,411 @@ __global__ void __launch_bounds__(kBwdBlock) dtw32_keep_walk_kernel(const Dtw32J
             // gradients, never zeros
             sc = (Dv > 0.0 || Dv != Dv) ? (float)(g / Dv) : 0.0f;
         }
-        bwd_walk<W>(B, 0, 1, words, D.cap, tab_cs, tab_base, lane, 32, w, sc, i, j, gr, gcol,
+        bwd_walk<W>(B, 0, 1, words, D.cap, tab_cs, tab_base, t & 31, 32, w, sc, i, j, gr, gcol,
                     done);
     }
+}
+
+// ---------------------------------------------------------------------------
+// Forward of few items (dtw): the strips of an item on several lanes.
+//
+// With one thread per item a batch of some thousand items leaves most warp
+// slots empty, and the call takes as long as its longest item on a warp by
+// itself.  Here G = 8, 16 or 32 lanes share an item: lane g sweeps strips g, g +
+// G, .. of S rows, a pair of columns per step, one pair behind lane g - 1,
+// whose bottom cells it takes by shuffle; lane 0 takes them from a row in
+// global memory that lane G - 1 wrote in the round before.  A lane keeps to its
+// strip's columns; round q + 1 starts `delta` steps after round q, the least
+// after which every lane is done with its strip and lane 0's row is written.
+// The cells' operations are fwd_column's, so the results have the same bits.
+//
+// Bound: instruction issue, 15 a cell (11 for the cell and its band mask; pairs
+// of columns, as one column per step took 17 to 20), at 2.6 of 4 per cycle: the
+// strips' registers leave 2 to 4 warps per scheduler.  A warp takes 4 items at a
+// time in the order of the batch (largest first), 1 or 2 where there are not
+// enough of them for every scheduler.  One GB300, items of 32 to 2048 values, r =
+// 0.1: 12288 (6.0e9 cells) 20.4 -> 4.7 ms, 1200 19.0 -> 1.3 ms (4 at a time: 2.4).
+
+constexpr int kWaveItems = 4;    // most items a warp takes at a time (32 / the least G)
+constexpr int kWaveBlock = 128;
+
+// An item with the shorter series on the rows (its own geometry has mn = 0).
+// Strips of S rows, columns in pairs: strip s runs over pairs [cs(s), ce(s)).
+template <int S>
+struct WaveGeom {
+    const float *X, *Y;
+    int n, m, r, mx, strips;
+    __host__ __device__ int cs(int s) const { return imax(0, 1 + s * S - r + 1) >> 1; }
+    __host__ __device__ int ce(int s) const { return (imin(m, imin(n, 1 + (s + 1) * S) - 1 + mx) + 1) >> 1; }
+    // steps from a round to the next: lane 0 reads a pair of the row one step
+    // before it uses it, after lane G - 1's step; and ce(s) - cs(s + G) <=
+    // min(m, mx + r + S - 2 - G S) / 2 + 1
+    __host__ __device__ int delta(int G) const {
+        return imax(G + 2, (imin(m, mx + r + S - 2 - G * S) >> 1) + 1);
+    }
+    __host__ __device__ int steps(int G) const {
+        return strips < 1 ? 0
+                          : (strips - 1) / G * delta(G) + ((strips - 1) & (G - 1)) + ((m + 1) >> 1);
+    }
+    // columns of the strips before s (whole ones): the sums of min(m, S (k + 1) +
+    // mx) and of max(0, 2 + S k - r) over k < s
+    __device__ int words_before(int s) const {
+        const int a = imin(imax(m - mx, 0) / S, s);
+        const int z = r >= 2 ? imin(s, (r - 2) / S + 1) : 0;
+        return S * (a * (a + 1) / 2) + a * mx + (s - a) * m - (s - z) * (2 - r) -
+               S * (s * (s - 1) / 2 - z * (z - 1) / 2);
+    }
+};
+
+template <int S>
+__device__ __forceinline__ WaveGeom<S> wave_item(const Dtw32Job &J, int64_t t, int64_t end) {
+    WaveGeom<S> w{};
+    if (t >= end) return w;
+    const Item it = load_item(J, t);
+    if (it.n < 1 || it.m < 1 || it.n >= J.ring_cols || it.m >= J.ring_cols) return w;
+    const bool swap = it.n > it.m;
+    w.X = swap ? it.Y : it.X;
+    w.Y = swap ? it.X : it.Y;
+    w.n = swap ? it.m : it.n;
+    w.m = swap ? it.n : it.m;
+    w.r = it.r;
+    w.mx = w.m - w.n + w.r;
+    w.strips = (w.n - 1 + S - 1) / S;
+    return w;
+}
+
+// band_bits with the shifts' clamp at 32
+__device__ __forceinline__ unsigned wave_bits(int e, int width) {
+    unsigned upper, lower;
+    asm("shr.u32 %0, 0xffffffff, %1;" : "=r"(upper) : "r"(imax(31 - e, 0)));
+    asm("shl.b32 %0, 0xffffffff, %1;" : "=r"(lower) : "r"(imax(e - width + 1, 0)));
+    return upper & lower;
+}
+
+__device__ __forceinline__ HL hl_shfl_up(HL v, int G) {
+    return HL{__shfl_up_sync(0xffffffffu, v.h, 1, G), __shfl_up_sync(0xffffffffu, v.l, 1, G)};
+}
+
+// fwd_column with the band mask.  Its three selections are additions of -0 (nz,
+// which the compiler does not know) under a predicate: they run on the FMA pipe
+// and leave the ALU pipe the minimum and the comparisons.
+template <int S>
+__device__ __forceinline__ void wave_column(const HL (&Pin)[S], HL (&Pout)[S], HL bup, HL bdiag,
+                                            float yc, const uint64_t (&xr2)[S / 2], unsigned M,
+                                            float nz, float inf) {
+    float cpair[2];
+    const uint64_t yp = pack2(yc, yc);
+#pragma unroll
+    for (int k = 0; k < S; k++) {
+        if ((k & 1) == 0) sqdiff2p(xr2[k / 2], yp, cpair[0], cpair[1]);
+        const HL dg = k == 0 ? bdiag : Pin[k - 1];
+        const HL up = k == 0 ? bup : Pout[k - 1];
+        const HL lf = Pin[k];
+        float cst = cpair[k & 1];
+        asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.eq.u32 p, t, 0;"
+            " @p add.rn.f32 %0, %3, %4;}"
+            : "+f"(cst)
+            : "r"(M), "r"(1u << k), "f"(inf), "f"(nz));
+        float bh, bl = dg.l;
+        asm("min.f32 %0, %1, %2, %3;" : "=f"(bh) : "f"(dg.h), "f"(up.h), "f"(lf.h));
+        asm("{.reg .pred p; setp.eq.f32 p, %1, %2; @p add.rn.f32 %0, %3, %4;}"
+            : "+f"(bl) : "f"(up.h), "f"(bh), "f"(up.l), "f"(nz));
+        asm("{.reg .pred p; setp.eq.f32 p, %1, %2; @p add.rn.f32 %0, %3, %4;}"
+            : "+f"(bl) : "f"(lf.h), "f"(bh), "f"(lf.l), "f"(nz));
+        const float sh = __fadd_rn(bh, cst);
+        const float err = __fsub_rn(cst, __fsub_rn(sh, bh));
+        Pout[k] = HL{sh, __fadd_rn(bl, err)};
+    }
+}
+
+// KEEP: the sweep with directions (bwd_column) into the items' batch regions, for
+// items of one shape (no lengths): the strip tables of a batch follow from it.
+template <int S, int NB, bool KEEP>
+__global__ void __launch_bounds__(kWaveBlock, NB)
+    dtw32_wave_kernel(const Dtw32Job J, const DirKeep D, float nz, float inf) {
+    static_assert(!KEEP || S == kGradStrip, "a word per strip column");
+    const unsigned FULL = 0xffffffffu;
+    constexpr int NEVER = 0x7fffffff;
+    const float qnan = __int_as_float(0x7fc00000);
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * kWaveBlock + threadIdx.x) >> 5;
+    const int per_turn = J.wave_items;
+    const int64_t slots = (int64_t)gridDim.x * (kWaveBlock / 32) * per_turn;
+    for (;;) {
+        unsigned long long first = 0;
+        if (lane == 0) first = atomicAdd(J.queue, (unsigned long long)per_turn);
+        const int64_t base = (int64_t)__shfl_sync(FULL, first, 0);
+        if (base >= J.n_items) break;
+        const int64_t end = J.n_items < base + per_turn ? J.n_items : base + per_turn;
+        // lanes per item: the least passes x steps
+        int G = 32;
+        {
+            const WaveGeom<S> w = wave_item<S>(J, base + (lane & (per_turn - 1)), end);
+            int best = NEVER;
+            for (int q = 32 / per_turn; q <= 32; q *= 2) {
+                const int cost = __reduce_max_sync(FULL, w.steps(q)) * (q * per_turn / 32);
+                if (cost < best) {
+                    best = cost;
+                    G = q;
+                }
+            }
+        }
+        const int g = lane & (G - 1), group = lane / G, per_warp = 32 / G;
+        float4 *ring = reinterpret_cast<float4 *>(J.ring) + warp * per_turn + group;
+        for (int64_t b0 = base; b0 < end; b0 += per_warp) {
+            const int64_t t = b0 + group;
+            const WaveGeom<S> w = wave_item<S>(J, t, end);
+            const int n = w.n, m = w.m, strips = w.strips;
+            const int lim = imin(m, w.mx);  // columns of row 0
+            const int lo = -(w.r - 1), width = w.mx - lo;
+            const int delta = w.delta(G);
+            const int steps = __reduce_max_sync(FULL, w.steps(G));
+            const float *const Y = w.Y;
+            HL result = hl_inf(), acc = hl_inf(), bdiag = hl_inf(), before = hl_inf();
+            float4 rq = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float x0 = n > 0 ? w.X[0] : 0.0f;
+            // cell (0, c) of row 0, c ascending
+            auto row0 = [&](int c, float y) {
+                const float v = __fsub_rn(x0, y);
+                const float cc = __fmul_rn(v, v);
+                acc = c == 0 ? HL{cc, 0.0f} : add_c(acc, cc);
+            };
+            if (n == 1 && g == 0) {
+                for (int c = 0; c < lim; c++) row0(c, Y[c]);
+                result = acc;
+            }
+            // the lane's strip: rows from i0, pairs [cs, ce), those of the row
+            // above [pcs, pce); p runs through it, below cs before its start
+            int s = g, p = -g, i0 = 1 + g * S;
+            int cs = NEVER, ce = NEVER, pcs = 0, pce = (lim + 1) >> 1, pres = -1;
+            bool store = false;
+            int *tab_cs = nullptr, *tab_base = nullptr;
+            uint32_t *words = nullptr;
+            int kcs = 0, kce = 0, kbase = 0;  // the strip's columns and first word
+            if (KEEP && t < end) keep_region(D, t & ~(int64_t)31, tab_cs, tab_base, words);
+            auto enter = [&]() {
+                const bool any = s < strips;
+                cs = any ? w.cs(s) : NEVER;
+                ce = any ? w.ce(s) : NEVER;
+                if (any && s > 0) {
+                    pcs = w.cs(s - 1);
+                    pce = w.ce(s - 1);
+                }
+                pres = s == strips - 1 ? (m - 1) >> 1 : -1;
+                store = g == G - 1 && s + 1 < strips;
+                i0 = 1 + s * S;
+                if (KEEP && any) {
+                    kcs = imax(0, i0 - w.r + 1);
+                    kce = imin(m, imin(n, i0 + S) - 1 + w.mx);
+                    kbase = w.words_before(s);
+                    if ((t & 31) == 0) {
+                        tab_cs[s] = kcs;
+                        tab_base[s] = kbase;
+                    }
+                }
+            };
+            enter();
+            float xn[S], yq0 = 0.0f, yq1 = 0.0f;
+            auto load_y = [&](int q) {
+                if ((unsigned)(2 * q) < (unsigned)m) yq0 = Y[2 * q];
+                if ((unsigned)(2 * q + 1) < (unsigned)m) yq1 = Y[2 * q + 1];
+            };
+#pragma unroll
+            for (int k = 0; k < S; k++) xn[k] = i0 + k < n ? w.X[i0 + k] : qnan;
+            load_y(p);
+            HL P[S], Q[S];
+            float xr[S];
+            uint64_t xr2[S / 2];
+#pragma unroll
+            for (int k = 0; k < S; k++) P[k] = Q[k] = hl_inf(), xr[k] = qnan;
+#pragma unroll
+            for (int k = 0; k < S / 2; k++) xr2[k] = 0ull;
+            for (int step = 0; step < steps; step++) {
+                HL up0 = hl_shfl_up(Q[S - 1], G), up1 = hl_shfl_up(P[S - 1], G);
+                const float y0 = yq0, y1 = yq1;
+                const int p1 = p + 1;
+                load_y(p1);
+                if (g == 0) {
+                    if (s > 0) {
+                        up0 = HL{rq.x, rq.y};
+                        up1 = HL{rq.z, rq.w};
+                        if (p1 >= pcs && p1 < pce) rq = ring[(int64_t)p1 * slots];
+                    } else if (p < pce) {
+                        row0(2 * p, y0);
+                        up0 = acc;
+                        up1 = hl_inf();
+                        if (2 * p + 1 < lim) {
+                            row0(1, y1);
+                            up1 = acc;
+                        }
+                    }
+                }
+                if (p >= cs) {
+                    if (p == cs) {
+                        bdiag = hl_inf();
+                        if (cs > pcs && cs <= pce) {
+                            bdiag = before;
+                            if (g == 0) {
+                                const float4 v = ring[(int64_t)(cs - 1) * slots];
+                                bdiag = HL{v.z, v.w};
+                            }
+                        }
+#pragma unroll
+                        for (int k = 0; k < S; k++) {
+                            P[k] = hl_inf();
+                            xr[k] = xn[k];
+                            const int i = i0 + G * S + k;
+                            xn[k] = i < n ? w.X[i] : qnan;
+                        }
+#pragma unroll
+                        for (int k = 0; k < S / 2; k++)
+                            xr2[k] = pack2(xr[2 * k], xr[2 * k + 1]);
+                    }
+                    HL a0 = up0, a1 = up1;
+                    if (p >= pce) a0 = a1 = hl_inf();
+                    const int c = 2 * p, e = c - i0 - lo;
+                    const unsigned M0 = wave_bits(e, width);
+                    const unsigned M1 = c + 1 < m ? wave_bits(e + 1, width) : 0u;
+                    if constexpr (KEEP) {
+                        uint32_t w0 = 0, w1 = 0;
+                        bwd_column<false, true>(P, Q, a0, bdiag, y0, xr, xr2, 0, M0, nullptr, S,
+                                                w0);
+                        bwd_column<false, true>(Q, P, a1, a0, y1, xr, xr2, 0, M1, nullptr, S,
+                                                w1);
+                        const int64_t at = kbase + c - kcs, k = t & 31;
+                        if (c >= kcs) words[dir_index(at, k, 32)] = w0;
+                        if (c + 1 < kce) words[dir_index(at + 1, k, 32)] = w1;
+                    } else {
+                        wave_column<S>(P, Q, a0, bdiag, y0, xr2, M0, nz, inf);
+                        wave_column<S>(Q, P, a1, a0, y1, xr2, M1, nz, inf);
+                    }
+                    bdiag = a1;
+                    if (store)
+                        ring[(int64_t)p * slots] =
+                            make_float4(Q[S - 1].h, Q[S - 1].l, P[S - 1].h, P[S - 1].l);
+                    if (p == pres) {
+#pragma unroll
+                        for (int k = 0; k < S; k++)
+                            if (i0 + k < n) result = (m & 1) ? Q[k] : P[k];
+                    }
+                }
+                before = up1;
+                p = p1;
+                if (p >= ce) {  // the lane's next strip
+                    s += G;
+                    p -= delta;
+                    enter();
+                    load_y(p);
+                    if (g == 0 && s < strips && p >= pcs && p < pce)
+                        rq = ring[(int64_t)p * slots];
+                }
+                __syncwarp();
+            }
+            // the lane of the last strip (lane 0 where row 0 is the only one)
+            const int owner = strips > 0 ? (strips - 1) & (G - 1) : 0;
+            if (t < end && g == owner) {
+                double res = __longlong_as_double(0x7ff8000000000000LL);  // NaN: empty series
+                if (n > 0) {
+                    const double cost = (double)result.h + (double)result.l;
+                    if (J.out_cost) J.out_cost[t] = cost;
+                    res = sqrt(cost);
+                } else if (J.out_cost) {
+                    J.out_cost[t] = res;
+                }
+                J.out[t] = res;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Items per turn and blocks of the kernel.  A turn of few items on more lanes
+// each takes fewer steps, which counts until every scheduler has a warp.  (Items
+// with lengths: as for a third and two thirds of the longest.)  The kernel's
+// rows take no more of the ring than one thread per item does.
+template <int S>
+static void wave_grid(Dtw32Job &J, int per_sm) {
+    const int64_t sms = device_info().sm_count, warps = kWaveBlock / 32;
+    WaveGeom<S> w{};
+    w.n = imin(J.x_len, J.y_len);
+    w.m = imax(J.x_len, J.y_len);
+    if (J.xlen || J.ylen) {
+        w.n = imax(w.m / 3, 1);
+        w.m = imax(2 * w.m / 3, w.n);
+    }
+    w.r = J.band_fixed > 0 ? J.band_fixed : imax((int)(w.n * J.r), 1);
+    w.mx = w.m - w.n + w.r;
+    w.strips = (w.n - 1 + S - 1) / S;
+    double best = 0.0;
+    for (int q = kWaveItems; q >= 1; q /= 2) {
+        int steps = 0x7fffffff;
+        for (int G = 32 / q; G <= 32; G *= 2) steps = imin(steps, w.steps(G) * (G * q / 32));
+        const double turns = (double)((J.n_items + q - 1) / q);
+        const double cost = steps * std::fmax(1.0, turns / (4.0 * (double)sms));
+        if (q == kWaveItems || cost < best) {
+            best = cost;
+            J.wave_items = q;
+        }
+    }
+    const int64_t turns = (J.n_items + J.wave_items - 1) / J.wave_items;
+    const int64_t fit = (int64_t)J.grid * J.block / (J.wave_items * warps);
+    const int64_t g = std::min((turns + warps - 1) / warps, (int64_t)per_sm * sms);
+    J.wave = (int)std::min(g, fit);
+}
+
+// Rows of a strip and blocks of the lanes-per-item forward for a planned job
+// (grid and block of one thread per item), or no such form.  Measured on one
+// GB300 (ms; one thread per item against the strips below):
+//   ragged to 2048, r = 0.1, 12288 items   20.4   8: 7.1  16: 5.0  24: 4.7
+//   ragged to 2048, r = 0.05, 24576        22.2      8.9      7.3      7.4
+//   ragged to 1024, r = 0.1, 12288          5.1      2.0      1.40     1.44
+//   ragged to 512, r = 0.1, 24576           1.7      0.77     0.83     1.06
+//   ragged to 500, r = 0.2, 1000            1.69     0.40     0.30     0.27 (0.19 with 2 a turn)
+//   ragged to 200, r = 0.05, 24576          0.31     0.23     0.32     0.42
+//   256 each, r = 0.1, 8000                 0.29     0.18     0.24     0.31
+//   256 each, r = 0.1, 32000                0.39     0.51     0.68     0.98
+//   1024 each, r = 0.1, 20000               3.7      2.9      2.6      2.6
+//   1024 each, r = 0.1, 120000             12.0     15.8     13.2     14.1
+//   64 each, r = 0.1, 10000                 0.072    0.077    0.091    0.117
+// so: up to 6 warps' worth of items per SM, fewer for short series.
+void dtw32_wave_plan(Dtw32Job &J) {
+    J.wave = 0;
+    if (J.weights) return;
+    const int64_t sms = device_info().sm_count;
+    const int rows = imin(J.x_len, J.y_len);
+    if (J.n_items > 32 * 6 * sms || (rows < 128 && J.n_items > 32 * sms)) return;
+    const int64_t turns = (J.n_items + kWaveItems - 1) / kWaveItems;
+    if (rows < 192 || (rows < 768 && turns > 16 * sms)) {
+        J.wave_rows = 8;
+        wave_grid<8>(J, 4);
+    } else if (rows < 1536) {
+        J.wave_rows = 16;
+        wave_grid<16>(J, 3);
+    } else {
+        J.wave_rows = 24;
+        wave_grid<24>(J, 2);
+    }
+}
+
+// The same for the sweep that keeps directions.  Measured as above, forward and
+// backward of a dtw matrix with its loss (one thread per item -> lanes): 162 x 5
+// of 471, r = 0.5, 6.9 -> 0.93 ms; 698 x 5 of 350, r = 0.2, 2.3 -> 0.94; 512 x 32
+// of 256 1.29 -> 1.13; 1024 x 32 of 256 1.56 -> 1.8.
+void dtw32_wave_keep_plan(Dtw32Job &J) {
+    J.wave = 0;
+    if (J.weights || J.xlen || J.ylen) return;
+    if (J.n_items > 32 * 6 * (int64_t)device_info().sm_count) return;
+    J.wave_rows = kGradStrip;
+    wave_grid<kGradStrip>(J, 3);
 }
 
 int dtw32_keep_forward(const Dtw32Job &J, const DirKeep &D, cudaStream_t s) {
     if (J.n_items == 0) return WB_OK;
     WB_CUDA(cudaMemsetAsync(J.queue, 0, sizeof(unsigned long long), s));
     timer_begin("dtw32_keep_forward_kernel", s);
-    if (J.weights) dtw32_keep_forward_kernel<true><<<J.grid, kBwdBlock, 0, s>>>(J, D);
+    if (J.wave > 0)
+        dtw32_wave_kernel<kGradStrip, 3, true><<<J.wave, kWaveBlock, 0, s>>>(J, D, -0.0f, HUGE_VALF);
+    else if (J.weights) dtw32_keep_forward_kernel<true><<<J.grid, kBwdBlock, 0, s>>>(J, D);
     else dtw32_keep_forward_kernel<false><<<J.grid, kBwdBlock, 0, s>>>(J, D);
     timer_end(s);
     WB_LAUNCH_CHECK("dtw32_keep_forward_kernel");
@@ -1375,10 +1456,10 @@ int dtw32_forward(const Dtw32Job &J, int strip, cudaStream_t s) {
     if (J.wave > 0) {
         timer_begin("dtw32_wave_kernel", s);
         const float nz = -0.0f, inf = HUGE_VALF;
-        if (J.wave_rows == 8) dtw32_wave_kernel<8, 4><<<J.wave, kWaveBlock, 0, s>>>(J, nz, inf);
-        else if (J.wave_rows == 16)
-            dtw32_wave_kernel<16, 3><<<J.wave, kWaveBlock, 0, s>>>(J, nz, inf);
-        else dtw32_wave_kernel<24, 2><<<J.wave, kWaveBlock, 0, s>>>(J, nz, inf);
+        auto run = [&](auto kfn) { kfn<<<J.wave, kWaveBlock, 0, s>>>(J, DirKeep{}, nz, inf); };
+        if (J.wave_rows == 8) run(dtw32_wave_kernel<8, 4, false>);
+        else if (J.wave_rows == 16) run(dtw32_wave_kernel<16, 3, false>);
+        else run(dtw32_wave_kernel<24, 2, false>);
         timer_end(s);
         WB_LAUNCH_CHECK("dtw32_wave_kernel");
         return WB_OK;

@@ -47,6 +47,7 @@ struct Dtw32Job {
     int grid = 0, block = 0;
     int wave = 0;                 // > 0: blocks of the lanes-per-item forward
     int wave_rows = 0;            // its rows per strip
+    int wave_items = 32;          // items a warp takes at a time (it, and the walk)
 };
 
 // Kept directions of a differentiable call (see dtw32.cu): one region of
@@ -67,6 +68,7 @@ int dtw32_keep_blocks_per_sm(bool walk, bool weighted);
 int dtw32_backward(const Dtw32Job &J, cudaStream_t s);
 int dtw32_blocks_per_sm(int strip, bool weighted, bool backward, int block);
 void dtw32_wave_plan(Dtw32Job &J);
+void dtw32_wave_keep_plan(Dtw32Job &J);
 int launch_grid_to_matrix(const double *in, int64_t nx, int64_t ny, int upper, double *out,
                           cudaStream_t s);
 int dtw32_plan(const wb_dtw32 *q, bool backward, Dtw32Job &J, size_t &bytes);
