@@ -626,9 +626,33 @@ __device__ bool bwd_strips(const BwdItem &B, int s0, int s1, const float2 *src, 
                 out[(int64_t)c * nth] = make_float2(Q[S - 1].h, Q[S - 1].l);
                 out[(int64_t)(c + 1) * nth] = make_float2(P[S - 1].h, P[S - 1].l);
                 bdiag = bup1;
-            } else {
+            } else if (W) {
+                // (with weights the block below and a register bound took 2 to 5 % more)
                 column(c, P, Q);
                 column(c + 1, Q, P);
+            } else {
+                // two columns with rows out of band, as one block as well
+                const HL bup0 = nb0, bup1 = nb1;
+                const float y0 = ny0, y1 = ny1;
+                nb0 = load_up(c + 2);
+                nb1 = load_up(c + 3);
+                ny0 = load_y(c + 2);
+                ny1 = load_y(c + 3);
+                const unsigned M0 = c < B.m ? band_bits(c - i0 - B.lo, B.width) : 0u;
+                const unsigned M1 = c + 1 < B.m ? band_bits(c + 1 - i0 - B.lo, B.width) : 0u;
+                uint32_t w0 = 0, w1 = 0;
+                bwd_column<W, true>(P, Q, bup0, bdiag, y0, xr, xr2, c - i0, M0, w, rows, w0);
+                bwd_column<W, true>(Q, P, bup1, bup0, y1, xr, xr2, c + 1 - i0, M1, w, rows, w1);
+                put_word(c, w0);
+                put_word(c + 1, w1);
+                if (last && (c == B.m - 1 || c + 1 == B.m - 1)) {
+#pragma unroll
+                    for (int k = 0; k < S; k++)
+                        if (k == krow) result = c == B.m - 1 ? Q[k] : P[k];
+                }
+                out[(int64_t)c * nth] = make_float2(Q[S - 1].h, Q[S - 1].l);
+                out[(int64_t)(c + 1) * nth] = make_float2(P[S - 1].h, P[S - 1].l);
+                bdiag = bup1;
             }
         }
         if (c < ce_w) column(c, P, Q);
@@ -834,7 +858,7 @@ __device__ __forceinline__ void bwd_setup(const Dtw32Job &J, int64_t t, BwdItem 
 }
 
 template <bool W>
-__global__ void __launch_bounds__(kBwdBlock) dtw32_backward_kernel(const Dtw32Job J) {
+__global__ void __launch_bounds__(kBwdBlock, W ? 0 : 3) dtw32_backward_kernel(const Dtw32Job J) {
     __shared__ int tab_cs_all[kBwdBlock / 32][kMaxSegStrips];
     __shared__ int tab_base_all[kBwdBlock / 32][kMaxSegStrips];
     // per lane 8 staged direction words, stride 33 words between slots so the
@@ -927,9 +951,14 @@ __device__ __forceinline__ void keep_region(const DirKeep &D, int64_t base, int 
 
 // The sweep with directions of every item into its batch region, and the
 // distance sqrt(hi + lo) of the same sweep (compensated predecessor choice).
+// Bound: issue and ALU of the 18 instructions of a cell.  Columns go in pairs,
+// those with rows out of band too (32 of 117 at r = 0.2, length 256: one at a time
+// they waited on the chain of their rows): 131072 items of 256, r = 0.2, 2.92 ->
+// 2.63 ms.  Packed differences and selections under predicates (14 instructions)
+// issue slower: 2.95 ms.
 template <bool W>
-__global__ void __launch_bounds__(kBwdBlock) dtw32_keep_forward_kernel(const Dtw32Job J,
-                                                                      const DirKeep D) {
+__global__ void __launch_bounds__(kBwdBlock, W ? 0 : 3) dtw32_keep_forward_kernel(const Dtw32Job J,
+                                                                         const DirKeep D) {
     __shared__ uint32_t stage_all[kBwdBlock * 33 / 4 + 8 * 33];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
