@@ -1056,6 +1056,15 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
     int64_t work = (J.mode == PM_PAIRED ? (J.rows.count + 31) / 32
                                         : (J.rows.count + 31) / 32 * J.cols.count) * 32;
     if (max_pairs > 0) work = std::min(work, max_pairs);
+    // wdtw between very unequal lengths: the path ends on a diagonal whose weight
+    // is up to 10^10 times that of the main one, near which cells cost less than
+    // the 32-bit resolution and are all collected.  With two warps per SM their
+    // FP64 latency decides: 60 x 50 pairs of 60 and 900 take 19.7 ms, the full
+    // recurrence 10.0 (200 and 300: 2.8 and 9.5; 231 x 34 of 527 and 375: 13.9
+    // and 15.5; with four times the pairs 16.3 and 26.6).
+    if (J.kind == K_WDTW && imax(n, m) >= 640 && 2 * std::abs(n - m) >= imax(n, m) &&
+        work <= 64 * dev.sm_count)
+        return p;
     const int64_t want = (work + kThreads - 1) / kThreads;
     for (int S = 8; S <= 16; S += 8) {
         const int ns = (n - 1 + S - 1) / S;
