@@ -41,14 +41,15 @@ WORKLOAD = {
     "metric": "dtw",
     "params": {"r": 0.1},
 }
-FP64_OPS_PER_CELL = 3  # v = x - y, v * v, min + v*v (mins run on the integer pipe)
+# operations of a band cell of the recurrence: v = x - y, v * v, min + v * v
+OPS_PER_CELL = 3
+FP32_LANES_PER_SM = 128  # add / multiply lanes of an SM
 FP64_OPS_PER_SM_CLK = 2  # GB300 FP64 pipe (ncu sm__inst_executed_pipe_fp64 / pipe activity)
-# DRAM bytes (read + write) of one launch of the headline kernel at 2000 x 2000,
-# L = 512, from one earlier ncu capture of `python bench.py --no-cpu --no-forms
-# --steps 2 --warmup 3` (dram__bytes_read.sum 17.12 MB + dram__bytes_write.sum
-# 10.75 KB); it is not measured in the timed run.  The 32 MB output is still in
-# L2 when the kernel ends.
-HEADLINE_DRAM_BYTES = 17.12e6 + 10.75e3
+# DRAM bytes (read + write) per pair of the headline kernel, from one earlier ncu
+# capture of the same call at 512 x 304 pairs (dram__bytes.sum: 15.8 GB);
+# it is not measured in the timed run.  The 32-bit sweep keeps the bottom row of
+# every 8 rows and every 8th column of each pair for the walk.
+HEADLINE_DRAM_BYTES_PER_PAIR = 101.3e3
 
 
 def _rank():
@@ -996,35 +997,38 @@ def run_gpu(args):
             dist.destroy_process_group()
         return
 
-    # roofline of the recurrence kernel: FP64 ops per launch / launch time
+    # The headline kernel sweeps the band in 32-bit arithmetic and evaluates in
+    # FP64 only the cells that can lie on a best path, so its bound is the 32-bit
+    # operations of every band cell (3: subtract, multiply, add; minima not
+    # counted) on the FP32 lanes at the median SM clock of the timed region.
+    # fp64_recurrence is the rate that evaluating every cell in FP64 could reach
+    # on the FP64 pipe (2 operations per clock per SM) and the rate over it.
     probe_peak = _lib.alu_probe(_lib.WB_F64, 4096)
     kms = [k for k in kern_ms if k > 0]
     k_avg = sum(kms) / len(kms) if kms else t_step
-    achieved = FP64_OPS_PER_CELL * cells / (k_avg * 1e-3)
-    # the FP64 pipe issues 2 operations per clock per SM (ncu: the probe kernel
-    # keeps the pipe 84.2 % busy at 0.0526 FP64 warp-instructions per
-    # SM-cycle), times the SM count and the median SM clock sampled during the
-    # timed region
+    achieved = OPS_PER_CELL * cells / (k_avg * 1e-3)
     clk = clocks.summary()
     sm_mhz = clk.get("sm_mhz") or 2070.0
-    pipe_peak = FP64_OPS_PER_SM_CLK * torch.cuda.get_device_properties(dev).multi_processor_count \
-        * sm_mhz * 1e6
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    peak = FP32_LANES_PER_SM * sms * sm_mhz * 1e6
+    fp64_cells = FP64_OPS_PER_SM_CLK * sms * sm_mhz * 1e6 / OPS_PER_CELL
+    n_pairs = wl["nx"] * wl["ny"]
     roofline = {
-        "bound": "fp64",
+        "bound": "fp32",
         "achieved": achieved / 1e12,
-        "peak": pipe_peak / 1e12,
-        "unit": "TFLOP/s (FP64 pipe: 2 ops/clk/SM x SMs x the median SM clock of the run)",
-        "frac": achieved / pipe_peak,
-        "probe_peak": probe_peak / 1e12,
-        "frac_of_probe": achieved / probe_peak,
-        # measured for the default 2000 x 2000 workload only
-        "traffic": HEADLINE_DRAM_BYTES if (wl["nx"], wl["ny"]) == (2000, 2000) else None,
-        "traffic_unit": "bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum)",
-        "traffic_source": "one earlier ncu capture of this workload, not measured in this run",
+        "peak": peak / 1e12,
+        "unit": "TOP/s (band cells x 3; FP32 lanes: 128 per SM x SMs x the median SM clock)",
+        "frac": achieved / peak,
+        "fp64_recurrence": {"gcups": fp64_cells / 1e9, "value_over_it": value / world
+                            / (fp64_cells / 1e9), "probe_tflops": probe_peak / 1e12},
+        "traffic": HEADLINE_DRAM_BYTES_PER_PAIR * n_pairs,
+        "traffic_unit": "bytes per launch (ncu dram__bytes.sum)",
+        "traffic_source": "pairs x the bytes per pair of one earlier ncu capture at 512 x 304 "
+                          "pairs, not measured in this run",
         "algorithmic_bytes": int(X.nbytes + Y.nbytes + wl["nx"] * wl["ny"] * 8),
-        "kernel": "elastic_pairs_kernel<K_DTW>",
+        "kernel": "guided_pairs_kernel<K_DTW, 8>",
         "kernel_ms": k_avg,
-        "ops_per_cell": FP64_OPS_PER_CELL,
+        "ops_per_cell": OPS_PER_CELL,
     }
     cpu = None
     parity = None

@@ -765,9 +765,10 @@ static int strip_launch(const ElasticJob &J, Workspace *ws, size_t *bytes) {
     typename A::R *ring = ws->take<typename A::R>(nring);
     if (!ring) return fail(WB_ENOMEM, "workspace reservation exceeded");
     cudaStream_t s = ws->stream();
-    timer_begin(is_f64<A>() ? "strip_pairs_kernel<f64>" : "strip_pairs_kernel<f32>", s);
+    if (!J.pending)
+        timer_begin(is_f64<A>() ? "strip_pairs_kernel<f64>" : "strip_pairs_kernel<f32>", s);
     strip_pairs_kernel<KIND, S, A><<<grid, kStripThreads, 0, s>>>(J, ring);
-    timer_end(s);
+    if (!J.pending) timer_end(s);
     WB_LAUNCH_CHECK("strip_pairs_kernel");
     return WB_OK;
 }

@@ -604,17 +604,17 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
                                          (int)tsm));
             const int64_t tb = J.x.count * J.n_chunks;
             const int tgrid = (int)(tb < cap ? tb : cap);
-            timer_begin("subseq_scaled_tiled_kernel", s);
+            if (!J.kept) timer_begin("subseq_scaled_tiled_kernel", s);
             kt<<<tgrid, kSubThreads, tsm, s>>>(Jf, norm, mean_tab, std_tab);
-            timer_end(s);
+            if (!J.kept) timer_end(s);
             WB_LAUNCH_CHECK("subseq_scaled_tiled_kernel");
             return WB_OK;
         }
         auto k = subseq_scan_kernel<true>;
         WB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        timer_begin("subseq_scan_kernel<scaled>", s);
+        if (!J.kept) timer_begin("subseq_scan_kernel<scaled>", s);
         k<<<grid, kSubThreads, smem, s>>>(J, norm, mean_tab, std_tab);
-        timer_end(s);
+        if (!J.kept) timer_end(s);
         WB_LAUNCH_CHECK("subseq_scan_kernel<scaled>");
     } else if (J.paired) {
         timer_begin("subseq_paired_kernel", s);
@@ -633,9 +633,9 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
         const size_t fsmem = (size_t)J.x.len * 12 + 16;
         auto k = subseq_scan_kernel<false>;
         WB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
-        timer_begin("subseq_scan_kernel", s);
+        if (!J.kept) timer_begin("subseq_scan_kernel", s);
         k<<<grid, kSubThreads, fsmem, s>>>(Jf, nullptr, nullptr, nullptr);
-        timer_end(s);
+        if (!J.kept) timer_end(s);
         WB_LAUNCH_CHECK("subseq_scan_kernel");
     }
     return WB_OK;
