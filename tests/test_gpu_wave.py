@@ -59,3 +59,28 @@ def test_same_bits_as_the_ring_kernel(metric, params, kind, monkeypatch):
         monkeypatch.setenv("WB_GPU_ELASTIC", "ring")
         for a, b in zip(got, calls()):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("metric", ["erp", "msm", "twe"])
+def test_dims_and_device_inputs(metric, monkeypatch):
+    """A dim of a multivariate set (strided rows), host and device, float32 and
+    a reversed view."""
+    rng = np.random.default_rng(3)
+    X = np.cumsum(rng.standard_normal((9, 3, 41)), axis=2)
+    Y = np.cumsum(rng.standard_normal((6, 3, 50)), axis=2)
+
+    def calls():
+        xd, yd = torch.as_tensor(X, device="cuda"), torch.as_tensor(Y, device="cuda")
+        return [
+            pairwise_distance(X, Y, dim=2, metric=metric),
+            pairwise_distance(X, dim=1, metric=metric),
+            pairwise_distance(xd, yd, dim=1, metric=metric).cpu().numpy(),
+            pairwise_distance(X[::-1, :, ::-1], Y, dim=0, metric=metric),
+            pairwise_distance(X.astype(np.float32), Y.astype(np.float32), dim=0, metric=metric),
+        ]
+
+    monkeypatch.delenv("WB_GPU_ELASTIC", raising=False)
+    got = calls()
+    monkeypatch.setenv("WB_GPU_ELASTIC", "ring")
+    for a, b in zip(got, calls()):
+        np.testing.assert_array_equal(a, b)

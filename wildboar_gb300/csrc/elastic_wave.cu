@@ -14,16 +14,18 @@
 // of latency that the warp waits for.  So
 //   * warps: one block per warp and the same number of pairs for every group of
 //     lanes, so that the SMs get equal shares; G is the one with the least
-//     steps x max(latency of a step, its FP64 time x warps of an SM);
+//     steps x hypot(latency of a step, its FP64 time x warps of an SM);
 //   * operations: msm 7.8 FP64 instructions a cell -> 4.3.  c + |x_i - y_j| is
 //     formed once for both moves, c + |x_i - x_{i-1}| once per row and c +
 //     |y_j - y_{j-1}| once per column (c + min(a, b) == min(c + a, c + b), the
 //     rounding being monotone), on the integer and FP32 pipes; twe 8 -> 7:
-//     |x_{i-1} - y_{j-1}| is the previous diagonal cell's |x_i - y_j|.
+//     |x_{i-1} - y_{j-1}| is the previous diagonal cell's |x_i - y_j|, and the
+//     stiffness of a diagonal moves down a strip instead of being loaded (200 x
+//     150 pairs of 256 34.1 -> 32.4 ms).
 // Measured on one GB300 against the strip and ring kernels (one thread per
 // pair, whose busiest SM had 1.27 times the mean): msm, 301 x 290 pairs of 256 x
 // 250 111.7 -> 50.9 ms (44 ms of FP64 instructions), 9 x 10 of 256 26.2 ->
-// 0.94 ms; twe, 20 x 20 of 500 96.7 -> 3.0 ms; erp, 200 x 150 of 256 20.9 -> 16.9
+// 0.94 ms; twe, 20 x 20 of 500 95.8 -> 3.0 ms; erp, 200 x 150 of 256 20.9 -> 16.9
 // ms.
 
 #include <algorithm>
@@ -125,24 +127,27 @@ __global__ void __launch_bounds__(32)
         double P[kRows], x[kRows];
         double rx[kRows];  // erp |x_i - g|; twe |x_{i-1} - x_i|; msm c + |x_i - x_{i-1}|
         double ad[kRows];  // twe |x_i - y| of the last column
+        double st[kRows];  // twe stiffness |c - i|: a diagonal keeps its value
         float xf[kRows];
         float pxf = 0.0f;
         double xprev = 0.0;
 #pragma unroll
-        for (int k = 0; k < kRows; k++) P[k] = x[k] = rx[k] = ad[k] = 0.0, xf[k] = 0.0f;
+        for (int k = 0; k < kRows; k++) P[k] = x[k] = rx[k] = ad[k] = st[k] = 0.0, xf[k] = 0.0f;
         double bot = 0.0, bdiag = 0.0, top = 0.0;
-        double yp = 0.0, yn = 0.0, rn = 0.0, gn = 0.0;
+        double yp = 0.0, yn = 0.0, rn = 0.0, gn = 0.0, sn = 0.0;
         float ypf = 0.0f;
         int c = -g, strip = g;
         if (g == 0) {
             yn = __ldg(Y);
             if constexpr (KIND == K_ERP) gn = __ldg(gY);
+            if constexpr (KIND == K_TWE) sn = __ldg(J.stab);
         }
         for (int64_t t = 0; t < steps; t++) {
             const double above = __shfl_up_sync(FULL, bot, 1, G);
             const bool act = c >= 0 && c < m && strip < strips;
             const double y = yn, rv = rn;
             double colv = gn;
+            const double s0 = sn;
             int c1 = c + 1, s1 = strip;
             if (c1 == period) {
                 c1 = 0;
@@ -151,6 +156,7 @@ __global__ void __launch_bounds__(32)
             if (c1 >= 0 && c1 < m && s1 < strips) {
                 yn = __ldg(Y + c1);
                 if constexpr (KIND == K_ERP) gn = __ldg(gY + c1);
+                if constexpr (KIND == K_TWE) sn = __ldg(J.stab + abs(c1 - s1 * kRows));
                 if (g == 0 && s1 > 0) rn = ring[(int64_t)c1 * slots];
             }
             if (act) {
@@ -177,6 +183,8 @@ __global__ void __launch_bounds__(32)
                         if constexpr (KIND == K_TWE) {
                             rx[k] = abs_of((k ? x[k > 0 ? k - 1 : 0] : xprev) - x[k]);
                             ad[k] = abs_of(x[k]);
+                            // of the column before the first
+                            st[k] = __ldg(J.stab + imin(i0 + k + 1, n - 1));
                             P[k] = INF;
                         }
                         if constexpr (KIND == K_MSM)
@@ -218,6 +226,9 @@ __global__ void __launch_bounds__(32)
                     if constexpr (KIND == K_TWE) {
                         colv = abs_of(yp - y);
                         adg = abs_of(xprev - yp);
+#pragma unroll
+                        for (int k = kRows - 1; k > 0; k--) st[k] = st[k - 1];
+                        st[0] = s0;
                     }
 #pragma unroll
                     for (int k = 0; k < kRows; k++) {
@@ -238,8 +249,7 @@ __global__ void __launch_bounds__(32)
                         } else {
                             const double del = nn_min(up + rx[k], lf + colv) + pen;
                             const double a = abs_of(x[k] - y);
-                            const double st = __ldg(J.stab + abs(c - imin(i0 + k, n - 1)));
-                            nv = nn_min(del, ((dg + a) + adg) + st);
+                            nv = nn_min(del, ((dg + a) + adg) + st[k]);
                             adg = ad[k];
                             ad[k] = a;
                         }
