@@ -1,7 +1,8 @@
 // dtw32.cu -- FP32 dtw / wdtw with compensated accumulation, forward and
 // backward, for batches of (possibly ragged) pairs.
 //
-// One thread per (x, y) problem, persistent: warps take 32 consecutive items
+// One thread per (x, y) problem (few problems: several lanes each, see the forward
+// of few items below), persistent: warps take 32 consecutive items
 // at a time from an atomic counter, so a batch sorted by cost keeps the 32
 // lanes of a warp on problems of similar size.  dtw items are transposed so
 // that the rows of the recurrence are the shorter series (wdtw keeps x on the

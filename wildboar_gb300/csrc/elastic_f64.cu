@@ -1,4 +1,7 @@
-// elastic_f64.cu -- FP64 elastic distances, one thread per pair.
+// elastic_f64.cu -- FP64 elastic distances, one thread per pair and every band
+// cell evaluated.  (dtw, wdtw and adtw with bands of 12 cells or more, and the
+// edit metrics over the full band, reach these kernels only with the pairs or jobs
+// that guided.cu, bit_edit.cu and elastic_wave.cu leave.)
 //
 // Layout.  A warp holds 32 pairs that share one column series (the metric's
 // Y, read with warp-uniform broadcast loads) and have 32 different row series

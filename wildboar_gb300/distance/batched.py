@@ -12,7 +12,8 @@ Three layers, all on CUDA torch tensors:
   and only supports one length per array).  The (pair, dim) problems are
   sorted by their band cell count so every warp gets problems of similar size
   (length bucketing), and the kernel configuration (rows per register strip,
-  block size) comes from ``Autotuner``.
+  block size) comes from ``Autotuner`` (for batches of more than some 29 000
+  problems; fewer take several lanes each, whatever the configuration).
 * ``BatchedDTW`` -- the same computation on fixed device buffers, captured in
   a CUDA graph after a warm-up and replayed.
 """
