@@ -12,7 +12,7 @@
 //     rows in registers, 4 columns per step) and keeps the bottom row of every
 //     strip and the cells of every S-th column (one byte per cell for S = 8,
 //     which the DRAM writes bound at about 8 ms for the shape below; S = 16
-//     halves it where S = 8 would not fit the budget);
+//     halves it where S = 8 would not fit its budget);
 //  2. walks back from (n-1, m-1) over the S x S blocks between those kept rows
 //     and columns: a block's cells are recomputed from them, every predecessor
 //     whose value lies within the error bound of the cell's smallest
@@ -57,7 +57,7 @@
 // kGuidedPending until launch_elastic's second pass over exactly those pairs.
 //
 // Measured on one GB300 (full recurrence -> guided): dtw r = 0.1, 1000 x 1000,
-// length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.3
+// length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.0
 // ms; wdtw r = 1, 500 x 403, length 256: 107 -> 9.0 ms.  Of the first, the
 // sweep takes a third, the walk a fourth and the FP64 part two fifths (2100
 // iterations for the 890 cells of a pair: lanes wait for the turn's longest
@@ -1037,8 +1037,13 @@ int blocks_per_sm(int S) {
 
 int64_t round_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
-// per-thread memory budget of the kept rows and columns of all resident pairs
-constexpr size_t kGuidedBudget = (size_t)8 << 30;
+// Budget of the kept rows and columns of all resident pairs, for blocks of 8
+// cells and of 16.  Where 8 cells need more, their rows and columns bound the
+// kernel by DRAM writes (310 x 301 pairs of 400 x 361, r = 1: 10.3 ms with 12 GB,
+// 8.1 with blocks of 16); blocks of 16 are worth every resident warp (600 x 500
+// pairs of 900, r = 0.2, 14 GB: 84 -> 71 ms against the 62 % that 8 GB hold).
+constexpr size_t kGuidedBudget8 = (size_t)8 << 30;
+constexpr size_t kGuidedBudget16 = (size_t)16 << 30;
 
 // max_pairs > 0: for lists of at most so many pairs
 Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
@@ -1093,7 +1098,8 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
             default: nb = blocks_per_sm<K_ADTW>(S); break;
         }
         const int64_t full = std::min<int64_t>(want, (int64_t)imax(nb, 1) * dev.sm_count);
-        size_t room = std::min(kGuidedBudget, avail > p.shared_bytes ? avail - p.shared_bytes : 0);
+        const size_t room = std::min(S == 8 ? kGuidedBudget8 : kGuidedBudget16,
+                                     avail > p.shared_bytes ? avail - p.shared_bytes : 0);
         const int64_t fit = (int64_t)(room / (p.thread_bytes * kThreads));
         p.grid = (int)std::min(full, fit);
         // enough resident pairs to keep the SMs busy, else larger blocks or
