@@ -926,10 +926,20 @@ guided_pairs_kernel(const GuidedArgs A) {
     const float K = (float)(B.n + B.m);
 
     for (;;) {
-        unsigned long long t64 = 0;
-        if (lane == 0) t64 = atomicAdd(&A.prep->queue, 1ull);
+        unsigned long long t64 = 0, left = 0;
+        if (lane == 0) {
+            t64 = atomicAdd(&A.prep->queue, 1ull);
+            left = *reinterpret_cast<volatile unsigned long long *>(&A.prep->heavy);
+        }
         const int64_t t = (int64_t)__shfl_sync(FULL, t64, 0);
         if (t >= ntiles) break;
+        // Where three quarters of the pairs of the first tiles were left to the full
+        // recurrence or had a fourth of a wide band's blocks collected (values that
+        // tie everywhere), the rest goes there at once: 1000 x 800 pairs of 512, one
+        // spike each, r = 0.1 242 ms (full recurrence 237), r = 1, 500 x 400 412, was 536
+        // (320); 0 / 1 values, r = 0.1 251, was 319 (237).
+        const int64_t done = t - (int64_t)gridDim.x * (kThreads / 32);
+        const bool give_up = done >= 128 && (int64_t)__shfl_sync(FULL, left, 0) >= 24 * done;
         int64_t cs = t / chunks;
         int64_t rs = (t - cs * chunks) * 32 + lane;
         if (J.mode == PM_PAIRED) {
@@ -945,6 +955,22 @@ guided_pairs_kernel(const GuidedArgs A) {
             rs = p % J.rows.count;
         }
         if (!__any_sync(FULL, active)) continue;
+        auto store = [&](double res) {
+            if (J.mode == PM_PAIRED) {
+                J.out[rs] = res;
+            } else {
+                J.out[rs * J.out_ld + cs] = res;
+                if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = res;
+            }
+        };
+        if (give_up) {
+            if (active) {
+                store(__longlong_as_double(kGuidedPending));
+                atomicAdd(&A.prep->pending, 1ull);
+                atomicAdd(&A.prep->heavy, 1ull);
+            }
+            continue;
+        }
         if (!active && !listed) {  // sweeps along on a valid pair
             rs = J.rows.count - 1;
             cs = J.mode == PM_PAIRED ? rs : cs;
@@ -995,18 +1021,16 @@ guided_pairs_kernel(const GuidedArgs A) {
         if (KIND != K_WDTW && fix) count = collect<KIND, S, KIND != K_WDTW>(A, B, D, e, live, gt, row0);
         else count = collect<KIND, S, false>(A, B, D, e, live, gt, row0);
 
+        const unsigned heavy = __ballot_sync(
+            FULL, active && (count <= 0 || (A.blocks >= 12 && 4 * count > B.ns * A.blocks)));
+        if (lane == 0 && heavy) atomicAdd(&A.prep->heavy, (unsigned long long)__popc(heavy));
+
         double value = 0.0;
         if (__any_sync(FULL, count > 0))
             value = evaluate<KIND, S>(A, A.xd + rs * A.xs + 3, A.yd + cs * A.ys, count, row0, gt,
                                       stage);
         if (active) {
-            const double res = count > 0 ? sqrt(value) : __longlong_as_double(kGuidedPending);
-            if (J.mode == PM_PAIRED) {
-                J.out[rs] = res;
-            } else {
-                J.out[rs * J.out_ld + cs] = res;
-                if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = res;
-            }
+            store(count > 0 ? sqrt(value) : __longlong_as_double(kGuidedPending));
             if (count <= 0) atomicAdd(&A.prep->pending, 1ull);
         }
     }
@@ -1232,7 +1256,7 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
 
 int guided_run(const GuidedContext &C, cudaStream_t s) {
     GuidedPrep *prep = C.args.prep;
-    WB_CUDA(cudaMemsetAsync(&prep->queue, 0, sizeof(prep->queue) + sizeof(prep->pending), s));
+    WB_CUDA(cudaMemsetAsync(&prep->queue, 0, 3 * sizeof(unsigned long long), s));
     switch (C.args.J.kind) {
         case K_DTW: return run_kernel<K_DTW>(C, s);
         case K_WDTW: return run_kernel<K_WDTW>(C, s);

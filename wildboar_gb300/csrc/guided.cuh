@@ -23,6 +23,7 @@ struct GuidedPrep {
     long long lo, hi;            // order codes of the smallest / largest input
     unsigned long long queue;    // next tile of 32 pairs
     unsigned long long pending;  // pairs left to the full recurrence
+    unsigned long long heavy;    // they and those with a fourth of their blocks collected
 };
 
 // Extremes of a series: fixed point, and the largest float magnitude.
