@@ -51,10 +51,11 @@
 // bound cannot lie on a best path.  (adtw adds a rounded penalty per move:
 // K / 2 more on either side.)
 //
-// Pairs whose collected cells do not fit the thread's list (half of the
-// band's blocks: long runs of equal values tie everywhere) or whose inputs
+// Pairs whose collected cells do not fit the thread's list (a fourth to half of
+// the band's blocks: long runs of equal values tie everywhere) or whose inputs
 // are not finite are left to the full recurrence: their output holds
-// kGuidedPending until launch_elastic's second pass over exactly those pairs.
+// kGuidedPending until guided_tail_kernel (few pairs) or launch_elastic's second
+// pass over exactly those pairs.
 //
 // Measured on one GB300 (full recurrence -> guided): dtw r = 0.1, 1000 x 1000,
 // length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.0
@@ -1037,6 +1038,137 @@ guided_pairs_kernel(const GuidedArgs A) {
 }
 
 // --------------------------------------------------------------------------
+// Few pairs left over: the full recurrence of a pair on the 32 lanes of a warp,
+// lane l on strips l, l + 32, .. of 8 rows, one column per step and one behind lane
+// l - 1, whose bottom cell it takes by shuffle (lane 0: from a row in memory that
+// lane 31 wrote); the cells' operations are the strip kernel's.  One thread per
+// pair, as the second pass has them, takes 330 cycles for every cell: a single
+// pair of 400 x 361, r = 1, kept the call waiting for 13 ms, here 1.
+constexpr int kTailRows = 8;
+constexpr int64_t kTailPairs = 2048;  // more of them fill the second pass's warps
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) guided_tail_kernel(const GuidedArgs A) {
+    constexpr int S = kTailRows, G = 32;
+    const unsigned FULL = 0xffffffffu;
+    const ElasticJob &J = A.J;
+    const unsigned long long left = A.prep->pending;
+    if (left == 0 || left > (unsigned long long)kTailPairs) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
+    const int64_t warps = ((int64_t)gridDim.x * kThreads) >> 5;
+    double *row = A.brow + warp * A.brow_cols;
+    const Band B(J, S);
+    const int n = B.n, m = B.m, lim = imin(m, B.mx);
+    const double INF = WB_DBL_INF;
+    const int strips = B.ns;
+    // steps from a round to the next: every lane is done with its strip and its
+    // row is written a step before lane 0 reads it
+    const int delta = imax(G + 2, imin(m, S + B.mx + B.mn + B.r - 2 - G * S));
+    const int steps = (strips - 1) / G * delta + ((strips - 1) & (G - 1)) + m;
+    const int64_t total = J.mode == PM_PAIRED ? J.rows.count : J.rows.count * J.cols.count;
+    for (int64_t base = warp * 32; base < total; base += warps * 32) {
+        const int64_t p = base + lane;
+        int64_t rs = p, cs = p;
+        if (J.mode != PM_PAIRED) {
+            rs = p / J.cols.count;
+            cs = p - rs * J.cols.count;
+        }
+        bool mine = p < total && !(J.mode == PM_UPPER && rs >= cs);
+        if (mine) mine = is_pending(J.mode == PM_PAIRED ? J.out[rs] : J.out[rs * J.out_ld + cs]);
+        for (unsigned todo = __ballot_sync(FULL, mine); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const int64_t r1 = __shfl_sync(FULL, rs, src), c1 = __shfl_sync(FULL, cs, src);
+            const double *X = J.rows.base + r1 * J.rows.stride;
+            const double *Y = J.cols.base + c1 * J.cols.stride;
+            double P[S], x[S], result = 0.0, acc = 0.0, bot = INF, bdiag = INF, before = INF;
+#pragma unroll
+            for (int k = 0; k < S; k++) P[k] = INF, x[k] = 0.0;
+            const double x0 = X[0];
+            int s = lane, c = -lane;
+            for (int t = 0; t < steps; t++) {
+                const double above = __shfl_up_sync(FULL, bot, 1);
+                const bool any = s < strips;
+                const int i0 = 1 + s * S;
+                const int first = any ? B.cs(s, S) : m, end = any ? B.ce(s, S) : m;
+                const int pfirst = any ? B.cs(s - 1, S) : 0, pend = any ? B.ce(s - 1, S) : 0;
+                double up = above;
+                if (lane == 0 && any) {
+                    up = INF;
+                    if (s > 0) {
+                        if (c >= pfirst && c < pend) up = row[c];
+                    } else if (c < lim) {
+                        const double v = x0 - __ldg(Y + c);
+                        double cst = v * v;
+                        if (KIND == K_WDTW) cst = cst * __ldg(J.weights + imax(c - 1, 0));
+                        acc = c == 0 ? cst : acc + cst;
+                        up = acc;
+                    }
+                }
+                const double raw = up;
+                if (any && c >= first) {
+                    if (c == first) {
+                        bdiag = INF;
+                        if (c > pfirst && c <= pend) {
+                            bdiag = before;
+                            if (lane == 0 && s > 0) bdiag = row[c - 1];
+                        }
+#pragma unroll
+                        for (int k = 0; k < S; k++) {
+                            P[k] = INF;
+                            x[k] = X[imin(i0 + k, n - 1)];
+                        }
+                    }
+                    if (c >= pend) up = INF;
+                    const double y = __ldg(Y + c), above_cell = up;
+                    double dg = bdiag;
+#pragma unroll
+                    for (int k = 0; k < S; k++) {
+                        const int d = c - (i0 + k);
+                        const double lf = P[k], v = x[k] - y;
+                        double cst = v * v;
+                        if (KIND == K_WDTW)
+                            cst = cst * __ldg(J.weights + abs(c - imin(i0 + k, n - 1)));
+                        double mv = nn_min(up, lf);
+                        if (KIND == K_ADTW) mv = mv + J.p;
+                        double nv = nn_min(mv, dg) + cst;
+                        if (d < B.lo || d > B.mx - 1) nv = INF;
+                        dg = lf;
+                        up = nv;
+                        P[k] = nv;
+                    }
+                    bot = P[S - 1];
+                    bdiag = above_cell;
+                    if (lane == G - 1 && s + 1 < strips) row[c] = bot;
+                    if (s == strips - 1 && c == m - 1) {
+#pragma unroll
+                        for (int k = 0; k < S; k++)
+                            if (i0 + k < n) result = P[k];
+                    }
+                }
+                before = raw;
+                c++;
+                if (any && c >= end) {
+                    s += G;
+                    c -= delta;
+                }
+                __syncwarp();
+            }
+            const double v = sqrt(__shfl_sync(FULL, result, (strips - 1) & (G - 1)));
+            if (lane == 0) {
+                if (J.mode == PM_PAIRED) {
+                    J.out[r1] = v;
+                } else {
+                    J.out[r1 * J.out_ld + c1] = v;
+                    if (J.mode == PM_UPPER) J.out[c1 * J.out_ld + r1] = v;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// --------------------------------------------------------------------------
 // host side
 
 struct Plan {
@@ -1100,7 +1232,11 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
         p.S = S;
         p.groups = (imin(m, width + S - 1) + 3) / 4 + 1;
         p.blocks = p.groups / (S / 4) + 2;
-        p.list_cap = imax((n + m) / S + 8, ns * p.blocks / 2);
+        // a wide band's pairs with more of its blocks are faster in guided_tail_kernel
+        // (a list's pairs have no such pass: half); 600 x 500 pairs of 900, r =
+        // 0.2: 58 to 61 ms, with half of them 64 to 102, waiting for one pair
+        p.list_cap = imax((n + m) / S + 8,
+                          ns * p.blocks / (max_pairs > 0 || p.blocks < 12 ? 2 : 4));
         p.brow_cols = (int)round_up(m, S);
         p.xs = round_up(3 + 1 + (int64_t)ns * S, 4);
         p.ys = round_up(m, 16);
@@ -1140,6 +1276,17 @@ int run_kernel(const GuidedContext &C, cudaStream_t s) {
     if (C.S == 8) guided_pairs_kernel<KIND, 8><<<C.grid, kThreads, 0, s>>>(C.args);
     else guided_pairs_kernel<KIND, 16><<<C.grid, kThreads, 0, s>>>(C.args);
     WB_LAUNCH_CHECK("guided_pairs_kernel");
+    return WB_OK;
+}
+
+int run_tail(const GuidedContext &C, cudaStream_t s) {
+    const int grid = imin(C.grid, 4 * device_info().sm_count);
+    switch (C.args.J.kind) {
+        case K_DTW: guided_tail_kernel<K_DTW><<<grid, kThreads, 0, s>>>(C.args); break;
+        case K_WDTW: guided_tail_kernel<K_WDTW><<<grid, kThreads, 0, s>>>(C.args); break;
+        default: guided_tail_kernel<K_ADTW><<<grid, kThreads, 0, s>>>(C.args); break;
+    }
+    WB_LAUNCH_CHECK("guided_tail_kernel");
     return WB_OK;
 }
 
@@ -1273,6 +1420,7 @@ int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
     timer_begin("guided_pairs_kernel", ws.stream());
     WB_TRY(guided_run(C, ws.stream()));
     timer_end(ws.stream());
+    WB_TRY(run_tail(C, ws.stream()));
     *pending = &C.args.prep->pending;
     return WB_OK;
 }
