@@ -58,7 +58,7 @@
 // pass over exactly those pairs.
 //
 // Measured on one GB300 (full recurrence -> guided): dtw r = 0.1, 1000 x 1000,
-// length 512: 292 -> 40 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.0
+// length 512: 292 -> 36 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.3
 // ms; wdtw r = 1, 500 x 403, length 256: 107 -> 9.0 ms.  Of the first, the
 // sweep takes a third, the walk a fourth and the FP64 part two fifths (2100
 // iterations for the 890 cells of a pair: lanes wait for the turn's longest
