@@ -77,13 +77,17 @@ constexpr int kThreads = 128;
 constexpr unsigned kCap = 1u << 30;  // saturated value, and out of band
 constexpr int kFixOne = (1 << 29) - 1;  // 1.0 in fixed point
 
-// Smallest and largest value of both series sets.
+// Smallest and largest value of both series sets.  (The second is passed over
+// only as the very same set: device arrays are used in place, so a set may
+// start where the other does and hold more of it.)
 __global__ void __launch_bounds__(256)
 guided_range_kernel(const SeriesSet a, const SeriesSet b, GuidedPrep *prep) {
     double lo = WB_DBL_INF, hi = -WB_DBL_INF;
     for (int set = 0; set < 2; set++) {
         const SeriesSet &S = set ? b : a;
-        if (set && b.base == a.base) break;
+        if (set && b.base == a.base && b.stride == a.stride && b.len == a.len &&
+            b.count == a.count)
+            break;
         const int64_t total = S.count * (int64_t)S.len;
         for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total;
              t += (int64_t)gridDim.x * 256) {
