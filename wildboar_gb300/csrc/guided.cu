@@ -48,8 +48,9 @@
 //   A(p) <= A(q) + K + 16 2^-24 A_max + 4 e sqrt(K) sqrt(A_max) + 4 e^2 K,
 // A the swept values, A_max a bound of A along the path from its value at
 // (n-1, m-1); the constants below are rounded up.  Predecessors outside that
-// bound cannot lie on a best path.  (adtw adds a rounded penalty per move:
-// K / 2 more on either side.)
+// bound cannot lie on a best path, nor can saturated ones: the sums along the
+// path stay below A_max, and pairs whose bound would reach from there to kCap are
+// not taken.  (adtw adds a rounded penalty per move: K / 2 more on either side.)
 //
 // Pairs whose collected cells do not fit the thread's list (a fourth to half of
 // the band's blocks: long runs of equal values tie everywhere) or whose inputs
@@ -599,7 +600,8 @@ __device__ __forceinline__ void block_bits(const GuidedArgs &A, const Band &B, i
                 const unsigned up = i == 0 ? top[q] : Q[j];
                 const unsigned lf = P[i];
                 const unsigned best = best_of<KIND>(dg, up, lf, pen);
-                const int t = (int)(best + tol);
+                // (saturated cells, those out of band among them, are never kept)
+                const int t = (int)__viaddmin_u32(best, tol, kCap - 1u);
                 const int tm = KIND == K_ADTW ? t - (int)pen : t;
                 bd_ = push_sign(bd_, t - (int)dg);
                 bu_ = push_sign(bu_, tm - (int)up);
@@ -658,7 +660,7 @@ __device__ __forceinline__ int collect(const GuidedArgs &A, const Band &B, const
         __fmaf_ru(KIND == K_ADTW ? 2.02f : 1.01f, K,
                   FIX ? 0.0f : __fmul_ru(1.2e-6f, __fmul_ru(ra, ra))),
         __fadd_ru(__fmul_ru(__fmul_ru(4.2f, ek), __fadd_ru(ra, ek)), 8.0f));
-    live = live && au < kCap && tolf < 2.5e8f;
+    live = live && au < kCap && tolf < 2.5e8f && __fadd_ru((float)au, tolf) < (float)kCap;
     const unsigned tol = live ? (unsigned)tolf : 0u;
 
     int s = B.ns - 1, b = (B.m - 1) / S;
