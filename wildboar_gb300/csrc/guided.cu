@@ -994,7 +994,8 @@ guided_pairs_kernel(const GuidedArgs A) {
         float e = __fmaf_ru(6.0e-8f, __fadd_ru(rx.mag, ry.mag), 1e-37f);
         float ub = __fsqrt_ru(straight_path<KIND>(A, B, D.xf, D.yf, penf));
         ub = __fmaf_ru(e, __fsqrt_ru(K), ub);
-        ub = fmaxf(__fmul_ru(ub, ub), 1e-30f);
+        // (from 2^-97 on units are at most 2^124, so that a penalty of 0 stays 0)
+        ub = fmaxf(__fmul_ru(ub, ub), 0x1p-97f);
         const bool live = active && finite && ub < 1e30f;
         const int lub = ilogbf(ub);
         // Fixed point: units of d^2 2^(26 + 2k) (d the scaled difference), the
