@@ -77,3 +77,15 @@ def test_wdtw_argmin(monkeypatch, g):
     monkeypatch.setenv("WB_GPU_ARGMIN", "all")
     for a, b in zip(got, argmin_distance(X, Y, **kw)):
         np.testing.assert_array_equal(a, b)
+
+
+# penalties just above a float: each move is off by up to 2^-23 of it
+@pytest.mark.parametrize("length", [25, 28, 60, 300])
+@pytest.mark.parametrize("moves", [2, 8, 40])
+def test_adtw_penalty_rounding(monkeypatch, length, moves):
+    rng = np.random.default_rng(length)
+    X = rng.integers(-512, 513, (64, length)) / 512.0
+    Y = np.roll(X[:12], 2, axis=1)
+    X[0, 0], X[0, 1] = -1.0, 1.0
+    p = (1.0 + 2.0 ** -23 + 2.0 ** -40) * length / (8.0 * moves)
+    _check(monkeypatch, X, Y, "adtw", {"r": 0.5, "p": p})

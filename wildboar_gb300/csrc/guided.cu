@@ -50,7 +50,9 @@
 // (n-1, m-1); the constants below are rounded up.  Predecessors outside that
 // bound cannot lie on a best path, nor can saturated ones: the sums along the
 // path stay below A_max, and pairs whose bound would reach from there to kCap are
-// not taken.  (adtw adds a rounded penalty per move: K / 2 more on either side.)
+// not taken.  (adtw adds a rounded penalty per move: K / 2 more on either side,
+// and in fixed point too 2^-23 + 2^-24 of A_max on either side, since the penalty
+// is a float before it is in units.)
 //
 // Pairs whose collected cells do not fit the thread's list (a fourth to half of
 // the band's blocks: long runs of equal values tie everywhere) or whose inputs
@@ -658,7 +660,7 @@ __device__ __forceinline__ int collect(const GuidedArgs &A, const Band &B, const
         __fmaf_ru(2.1f, ek, __fmul_ru(__fsqrt_ru(__fadd_ru((float)au, K)), 1.000001f));
     const float tolf = __fadd_ru(
         __fmaf_ru(KIND == K_ADTW ? 2.02f : 1.01f, K,
-                  FIX ? 0.0f : __fmul_ru(1.2e-6f, __fmul_ru(ra, ra))),
+                  __fmul_ru(FIX ? (KIND == K_ADTW ? 4e-7f : 0.0f) : 1.2e-6f, __fmul_ru(ra, ra))),
         __fadd_ru(__fmul_ru(__fmul_ru(4.2f, ek), __fadd_ru(ra, ek)), 8.0f));
     live = live && au < kCap && tolf < 2.5e8f && __fadd_ru((float)au, tolf) < (float)kCap;
     const unsigned tol = live ? (unsigned)tolf : 0u;
