@@ -505,7 +505,8 @@ __global__ void __launch_bounds__(128) dot_exact_kernel(const DotArgs A) {
     }
 }
 
-// smallest sum of each pair, the first window of equal ones
+// smallest sum of each pair, the first window of equal ones; a pair without a
+// finite one goes to the FP64 scan, which takes no window of an infinite sum
 __global__ void __launch_bounds__(256)
 dot_select_kernel(const DotArgs A, int64_t pairs, unsigned long long *redo) {
     const int64_t pair = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -524,6 +525,11 @@ dot_select_kernel(const DotArgs A, int64_t pairs, unsigned long long *redo) {
             best = d;
             at = w;
         }
+    }
+    if (!(best < WB_DBL_INF)) {
+        A.kept[pair] = 0;
+        atomicAdd(redo, 1ull);
+        return;
     }
     A.J.out_dist[pair] = sqrt(best);
     A.J.out_idx[pair] = at;

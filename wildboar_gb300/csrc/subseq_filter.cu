@@ -344,7 +344,8 @@ subseq_exact_kernel(const FilterArgs A, double *gring, int P) {
     }
 }
 
-// the smallest sum of each pair, the first window of equal ones
+// the smallest sum of each pair, the first window of equal ones; a pair without
+// a finite one goes to the FP64 scan, which takes no window of an infinite sum
 __global__ void __launch_bounds__(256)
 subseq_select_kernel(const FilterArgs A, int64_t pairs, unsigned long long *redo) {
     const int64_t pair = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -361,6 +362,11 @@ subseq_select_kernel(const FilterArgs A, int64_t pairs, unsigned long long *redo
             best = A.sums[pair * kKeep + q];
             at = A.windows[pair * kKeep + q];
         }
+    if (!(best < WB_DBL_INF)) {
+        A.kept[pair] = 0;
+        atomicAdd(redo, 1ull);
+        return;
+    }
     A.J.out_dist[pair] = sqrt(best);
     A.J.out_idx[pair] = at;
 }
