@@ -231,6 +231,11 @@ typedef struct wb_dtw32 {
 /* dtw distance of every item: out[t] = sqrt(cost), out_cost[t] = cost (or NULL) */
 int wb_dtw32_distance(const wb_dtw32 *job, double *out, double *out_cost, void *stream);
 
+/* How wb_dtw32_distance (keep != 0: wb_dtw32_distance_keep) would run the job:
+ * the rows per strip where several lanes share an item, 0 for one thread per
+ * item, -1 for an invalid job.  No device work. */
+int32_t wb_dtw32_lanes(const wb_dtw32 *job, int32_t keep);
+
 /* d distance[t] / d x and d distance[t] / d y of every item, scaled by
  * grad_out[t] (NULL = 1): grad_x row t at grad_x + t * gx_stride (x_len
  * floats), grad_y likewise.  Recomputes the forward with a direction bitmap

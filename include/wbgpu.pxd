@@ -126,6 +126,7 @@ cdef extern from "wbgpu.h" nogil:
     int wb_dtw32_distance(const wb_dtw32 *job, double *out, double *out_cost, void *stream)
     int wb_dtw32_backward(const wb_dtw32 *job, const double *grad_out, float *grad_x,
                           int64_t gx_stride, float *grad_y, int64_t gy_stride, void *stream)
+    int32_t wb_dtw32_lanes(const wb_dtw32 *job, int32_t keep)
     int64_t wb_dtw32_keep_bytes(const wb_dtw32 *job)
     int wb_dtw32_distance_keep(const wb_dtw32 *job, double *out, double *out_cost,
                                void *keep, int64_t keep_bytes, void *stream)

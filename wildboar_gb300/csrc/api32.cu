@@ -197,6 +197,18 @@ extern "C" int wb_dtw32_distance(const wb_dtw32 *q, double *out, double *out_cos
     return dtw32_forward(J, q->strip ? q->strip : 16, s);
 }
 
+extern "C" int32_t wb_dtw32_lanes(const wb_dtw32 *q, int32_t keep) {
+    WB_TRACE();
+    Dtw32Job J;
+    size_t bytes = 0;
+    if (dtw32_plan(q, false, J, bytes) != WB_OK) return -1;
+    if (keep) {
+        J.wave = 0;
+        if (q->grid <= 0) dtw32_wave_keep_plan(J);
+    }
+    return J.wave > 0 ? J.wave_rows : 0;
+}
+
 extern "C" int wb_dtw32_backward(const wb_dtw32 *q, const double *grad_out, float *grad_x,
                                  int64_t gx_stride, float *grad_y, int64_t gy_stride,
                                  void *stream_) {

@@ -1347,12 +1347,31 @@ __global__ void __launch_bounds__(kWaveBlock, NB)
     }
 }
 
+// Whether the steps of every item of the job, times its passes, stay within an int
+// (wave_item, the kernel's choice of G).  With G lanes and q items a turn that is
+// at most (strips / G delta(G) + m / 2 + G) G q / 32, q / 32 <= 1 / 8; an item with
+// lengths of its own may have a band of any width.  At r = 1 that ends at a length
+// of some 300 000 points, whose cells take one thread per item hours as well.
+template <int S>
+static bool wave_counts_fit(const Dtw32Job &J) {
+    const int64_t n = imin(J.x_len, J.y_len), m = imax(J.x_len, J.y_len);
+    int64_t reach = m;  // columns from a strip's first to the end of the band
+    if (!J.xlen && !J.ylen) {
+        const int64_t r = (J.band_fixed > 0 ? J.band_fixed : imax((int)(n * J.r), 1)) + 2;
+        reach = std::min(m, m - n + 2 * r + S);
+    }
+    const int64_t strips = (n - 1 + S - 1) / S;
+    const int64_t delta = std::max<int64_t>(34, reach / 2 + 1);
+    return strips * delta / 8 + 4 * (m / 2 + 1 + delta + 32) < (int64_t)1 << 30;
+}
+
 // Items per turn and blocks of the kernel.  A turn of few items on more lanes
 // each takes fewer steps, which counts until every scheduler has a warp.  (Items
 // with lengths: as for a third and two thirds of the longest.)  The kernel's
 // rows take no more of the ring than one thread per item does.
 template <int S>
 static void wave_grid(Dtw32Job &J, int per_sm) {
+    if (!wave_counts_fit<S>(J)) return;
     const int64_t sms = device_info().sm_count, warps = kWaveBlock / 32;
     WaveGeom<S> w{};
     w.n = imin(J.x_len, J.y_len);
@@ -1395,7 +1414,8 @@ static void wave_grid(Dtw32Job &J, int per_sm) {
 //   1024 each, r = 0.1, 20000               3.7      2.9      2.6      2.6
 //   1024 each, r = 0.1, 120000             12.0     15.8     13.2     14.1
 //   64 each, r = 0.1, 10000                 0.072    0.077    0.091    0.117
-// so: up to 6 warps' worth of items per SM, fewer for short series.
+// so: up to 6 warps' worth of items per SM, fewer for short series.  (Series so long that
+// a step count would leave the int range keep one thread per item.)
 void dtw32_wave_plan(Dtw32Job &J) {
     J.wave = 0;
     if (J.weights) return;
