@@ -11,7 +11,6 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <numeric>
 #include <vector>
@@ -102,68 +101,6 @@ const DeviceInfo &device_info() {
         have[dev] = true;
     }
     return cache[dev];
-}
-
-// --------------------------------------------------------------------------
-// workspace
-
-static std::mutex g_arena_mu;
-static std::map<std::pair<int, cudaStream_t>, Arena *> g_arenas;
-
-static Arena *arena_for(cudaStream_t s) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> g(g_arena_mu);
-    auto key = std::make_pair(dev, s);
-    auto it = g_arenas.find(key);
-    if (it != g_arenas.end()) return it->second;
-    Arena *a = new Arena();
-    g_arenas[key] = a;
-    return a;
-}
-
-Workspace::Workspace(cudaStream_t stream)
-    : arena_(arena_for(stream)), stream_(stream), lock_(arena_->mu) {
-    arena_->used = 0;
-}
-
-Workspace::~Workspace() { arena_->used = 0; }
-
-int Workspace::reserve(size_t bytes, size_t least) {
-    if (injected(INJ_RESERVE))
-        return fail(WB_ENOMEM, "cannot allocate device workspace (injected fault)");
-    bytes = align256(bytes) + 4096;
-    least = align256(least) + 4096;
-    // (a size that the device had no room for is not asked for again while the
-    // arena holds what the call needs)
-    if (bytes > arena_->cap && !(least <= arena_->cap && bytes >= arena_->denied)) {
-        if (arena_->base) {
-            // cudaFree waits for the device, so earlier work on this stream
-            // that still reads the arena has finished
-            cudaError_t e = cudaFree(arena_->base);
-            arena_->base = nullptr;
-            arena_->cap = 0;
-            if (e != cudaSuccess) return cuda_fail(e, "cudaFree(workspace)");
-        }
-        size_t cap = bytes + std::min(bytes / 4, (size_t)256 << 20);
-        cudaError_t e = cudaMalloc((void **)&arena_->base, cap);
-        while (e == cudaErrorMemoryAllocation && cap > least) {
-            cudaGetLastError();
-            arena_->denied = std::min(arena_->denied, cap);
-            cap = std::max(cap / 2, least);
-            e = cudaMalloc((void **)&arena_->base, cap);
-        }
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            arena_->base = nullptr;
-            if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMalloc(workspace)");
-            return fail(WB_ENOMEM, "cannot allocate " + std::to_string(cap) +
-                                       " bytes of device workspace");
-        }
-        arena_->cap = cap;
-    }
-    arena_->used = 0;
-    return WB_OK;
 }
 
 // --------------------------------------------------------------------------
@@ -1467,23 +1404,3 @@ extern "C" const char *wb_last_error(void) { return g_last_error.c_str(); }
 extern "C" int32_t wb_version(void) { return 1; }
 
 extern "C" int64_t wb_launch_count(void) { return g_launches.load(); }
-
-extern "C" int wb_release_workspace(void *stream_) {
-    WB_TRACE();
-    std::lock_guard<std::mutex> g(g_arena_mu);
-    for (auto it = g_arenas.begin(); it != g_arenas.end();) {
-        if (stream_ == nullptr || it->first.second == (cudaStream_t)stream_) {
-            Arena *a = it->second;
-            std::lock_guard<std::mutex> ga(a->mu);
-            if (a->base) cudaFree(a->base);
-            a->base = nullptr;
-            a->cap = 0;
-            it = g_arenas.erase(it);
-            // the arena object itself is kept alive: a concurrent Workspace
-            // may still hold a pointer to it
-        } else {
-            ++it;
-        }
-    }
-    return WB_OK;
-}

@@ -74,7 +74,7 @@ struct Arena {
     char *base = nullptr;
     size_t cap = 0;
     size_t used = 0;
-    size_t denied = SIZE_MAX;  // smallest size the device had no room for
+    size_t refused = 0;  // room of the device when it last refused a size (0: it did not)
     std::mutex mu;
 };
 
@@ -87,8 +87,8 @@ class Workspace {
     // the call's total exceeds it.  Must be called before any pointer from
     // this call is used (all requests are made up front by `plan`).
     int reserve(size_t bytes) { return reserve(bytes, bytes); }
-    // the same, content with any amount from `least` up when the device has no
-    // room for `bytes` (a consumer sizes itself by `remaining`)
+    // the same, content with any amount from `least` up where the device has no
+    // room for `bytes` (workspace.cu; a consumer sizes itself by `remaining`)
     int reserve(size_t bytes, size_t least);
     size_t remaining() const { return arena_->cap - arena_->used; }
     // nullptr when the call's reservation is exhausted (see WB_TAKE)
