@@ -1,6 +1,7 @@
 """The device workspace (csrc/workspace.cu) over a fake CUDA runtime with a
 settable amount of memory: how much a call gets, and that calls repeated where
-memory is short neither reallocate each time nor stay small once there is room."""
+memory is short neither reallocate each time nor stay small once there is room.
+And the kernels' shared-memory limits, which a call never lowers."""
 
 import ctypes
 import os
@@ -23,7 +24,14 @@ bool injected(int) { return false; }
 int fail(int code, const std::string &) { return code; }
 int cuda_fail(cudaError_t, const char *) { return WB_ECUDA; }
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
+const DeviceInfo &device_info() {
+    static DeviceInfo d;
+    d.max_smem_optin = 232448;
+    return d;
 }
+}
+static std::map<const void *, int> g_limit;
+static long g_sets;
 extern "C" {
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
@@ -44,6 +52,21 @@ cudaError_t cudaMalloc(void **p, size_t n) {
     return cudaSuccess;
 }
 cudaError_t cudaFree(void *p) { g_free += g_blocks[p]; g_blocks.erase(p); return cudaSuccess; }
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes *a, const void *k) {
+    *a = cudaFuncAttributes();
+    a->sharedSizeBytes = 8192;
+    a->maxDynamicSharedSizeBytes = g_limit.count(k) ? g_limit[k] : 49152 - 8192;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void *k, cudaFuncAttribute, int v) {
+    g_sets++;
+    if (v > 232448 - 8192) return cudaErrorInvalidValue;
+    g_limit[k] = v;
+    return cudaSuccess;
+}
+int t_allow(long kernel, size_t bytes) { return wb::allow_shared((const void *)kernel, bytes); }
+int t_limit(long kernel) { return g_limit[(const void *)kernel]; }
+long t_sets() { return g_sets; }
 // a call that reserves: what it has, or a negative status
 int64_t t_reserve(long stream, size_t bytes, size_t least) {
     wb::Workspace ws((cudaStream_t)stream);
@@ -80,6 +103,9 @@ def ws(tmp_path, monkeypatch):
     L.t_set.argtypes = [size, size, ctypes.c_int]
     L.t_free.restype = size
     L.t_mallocs.restype = ctypes.c_long
+    L.t_allow.argtypes = [ctypes.c_long, size]
+    L.t_limit.argtypes = [ctypes.c_long]
+    L.t_sets.restype = ctypes.c_long
     L.wb_release_workspace.argtypes = [ctypes.c_void_p]
     return L
 
@@ -159,3 +185,20 @@ def test_the_budget(ws, monkeypatch):
     assert 74 * MB <= got <= 100 * MB
     monkeypatch.setenv("WB_GPU_WORKSPACE_MB", "0")
     assert ws.t_reserve(2, 6 * GB, 10 * MB) <= 14 * MB
+
+
+def test_a_shared_memory_limit_is_never_lowered(ws):
+    # a large call raises the limit, a small one of another thread comes before
+    # the large call's launch
+    assert ws.t_allow(1, 100_000) == 0 and ws.t_allow(1, 2_000) == 0
+    assert ws.t_limit(1) >= 100_000
+    assert ws.t_allow(1, 224_256) == 0 and ws.t_sets() == 1  # set once, to all there is
+    assert ws.t_allow(1, 224_257) != 0  # more than the device has
+    assert ws.t_allow(2, 40_000) == 0 and ws.t_sets() == 2  # within the default
+
+
+def test_no_call_sets_a_limit_by_itself():
+    csrc = os.path.join(ROOT, "wildboar_gb300", "csrc")
+    for f in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, f)) as fh:
+            assert f == "workspace.cu" or "MaxDynamicSharedMemorySize" not in fh.read(), f

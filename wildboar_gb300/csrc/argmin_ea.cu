@@ -375,8 +375,7 @@ int launch_argmin_ea(const ElasticJob &J, int metric, int xl, int yl, int64_t j0
     if (pl.form == 1) {
         const size_t smem = (size_t)pl.P * kEaThreads * sizeof(double);
         auto run = [&](auto kfn) -> int {
-            WB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+            WB_CUDA(allow_shared(kfn, smem));
             kfn<<<grid, kEaThreads, smem, s>>>(J, C, pl.P);
             WB_LAUNCH_CHECK("argmin_ea_kernel");
             return WB_OK;

@@ -488,8 +488,7 @@ int GuidedArgmin::prepare(const ElasticJob &J, Workspace &ws, size_t leave, bool
         transpose_kernel<<<tg, 256, 0, s>>>(A.xf, A.xs, J.rows.count, J.rows.len, xt, ld);
         WB_LAUNCH_CHECK("transpose_kernel");
         const size_t smem = (size_t)4 * J.cols.len * sizeof(float);
-        WB_CUDA(cudaFuncSetAttribute(envelope_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+        WB_CUDA(allow_shared(envelope_kernel, smem));
         const int64_t cap = (int64_t)device_info().sm_count * 8;
         envelope_kernel<<<(int)std::min(cap, J.cols.count), 256, smem, s>>>(J, A.yf, A.ys, env);
         WB_LAUNCH_CHECK("envelope_kernel");

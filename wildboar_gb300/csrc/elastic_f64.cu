@@ -139,8 +139,7 @@ static int launch_kind(const ElasticJob &J, Workspace &ws, int P, bool gring_mod
     } else {
         size_t smem = (size_t)P * kThreads * sizeof(double);
         auto kfn = elastic_pairs_kernel<KIND, false>;
-        WB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+        WB_CUDA(allow_shared(kfn, smem));
         if (!J.pending) timer_begin("elastic_pairs_kernel", s);
         kfn<<<grid, kThreads, smem, s>>>(J, nullptr, P);
     }
@@ -570,8 +569,7 @@ int launch_elastic_shared_ring(const ElasticJob &J, cudaStream_t s) {
 #define WB_SHR_CASE(K)                                                                   \
     case K: {                                                                            \
         auto kfn = elastic_pairs_kernel<K, false>;                                       \
-        WB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                     (int)smem));                                        \
+        WB_CUDA(allow_shared(kfn, smem));                                                \
         kfn<<<pl.grid, kThreads, smem, s>>>(J, nullptr, pl.P);                            \
         break;                                                                           \
     }

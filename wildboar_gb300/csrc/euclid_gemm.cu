@@ -589,14 +589,7 @@ int euclid_tc(const double *x, int64_t sx, int M, const double *y, int64_t sy, i
     WB_TRY(make_map(&mBl, blo, Np, Kp, kBN));
     // stage ring + one staging block of 32 x 17 floats per epilogue warp + alignment slack
     const int smem = kStages * kStageBytes + kEpiWarps * 32 * 17 * 4 + 1024;
-    static bool smem_set[64] = {};  // per device ordinal
-    int devno = 0;
-    WB_CUDA(cudaGetDevice(&devno));
-    if (devno < 0 || devno >= 64 || !smem_set[devno]) {
-        WB_CUDA(cudaFuncSetAttribute(euclid_tc_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        if (devno >= 0 && devno < 64) smem_set[devno] = true;
-    }
+    WB_CUDA(allow_shared(euclid_tc_kernel, smem));
     const int ntiles = (Mp / kBM) * (Np / kBN);
     const int grid = std::min(ntiles, device_info().sm_count);
     timer_begin("euclid_tc_kernel", s);

@@ -600,8 +600,7 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
             SubseqJob Jf = J;
             WB_TRY(make_f32_copies(J, norm, ws, Jf));
             auto kt = subseq_scaled_tiled_kernel;
-            WB_CUDA(cudaFuncSetAttribute(kt, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)tsm));
+            WB_CUDA(allow_shared(kt, tsm));
             const int64_t tb = J.x.count * J.n_chunks;
             const int tgrid = (int)(tb < cap ? tb : cap);
             if (!J.kept) timer_begin("subseq_scaled_tiled_kernel", s);
@@ -611,7 +610,7 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
             return WB_OK;
         }
         auto k = subseq_scan_kernel<true>;
-        WB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        WB_CUDA(allow_shared(k, smem));
         if (!J.kept) timer_begin("subseq_scan_kernel<scaled>", s);
         k<<<grid, kSubThreads, smem, s>>>(J, norm, mean_tab, std_tab);
         if (!J.kept) timer_end(s);
@@ -632,7 +631,7 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
         // T (doubles), its float copy and the max |t| word
         const size_t fsmem = (size_t)J.x.len * 12 + 16;
         auto k = subseq_scan_kernel<false>;
-        WB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+        WB_CUDA(allow_shared(k, fsmem));
         if (!J.kept) timer_begin("subseq_scan_kernel", s);
         k<<<grid, kSubThreads, fsmem, s>>>(Jf, nullptr, nullptr, nullptr);
         if (!J.kept) timer_end(s);

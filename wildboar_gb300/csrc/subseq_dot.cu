@@ -649,7 +649,7 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
         WB_LAUNCH_CHECK("dot_series_kernel");
         quad<<<quad_grid, 64, 0, s>>>(A, nq);
         WB_LAUNCH_CHECK("quad_kernel");
-        WB_CUDA(cudaFuncSetAttribute(filter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        WB_CUDA(allow_shared(filter, smem));
         timer_begin("dot_filter_kernel", s);
         filter<<<(unsigned)std::min<int64_t>(J.x.count * nu, (int64_t)1 << 30), kThreads, smem, s>>>(A);
         timer_end(s);

@@ -439,8 +439,7 @@ int launch_subseq_filter(SubseqElasticJob &J, int64_t total, double *gring, int 
         4, std::min<int64_t>(64, J.x.count * m / std::max<int64_t>(want, 1)));
     const int64_t blocks = J.x.count * ((m + A.per_block - 1) / A.per_block);
     const size_t smem = (size_t)(J.x.len + 2 * kPad) * sizeof(float);
-    WB_CUDA(cudaFuncSetAttribute(subseq_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+    WB_CUDA(allow_shared(subseq_filter_kernel, smem));
     timer_begin("subseq_filter_kernel", s);
     subseq_filter_kernel<<<(unsigned)std::min<int64_t>(blocks, (int64_t)1 << 30), kThreads, smem,
                            s>>>(A);

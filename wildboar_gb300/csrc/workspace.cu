@@ -1,5 +1,5 @@
 // workspace.cu -- the device workspace: one arena per (device, stream),
-// bump-allocated per call.
+// bump-allocated per call; the kernels' limits of shared memory.
 //
 // A call needs `least` bytes and runs its faster forms where it gets `bytes`.
 // The difference is asked for only as far as the device has room: at most half of
@@ -113,6 +113,15 @@ int Workspace::reserve(size_t bytes, size_t least) {
     a.cap = cap;
     if (want > least) a.refused = cap < want ? room : 0;
     return WB_OK;
+}
+
+cudaError_t allow_shared(const void *kernel, size_t bytes) {
+    cudaFuncAttributes at;
+    cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+    if (e != cudaSuccess || (size_t)at.maxDynamicSharedSizeBytes >= bytes) return e;
+    const int most = device_info().max_smem_optin - (int)at.sharedSizeBytes;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                bytes > (size_t)imax(most, 0) ? (int)bytes : most);
 }
 
 }  // namespace wb
