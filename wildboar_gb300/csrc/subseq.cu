@@ -295,6 +295,8 @@ subseq_scaled_tiled_kernel(const SubseqJob J, const double *norm, const double *
         const int L = J.group_len[g];
         const int nwin = nt - L + 1;
         const int64_t row = (int64_t)g * J.x.count + si;
+        // (before the windows' divisions, which are most of the work)
+        if (J.redo_rows && !J.redo_rows[row]) continue;
         const double *mt = mean_tab + row * J.win_stride;
         const double *st = std_tab + row * J.win_stride;
         __syncthreads();

@@ -42,9 +42,11 @@ struct SubseqJob {
     const float *shp_f32 = nullptr;      // packed shapelets (z-normalised when scaled)
     const float *shp_absmax = nullptr;   // (m,) max |value| of each shapelet, rounded up
     // after the dot-product filter (subseq_dot.cu): the scan takes only pairs
-    // with kept[pair] <= 0, *redo of them
+    // with kept[pair] <= 0, *redo of them; redo_rows[group * x.count + series]
+    // says whether there are any
     const int *kept = nullptr;
     const unsigned long long *redo = nullptr;
+    const unsigned char *redo_rows = nullptr;
     double *out_dist = nullptr;          // (x.count, m)
     int64_t *out_idx = nullptr;          // (x.count, m)
 };

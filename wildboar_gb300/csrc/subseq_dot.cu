@@ -199,21 +199,22 @@ __device__ __forceinline__ void window_stats(double ex, double ex2, int L, doubl
     sd = tmp > 0 ? sqrt(tmp) : 1.0;
 }
 
-// running sums -> mean and std in place, for the FP64 scan of pending pairs
+// running sums -> mean and std in place, for the FP64 scan of the rows (length
+// group, series) with pairs left
 __global__ void __launch_bounds__(256)
 finish_stats_kernel(const SubseqJob J, double *ex_tab, double *ex2_tab,
-                    const unsigned long long *redo) {
+                    const unsigned long long *redo, const unsigned char *redo_rows) {
     if (*redo == 0) return;
-    const int64_t total = J.x.count * (int64_t)J.n_groups * J.win_stride;
-    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * 256) {
-        const int64_t row = t / J.win_stride;
+    for (int64_t row = blockIdx.x; row < J.x.count * (int64_t)J.n_groups; row += gridDim.x) {
+        if (!redo_rows[row]) continue;
         const int L = J.group_len[row / J.x.count];
-        if (t - row * J.win_stride > J.x.len - L) continue;
-        double mean, sd;
-        window_stats(ex_tab[t], ex2_tab[t], L, mean, sd);
-        ex_tab[t] = mean;
-        ex2_tab[t] = sd;
+        double *ex = ex_tab + row * J.win_stride, *ex2 = ex2_tab + row * J.win_stride;
+        for (int w = threadIdx.x; w <= J.x.len - L; w += 256) {
+            double mean, sd;
+            window_stats(ex[w], ex2[w], L, mean, sd);
+            ex[w] = mean;
+            ex2[w] = sd;
+        }
     }
 }
 
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(kThreads, 5) dot_filter_kernel(const DotArgs A
         // constants of the windows: scaled (2 / std', 2 mean' / std',
         // |t'| / (std' sqrt(L))), euclidean (sum t'^2)
         const int64_t row = ((int64_t)U.group * J.x.count + si) * J.win_stride;
+        bool open = false;  // one of the thread's windows is not bounded
         for (int w = threadIdx.x; w < nwin; w += kThreads) {
             const int p = padded(w);
             if constexpr (SCALED) {
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(kThreads, 5) dot_filter_kernel(const DotArgs A
                     wm[p] = 2.0f * is * mu;
                     wf[p] = sqrtf(1.0f + mu * is * mu * is) * 1.00001f;
                 } else {  // not bounded
+                    open = true;
                     wb[p] = 0.0f;
                     wm[p] = 0.0f;
                     wf[p] = 1e30f;
@@ -341,6 +344,10 @@ __global__ void __launch_bounds__(kThreads, 5) dot_filter_kernel(const DotArgs A
                 wf[p] = (float)(pre[w + L] - pre[w]);
             }
         }
+        // Windows without a bound stay in every pair (a flat stretch of the series,
+        // or values far from 0): with more than kKeep of them the pairs go to the
+        // scan whatever the products are.
+        if (SCALED && __syncthreads_count(open) > kKeep) continue;
         float eabs = 0.0f;  // euclidean: rounding of the prefix sums
         if constexpr (!SCALED) eabs = __double2float_ru(A.prefix[si * (T + 1) + T] * 1e-11);
         const int tiles = (nwin + kTile - 1) / kTile;
@@ -508,12 +515,18 @@ __global__ void __launch_bounds__(128) dot_exact_kernel(const DotArgs A) {
 // smallest sum of each pair, the first window of equal ones; a pair without a
 // finite one goes to the FP64 scan, which takes no window of an infinite sum
 __global__ void __launch_bounds__(256)
-dot_select_kernel(const DotArgs A, int64_t pairs, unsigned long long *redo) {
+dot_select_kernel(const DotArgs A, int64_t pairs, unsigned long long *redo,
+                  unsigned char *redo_rows) {
     const int64_t pair = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (pair >= pairs) return;
     const int count = A.kept[pair];
-    if (count <= 0) {
+    auto leave = [&]() {
+        const int64_t si = pair / A.J.m;
+        redo_rows[(int64_t)A.J.group_of[pair - si * A.J.m] * A.J.x.count + si] = 1;
         atomicAdd(redo, 1ull);
+    };
+    if (count <= 0) {
+        leave();
         return;
     }
     double best = A.sums[pair * kKeep];
@@ -528,7 +541,7 @@ dot_select_kernel(const DotArgs A, int64_t pairs, unsigned long long *redo) {
     }
     if (!(best < WB_DBL_INF)) {
         A.kept[pair] = 0;
-        atomicAdd(redo, 1ull);
+        leave();
         return;
     }
     A.J.out_dist[pair] = sqrt(best);
@@ -582,7 +595,8 @@ size_t subseq_dot_bytes(const SubseqJob &J, bool scaled) {
            (scaled ? 0 : align256(J.x.count * ((int64_t)J.x.len + 1) * 8)) +
            align256(sizeof(GuidedPrep)) + align256(pairs * kKeep * 4) +
            align256(pairs * kKeep * 8) + align256(pairs * 4) +
-           align256(pairs * (kKeep - 1) * 4) + align256(4) + 4096;
+           align256(pairs * (kKeep - 1) * 4) + align256(4) +
+           align256(J.x.count * (int64_t)J.n_groups) + 4096;
 }
 
 int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex, double *ex2,
@@ -611,6 +625,8 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     WB_TAKE(kept, int, ws, pairs);
     WB_TAKE(extra, uint32_t, ws, pairs * (kKeep - 1));
     WB_TAKE(n_extra, unsigned, ws, 1);
+    const size_t rows_bytes = (size_t)J.x.count * J.n_groups;
+    WB_TAKE(redo_rows, unsigned char, ws, rows_bytes);
     WB_CUDA(cudaMemcpyAsync(quads, plan->quads.data(), nq * sizeof(Quad), cudaMemcpyHostToDevice, s));
     WB_CUDA(cudaMemcpyAsync(units, plan->units.data(), nu * sizeof(Unit), cudaMemcpyHostToDevice, s));
     WB_CUDA(cudaMemsetAsync(&prep->lo, 0x7f, sizeof(prep->lo), s));
@@ -618,6 +634,7 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     WB_CUDA(cudaMemsetAsync(&prep->queue, 0, sizeof(prep->queue) + sizeof(prep->pending), s));
     WB_CUDA(cudaMemsetAsync(kept, 0, pairs * sizeof(int), s));
     WB_CUDA(cudaMemsetAsync(n_extra, 0, sizeof(unsigned), s));
+    WB_CUDA(cudaMemsetAsync(redo_rows, 0, rows_bytes, s));
     DotArgs A;
     A.J = J;
     A.norm = norm;
@@ -671,14 +688,17 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
         WB_TRY(run(dot_range_kernel<false>, dot_series_kernel<false>, quad_kernel<false>,
                    dot_filter_kernel<false>, dot_exact_kernel<false>));
     }
-    dot_select_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(A, pairs, &prep->pending);
+    dot_select_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(A, pairs, &prep->pending,
+                                                                      redo_rows);
     WB_LAUNCH_CHECK("dot_select_kernel");
     if (scaled) {
-        finish_stats_kernel<<<dev.sm_count * 8, 256, 0, s>>>(J, ex, ex2, &prep->pending);
+        finish_stats_kernel<<<dev.sm_count * 8, 256, 0, s>>>(J, ex, ex2, &prep->pending,
+                                                             redo_rows);
         WB_LAUNCH_CHECK("finish_stats_kernel");
     }
     J.kept = kept;
     J.redo = &prep->pending;
+    J.redo_rows = redo_rows;
     return WB_OK;
 }
 
