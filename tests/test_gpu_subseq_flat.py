@@ -36,3 +36,22 @@ def test_some_flat_series(longest, stretch, flat):
     od, oi = O.subsequence(S, X, metric="scaled_euclidean")
     np.testing.assert_array_equal(i, oi)
     np.testing.assert_allclose(d, od, rtol=1e-12, atol=0)
+
+
+# every series at a level and of a size of its own: the bounds of one do not
+# suffer from another's
+@pytest.mark.parametrize("levels", [[0, 1e3, -1e6, 1e9], [0, 0, 0, 1e160], [1e-200, 1e200, 0, 1],
+                                    [1e-300, 1e-160, 1e300, 1e308]])
+@pytest.mark.parametrize("size", [1.0, 1e-3, 1e4])
+def test_series_of_different_levels(levels, size):
+    rng = np.random.default_rng(3)
+    X = np.cumsum(rng.standard_normal((5, 300)), axis=1)
+    for i, v in enumerate(levels):
+        X[i] = X[i] * size + v if abs(v) < 1e100 else X[i] * (v / 1e3)
+    S = [np.cumsum(rng.standard_normal(k)) for k in (9, 17, 17, 40, 200)]
+    S.append(X[1, 50:90].copy())
+    with np.errstate(all="ignore"):
+        d, i = pairwise_subsequence_distance(S, X, metric="scaled_euclidean", return_index=True)
+        od, oi = O.subsequence(S, X, metric="scaled_euclidean")
+    np.testing.assert_array_equal(i, oi)
+    np.testing.assert_allclose(d, od, rtol=1e-12, atol=0)

@@ -141,9 +141,9 @@ __device__ __forceinline__ double order_value(long long c) {
 
 // Centre and power-of-two scale that map [lo, hi] into [-1, 1]; false where the
 // values are not finite or too small.
-__device__ __forceinline__ bool centre_scale(const GuidedPrep *prep, double &centre,
-                                             double &scale) {
-    const double lo = order_value(prep->lo), hi = order_value(prep->hi);
+__device__ __forceinline__ bool centre_scale(long long lo_code, long long hi_code,
+                                             double &centre, double &scale) {
+    const double lo = order_value(lo_code), hi = order_value(hi_code);
     const double half = hi * 0.5 - lo * 0.5;
     if (!(isfinite(lo) && isfinite(hi) && isfinite(half))) return false;
     centre = lo * 0.5 + hi * 0.5;
@@ -153,6 +153,10 @@ __device__ __forceinline__ bool centre_scale(const GuidedPrep *prep, double &cen
     if (e < -400) return false;
     scale = scalbn(1.0, -e);
     return true;
+}
+__device__ __forceinline__ bool centre_scale(const GuidedPrep *prep, double &centre,
+                                             double &scale) {
+    return centre_scale(prep->lo, prep->hi, centre, scale);
 }
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {

@@ -7,7 +7,7 @@
 // first window (distance/_metric.pyx:561-682).  The same sums expand to
 //   euclidean   sum t^2 + sum s^2 - 2 sum s t
 //   scaled      sum s^2 + L - (2 / std) (sum s t' - mean' sum s),
-// t' and mean' relative to a common centre (sum ((t - mean) / std)^2 = L for
+// t' and mean' relative to a centre of the series (sum ((t - mean) / std)^2 = L for
 // the window's own mean and std), so all windows of a series against all
 // shapelets of one length are one sliding product: one fused multiply-add per
 // (window, shapelet, value) instead of a subtraction, a multiply-add, an
@@ -69,6 +69,10 @@ struct Unit {  // consecutive quads of one length
     int first, count, group, len;
 };
 
+struct Range {  // order codes of the smallest and largest value
+    long long lo, hi;
+};
+
 struct DotArgs {
     SubseqJob J;
     const double *norm = nullptr;           // scaled: normalised shapelets (else J.shapelets)
@@ -81,7 +85,7 @@ struct DotArgs {
     float2 *sn = nullptr;                   // [4 quad + j]: sum s^2, sum s
     const float *xf = nullptr;              // t' of the series, stride x.len
     const float *xmax2 = nullptr;           // scaled: largest t^2 of the series (scaled units)
-    const GuidedPrep *prep = nullptr;
+    const Range *range = nullptr;           // scaled: per series, euclidean: of everything
     uint32_t *windows = nullptr;            // [pair][kKeep]
     double *sums = nullptr;
     int *kept = nullptr;
@@ -89,10 +93,28 @@ struct DotArgs {
     unsigned *n_extra = nullptr;
 };
 
-// smallest and largest value (shapelets too unless scaled); one warp per row
+// Smallest and largest value, one warp per row: scaled, of every series (the
+// products' rounding counts against a window's deviation, so a series is centred
+// by itself); euclidean, of the series and shapelets together.
 template <bool SCALED>
-__global__ void __launch_bounds__(256) dot_range_kernel(const SubseqJob J, GuidedPrep *prep) {
+__global__ void __launch_bounds__(256) dot_range_kernel(const SubseqJob J, Range *range) {
     double lo = WB_DBL_INF, hi = -WB_DBL_INF;
+    auto reduce = [&](int64_t row) {
+        long long l = order_code(lo), h = order_code(hi);
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long l2 = __shfl_xor_sync(0xffffffffu, l, o);
+            const long long h2 = __shfl_xor_sync(0xffffffffu, h, o);
+            l = l2 < l ? l2 : l;
+            h = h2 > h ? h2 : h;
+        }
+        if ((threadIdx.x & 31) != 0) return;
+        if (SCALED) {
+            range[row] = Range{l, h};
+        } else {
+            atomicMin(&range->lo, l);
+            atomicMax(&range->hi, h);
+        }
+    };
     const int64_t total = J.x.count + (SCALED ? 0 : J.m);
     for (int64_t t = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5; t < total;
          t += ((int64_t)gridDim.x * 256) >> 5) {
@@ -106,31 +128,27 @@ __global__ void __launch_bounds__(256) dot_range_kernel(const SubseqJob J, Guide
             lo = v < lo ? v : lo;
             hi = v > hi ? v : hi;
         }
+        if (SCALED) {
+            reduce(t);
+            lo = WB_DBL_INF;
+            hi = -WB_DBL_INF;
+        }
     }
-    long long l = order_code(lo), h = order_code(hi);
-    for (int o = 16; o > 0; o >>= 1) {
-        const long long l2 = __shfl_xor_sync(0xffffffffu, l, o);
-        const long long h2 = __shfl_xor_sync(0xffffffffu, h, o);
-        l = l2 < l ? l2 : l;
-        h = h2 > h ? h2 : h;
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&prep->lo, l);
-        atomicMax(&prep->hi, h);
-    }
+    if (!SCALED) reduce(0);
 }
 
 // t' as floats; scaled: the largest t^2, euclidean: FP64 prefix sums of t'^2
 // (by chunks of 32 with a warp scan).  One warp per series.
 template <bool SCALED>
 __global__ void __launch_bounds__(256)
-dot_series_kernel(const SubseqJob J, const GuidedPrep *prep, float *xf, float *xmax2,
+dot_series_kernel(const SubseqJob J, const Range *range, float *xf, float *xmax2,
                   double *prefix) {
     const int lane = threadIdx.x & 31;
-    double centre = 0.0, scale = 1.0;
-    centre_scale(prep, centre, scale);
     for (int64_t s = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5; s < J.x.count;
          s += ((int64_t)gridDim.x * 256) >> 5) {
+        const Range R = range[SCALED ? s : 0];
+        double centre = 0.0, scale = 1.0;
+        centre_scale(R.lo, R.hi, centre, scale);
         const double *src = J.x.base + s * J.x.stride;
         float mx = 0.0f;
         double run = 0.0;
@@ -225,7 +243,7 @@ __global__ void __launch_bounds__(64) quad_kernel(const DotArgs A, int64_t n_qua
     const SubseqJob &J = A.J;
     const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
     double centre = 0.0, scale = 1.0;
-    centre_scale(A.prep, centre, scale);
+    if (!SCALED) centre_scale(A.range->lo, A.range->hi, centre, scale);
     for (int64_t qd = blockIdx.x; qd < n_quads; qd += gridDim.x) {
         const Quad Q = A.quads[qd];
         const int len = (Q.len + 7) & ~7;
@@ -304,12 +322,13 @@ __global__ void __launch_bounds__(kThreads, 5) dot_filter_kernel(const DotArgs A
     const SubseqJob &J = A.J;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int T = J.x.len;
-    double centre = 0.0, scale = 1.0;
-    if (!centre_scale(A.prep, centre, scale)) return;  // every pair goes to the FP64 scan
     const int cols = padded(staged(T)) + 1;  // of the padded arrays
     float *ts = sm, *wb = sm + cols, *wm = sm + 2 * cols, *wf = sm + 3 * cols;
     for (int64_t b = blockIdx.x; b < J.x.count * (int64_t)A.n_units; b += gridDim.x) {
         const int64_t si = b / A.n_units;
+        const Range R = A.range[SCALED ? si : 0];
+        double centre = 0.0, scale = 1.0;
+        if (!centre_scale(R.lo, R.hi, centre, scale)) continue;  // left to the FP64 scan
         const Unit U = A.units[b - si * A.n_units];
         const int L = U.len, nwin = T - L + 1;
         const int Lp = (L + 7) & ~7;
@@ -328,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 5) dot_filter_kernel(const DotArgs A
                 const double var = (A.ex2[row + w] * inv - mean * mean) * (scale * scale);
                 const float vf = (float)var;
                 const float mu = (float)((mean - centre) * scale);
-                if (vf >= __fmul_rn(1.1e-5f, A.xmax2[si])) {
+                if (vf > __fmul_rn(1.1e-5f, A.xmax2[si]) && vf <= FLT_MAX) {
                     const float is = 1.0f / sqrtf(vf);
                     wb[p] = 2.0f * is;
                     wm[p] = 2.0f * is * mu;
@@ -593,7 +612,8 @@ size_t subseq_dot_bytes(const SubseqJob &J, bool scaled) {
            align256((J.total_values + 8 * J.m) * 16) + align256(J.m * 4 * sizeof(float2)) +
            align256(J.x.count * (int64_t)J.x.len * 4) + align256(J.x.count * 4) +
            (scaled ? 0 : align256(J.x.count * ((int64_t)J.x.len + 1) * 8)) +
-           align256(sizeof(GuidedPrep)) + align256(pairs * kKeep * 4) +
+           align256(sizeof(GuidedPrep)) + align256((scaled ? J.x.count : 1) * sizeof(Range)) +
+           align256(pairs * kKeep * 4) +
            align256(pairs * kKeep * 8) + align256(pairs * 4) +
            align256(pairs * (kKeep - 1) * 4) + align256(4) +
            align256(J.x.count * (int64_t)J.n_groups) + 4096;
@@ -609,6 +629,7 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     keep.plan = plan;  // the uploads read it until the stream is synchronised
     const int64_t nq = (int64_t)plan->quads.size(), nu = (int64_t)plan->units.size();
     WB_TAKE(prep, GuidedPrep, ws, 1);
+    WB_TAKE(range, Range, ws, scaled ? J.x.count : 1);
     WB_TAKE(quads, Quad, ws, nq);
     WB_TAKE(units, Unit, ws, nu);
     WB_TAKE(s4, float4, ws, plan->s4);
@@ -629,8 +650,10 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     WB_TAKE(redo_rows, unsigned char, ws, rows_bytes);
     WB_CUDA(cudaMemcpyAsync(quads, plan->quads.data(), nq * sizeof(Quad), cudaMemcpyHostToDevice, s));
     WB_CUDA(cudaMemcpyAsync(units, plan->units.data(), nu * sizeof(Unit), cudaMemcpyHostToDevice, s));
-    WB_CUDA(cudaMemsetAsync(&prep->lo, 0x7f, sizeof(prep->lo), s));
-    WB_CUDA(cudaMemsetAsync(&prep->hi, 0x80, sizeof(prep->hi), s));
+    if (!scaled) {  // lo = a very large code, hi = a very small one
+        WB_CUDA(cudaMemsetAsync(&range->lo, 0x7f, sizeof(range->lo), s));
+        WB_CUDA(cudaMemsetAsync(&range->hi, 0x80, sizeof(range->hi), s));
+    }
     WB_CUDA(cudaMemsetAsync(&prep->queue, 0, sizeof(prep->queue) + sizeof(prep->pending), s));
     WB_CUDA(cudaMemsetAsync(kept, 0, pairs * sizeof(int), s));
     WB_CUDA(cudaMemsetAsync(n_extra, 0, sizeof(unsigned), s));
@@ -648,7 +671,7 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     A.sn = sn;
     A.xf = xf;
     A.xmax2 = xmax2;
-    A.prep = prep;
+    A.range = range;
     A.windows = windows;
     A.sums = sums;
     A.kept = kept;
@@ -659,10 +682,10 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     const int rows_grid = (int)std::min(cap, (J.x.count + J.m + 7) / 8);
     const int quad_grid = (int)std::min<int64_t>(nq, 65535);
     const size_t smem = dot_smem(J.x.len);
-    auto run = [&](auto range, auto series, auto quad, auto filter, auto exact) -> int {
-        range<<<rows_grid, 256, 0, s>>>(J, prep);
+    auto run = [&](auto range_of, auto series, auto quad, auto filter, auto exact) -> int {
+        range_of<<<rows_grid, 256, 0, s>>>(J, range);
         WB_LAUNCH_CHECK("dot_range_kernel");
-        series<<<rows_grid, 256, 0, s>>>(J, prep, xf, xmax2, prefix);
+        series<<<rows_grid, 256, 0, s>>>(J, range, xf, xmax2, prefix);
         WB_LAUNCH_CHECK("dot_series_kernel");
         quad<<<quad_grid, 64, 0, s>>>(A, nq);
         WB_LAUNCH_CHECK("quad_kernel");
