@@ -79,6 +79,8 @@ namespace {
 constexpr int kThreads = 128;
 constexpr unsigned kCap = 1u << 30;  // saturated value, and out of band
 constexpr int kFixOne = (1 << 29) - 1;  // 1.0 in fixed point
+constexpr int64_t kTailPairs = 2048;  // pairs left that guided_tail_kernel takes (more fill
+                                      // the second pass's warps)
 
 // Smallest and largest value of both series sets.  (The second is passed over
 // only as the very same set: device arrays are used in place, so a set may
@@ -777,10 +779,30 @@ __device__ __forceinline__ unsigned bottom_bits(uint64_t word) {
     return bits;
 }
 
+// Whether the pairs to come go to the full recurrence at once and the costly tiles
+// under way stop: three quarters of `need` or more pairs were left, shared a tile
+// with one left (a warp of the second pass takes as long for one pair as for 32), or
+// had a fourth of a wide band's blocks collected -- values that tie everywhere.
+// `need` is half of the resident pairs, so that a few columns of such series among
+// others decide nothing, and no job that the tail kernel takes.  dtw, length 512
+// (full recurrence / a rule at the start of a tile, by full tiles taken / this one):
+// 0 / 1 values, r = 0.1, 1000 x 800 pairs 237 / 244 / 242 ms, 33 x 3000 55 / 64 / 59;
+// r = 1, 500 x 400, runs of 8 equal values 319 / 358 / 341, one spike each 319 / 347 /
+// 333; 900 against themselves, one spike each, r = 0.1 128 / 141 / 135; four constant
+// series before 796 walks, 1000 walks, r = 0.1 237 / 220 / 42.
+__device__ __forceinline__ bool ties_everywhere(const GuidedArgs &A) {
+    const unsigned long long seen =
+        *reinterpret_cast<const volatile unsigned long long *>(&A.prep->seen);
+    const unsigned long long heavy =
+        *reinterpret_cast<const volatile unsigned long long *>(&A.prep->heavy);
+    return seen >= A.need && 4 * heavy >= 3 * seen;
+}
+
+// `watch`: a lane ends without a value, count = -1, once ties_everywhere.
 template <int KIND, int S>
 __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__restrict__ X,
-                                           const double *__restrict__ Y, int count, int row0,
-                                           int64_t gt, Stage<S> &St) {
+                                           const double *__restrict__ Y, int &count, int row0,
+                                           int64_t gt, Stage<S> &St, bool watch) {
     constexpr int W64 = S * S / 64;
     constexpr int C = 64 / S;
     constexpr unsigned SM = (1u << S) - 1u;
@@ -816,6 +838,10 @@ __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__
     // the next word, loaded while the current one is worked on
     uint4 next = left > 0 ? list[left - 1] : make_uint4(0u, 0u, 0u, 0u);
     while (__any_sync(0xffffffffu, todo != 0 || left > 0)) {
+        if (watch && todo == 0 && (left & 15) == 15 && ties_everywhere(A)) {
+            left = 0;
+            count = -1;
+        }
         if (todo == 0 && left > 0) {
             left--;
             const uint4 E = next;
@@ -935,20 +961,10 @@ guided_pairs_kernel(const GuidedArgs A) {
     const float K = (float)(B.n + B.m);
 
     for (;;) {
-        unsigned long long t64 = 0, left = 0;
-        if (lane == 0) {
-            t64 = atomicAdd(&A.prep->queue, 1ull);
-            left = *reinterpret_cast<volatile unsigned long long *>(&A.prep->heavy);
-        }
+        unsigned long long t64 = 0;
+        if (lane == 0) t64 = atomicAdd(&A.prep->queue, 1ull);
         const int64_t t = (int64_t)__shfl_sync(FULL, t64, 0);
         if (t >= ntiles) break;
-        // Where three quarters of the pairs of the first tiles were left to the full
-        // recurrence or had a fourth of a wide band's blocks collected (values that
-        // tie everywhere), the rest goes there at once: 1000 x 800 pairs of 512, one
-        // spike each, r = 0.1 242 ms (full recurrence 237), r = 1, 500 x 400 412, was 536
-        // (320); 0 / 1 values, r = 0.1 251, was 319 (237).
-        const int64_t done = t - (int64_t)gridDim.x * (kThreads / 32);
-        const bool give_up = done >= 128 && (int64_t)__shfl_sync(FULL, left, 0) >= 24 * done;
         int64_t cs = t / chunks;
         int64_t rs = (t - cs * chunks) * 32 + lane;
         if (J.mode == PM_PAIRED) {
@@ -972,11 +988,12 @@ guided_pairs_kernel(const GuidedArgs A) {
                 if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = res;
             }
         };
-        if (give_up) {
+        if (__any_sync(FULL, lane == 0 && ties_everywhere(A))) {
             if (active) {
                 store(__longlong_as_double(kGuidedPending));
                 atomicAdd(&A.prep->pending, 1ull);
                 atomicAdd(&A.prep->heavy, 1ull);
+                atomicAdd(&A.prep->seen, 1ull);
             }
             continue;
         }
@@ -1033,12 +1050,19 @@ guided_pairs_kernel(const GuidedArgs A) {
 
         const unsigned heavy = __ballot_sync(
             FULL, active && (count <= 0 || (A.blocks >= 12 && 4 * count > B.ns * A.blocks)));
-        if (lane == 0 && heavy) atomicAdd(&A.prep->heavy, (unsigned long long)__popc(heavy));
+        const int pairs = __popc(__ballot_sync(FULL, active));
+        const int costly = __any_sync(FULL, active && count <= 0) ? pairs : __popc(heavy);
+        if (lane == 0) {
+            if (costly) atomicAdd(&A.prep->heavy, (unsigned long long)costly);
+            atomicAdd(&A.prep->seen, (unsigned long long)pairs);
+        }
+        const bool watch = 4 * costly >= 3 * pairs;
 
         double value = 0.0;
+        if (watch && ties_everywhere(A)) count = -1;
         if (__any_sync(FULL, count > 0))
             value = evaluate<KIND, S>(A, A.xd + rs * A.xs + 3, A.yd + cs * A.ys, count, row0, gt,
-                                      stage);
+                                      stage, watch);
         if (active) {
             store(count > 0 ? sqrt(value) : __longlong_as_double(kGuidedPending));
             if (count <= 0) atomicAdd(&A.prep->pending, 1ull);
@@ -1054,7 +1078,6 @@ guided_pairs_kernel(const GuidedArgs A) {
 // pair, as the second pass has them, takes 330 cycles for every cell: a single
 // pair of 400 x 361, r = 1, kept the call waiting for 13 ms, here 1.
 constexpr int kTailRows = 8;
-constexpr int64_t kTailPairs = 2048;  // more of them fill the second pass's warps
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) guided_tail_kernel(const GuidedArgs A) {
@@ -1349,6 +1372,7 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     GuidedArgs &A = C.args;
     A.J = J;
     A.nth = nth;
+    A.need = (unsigned)std::max<int64_t>(kTailPairs, nth / 2);
     A.groups = p.groups;
     A.blocks = p.blocks;
     A.list_cap = p.list_cap;
@@ -1412,7 +1436,7 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
 
 int guided_run(const GuidedContext &C, cudaStream_t s) {
     GuidedPrep *prep = C.args.prep;
-    WB_CUDA(cudaMemsetAsync(&prep->queue, 0, 3 * sizeof(unsigned long long), s));
+    WB_CUDA(cudaMemsetAsync(&prep->queue, 0, 4 * sizeof(unsigned long long), s));
     switch (C.args.J.kind) {
         case K_DTW: return run_kernel<K_DTW>(C, s);
         case K_WDTW: return run_kernel<K_WDTW>(C, s);

@@ -23,7 +23,8 @@ struct GuidedPrep {
     long long lo, hi;            // order codes of the smallest / largest input
     unsigned long long queue;    // next tile of 32 pairs
     unsigned long long pending;  // pairs left to the full recurrence
-    unsigned long long heavy;    // they and those with a fourth of their blocks collected
+    unsigned long long seen;     // pairs whose blocks were collected, and of them those
+    unsigned long long heavy;    // with a fourth of the blocks or in a tile with one left
 };
 
 // Extremes of a series: fixed point, and the largest float magnitude.
@@ -49,6 +50,7 @@ struct GuidedArgs {
     const uint32_t *items = nullptr;
     const unsigned *n_items = nullptr;
     int64_t n_all = 0, col0 = 0;
+    unsigned need = 0;  // pairs seen before the kernel gives up
     // per resident thread, interleaved [...][thread]
     int64_t nth = 0;
     uint4 *ckrow = nullptr;   // [strip + 1][group of 4 columns] bottom rows
