@@ -72,6 +72,12 @@ struct ElasticJob {
     const unsigned long long *pending = nullptr;
 };
 
+// Tiles of 32 pairs go round the warps; in a second pass each round starts some
+// warps further on, since the pairs left often lie in a few rows, whose tiles are
+// as far apart as the rows' chunks are many (with 1 of 8 rows left: all of them on
+// 1 of 8 warps).
+constexpr int kPassShift = 37;
+
 // Ring length (in elements) needed for a band recurrence of an (n x m)
 // problem with half-width r: the live window spans columns js-1 .. je.
 inline int ring_len(int n, int m, int r) {

@@ -105,7 +105,13 @@ elastic_pairs_kernel(const ElasticJob J, double *gring, int P) {
         }
         const int64_t chunks = (J.rows.count + 31) >> 5;
         const int64_t ntiles = chunks * J.cols.count;
-        for (int64_t t = warp; t < ntiles; t += nwarps) {
+        const int64_t shift = PASS2 && J.pending ? kPassShift % nwarps : 0;
+        int64_t at = warp;
+        for (int64_t base = 0; base < ntiles; base += nwarps) {
+            const int64_t t = base + at;
+            at += shift;
+            if (at >= nwarps) at -= nwarps;
+            if (t >= ntiles) continue;
             const int64_t cs = t / chunks;
             const int64_t rs = (t - cs * chunks) * 32 + lane;
             if (J.mode == PM_UPPER) {
