@@ -732,7 +732,7 @@ extern "C" int wb_argmin_distance(const wb_series *x, const wb_series *y, int64_
                     C.cur_dist = A.state_dist;
                     C.lower_bound = lb;
                     ElasticJob Jp = Jb;
-                    WB_TRY(guided.launch_chunk((int)c, C, s, &Jp.pending));
+                    WB_TRY(guided.launch_chunk((int)c, C, s, Jp));
                     WB_TRY(launch_argmin_ea(Jp, metric, xl, yl, C.j0, C.nc, y->n, A.state_dist,
                                             lb, counters + c, ea_ring, s));
                     A.j0 = at[c];

@@ -46,7 +46,7 @@ constexpr int kEaThreads = 128;
 template <int KIND>
 __global__ void __launch_bounds__(kEaThreads)
 argmin_ea_kernel(const ElasticJob J, const EaChunk C, int P) {
-    if (J.pending && *J.pending == 0) return;
+    if (J.pending && *J.pending <= (unsigned long long)J.tail_cap) return;
     const RingS ring{(int)threadIdx.x, kEaThreads};
     const int n = J.rows.len, m = J.cols.len, r = J.band;
     const int mx = imax(0, m - n) + r;
@@ -145,7 +145,7 @@ argmin_ea_kernel(const ElasticJob J, const EaChunk C, int P) {
 template <int KIND, int S>
 __global__ void __launch_bounds__(kEaThreads)
 argmin_ea_strip_kernel(const ElasticJob J, const EaChunk C, double *ring_base, int64_t ring_ld) {
-    if (J.pending && *J.pending == 0) return;
+    if (J.pending && *J.pending <= (unsigned long long)J.tail_cap) return;
     const int64_t gtid = (int64_t)blockIdx.x * kEaThreads + threadIdx.x;
     double *ring = ring_base + gtid * ring_ld;
     const int n = J.rows.len, m = J.cols.len, r = J.band;

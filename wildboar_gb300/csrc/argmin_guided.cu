@@ -498,10 +498,10 @@ int GuidedArgmin::prepare(const ElasticJob &J, Workspace &ws, size_t leave, bool
 }
 
 // Distances of the candidates of chunk number `index`: exact where the
-// reference could push the candidate, else +inf; *pending counts the pairs left
-// to the full recurrence (their output is kGuidedPending).
+// reference could push the candidate, else +inf; the pairs left to the full
+// recurrence hold kGuidedPending.
 int GuidedArgmin::launch_chunk(int index, const EaChunk &C, cudaStream_t s,
-                               const unsigned long long **pending) {
+                               ElasticJob &second) {
     if (index >= kMaxChunks) return fail(WB_EINVAL, "too many candidate chunks");
     GuidedContext ctx = impl_->ctx;
     const ElasticJob &J = ctx.args.J;
@@ -536,7 +536,8 @@ int GuidedArgmin::launch_chunk(int index, const EaChunk &C, cudaStream_t s,
         ctx.args.n_items = n2;
     }
     WB_TRY(guided_run(ctx, s));
-    *pending = &ctx.args.prep->pending;
+    second.pending = &ctx.args.prep->pending;
+    second.tail_cap = ctx.args.tail_cap;
     return WB_OK;
 }
 

@@ -68,8 +68,12 @@ struct ElasticJob {
     double *key = nullptr;              // early-abandon keys (argmin), or null
     int all_zero = 0;                   // ddtw on series shorter than 3
     // second pass of a guided evaluation (guided.cu): only the pairs whose
-    // output is kGuidedPending, *pending of them
+    // output was kGuidedPending, *pending of them: none where these are at most
+    // tail_cap (guided_tail_kernel took them); where they are at most left_cap, `left`
+    // lists them (row + rows.count column, paired: the row)
     const unsigned long long *pending = nullptr;
+    const unsigned long long *left = nullptr;
+    int64_t left_cap = 0, tail_cap = 0;
 };
 
 // Tiles of 32 pairs go round the warps; in a second pass each round starts some

@@ -91,9 +91,21 @@ elastic_pairs_kernel(const ElasticJob J, double *gring, int P) {
     const int64_t gtid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t gthreads = (int64_t)gridDim.x * kThreads;
     constexpr bool PASS2 = guided_kind(KIND);
-    if (PASS2 && J.pending && *J.pending == 0) return;
+    if (PASS2 && J.pending && *J.pending <= (unsigned long long)J.tail_cap) return;
 
     auto body = [&](auto ring) {
+        if (PASS2 && J.pending && *J.pending <= (unsigned long long)J.left_cap) {
+            const int64_t left = (int64_t)*J.pending;
+            for (int64_t q = spread_lane(); q < left; q += gthreads) {
+                int64_t rs, cs;
+                double *out = left_pair(J, q, rs, cs);
+                if (!is_pending(*out)) continue;
+                double key = 0.0;
+                *out = finish(J, run_pair<KIND>(J, ring, P, rs, cs, key));
+                if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = *out;
+            }
+            return;
+        }
         if (J.mode == PM_PAIRED) {
             for (int64_t s = gtid; s < J.rows.count; s += gthreads) {
                 if (PASS2 && J.pending && !is_pending(J.out[s])) continue;
@@ -327,9 +339,12 @@ int launch_elastic(const ElasticJob &job, Workspace &ws, bool guided) {
         // that it leaves
         unsigned long long *pending = nullptr;
         const size_t full = elastic_workspace_bytes(J);
-        if (bit_edit_supported(J)) WB_TRY(launch_bit_edit(J, ws, full, &pending));
-        else WB_TRY(launch_guided(J, ws, full, &pending));
-        J.pending = pending;
+        if (bit_edit_supported(J)) {
+            WB_TRY(launch_bit_edit(J, ws, full, &pending));
+            J.pending = pending;
+        } else {
+            WB_TRY(launch_guided(J, ws, full));
+        }
     }
     if (use_strip_f64(J)) return launch_strip(J, ws, false);
     ElasticPlan pl = plan_elastic(J);

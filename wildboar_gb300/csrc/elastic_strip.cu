@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kStripThreads)
     typename A::R *ring = ring_base + gtid;
     const int n = J.rows.len, m = J.cols.len;
     constexpr bool PASS2 = guided_kind(KIND);
-    if (PASS2 && J.pending && *J.pending == 0) return;
+    if (PASS2 && J.pending && *J.pending <= (unsigned long long)J.tail_cap) return;
 
     auto run = [&](int64_t rs, int64_t cs) -> double {
         if (J.all_zero) return 0.0;
@@ -565,6 +565,17 @@ __global__ void __launch_bounds__(kStripThreads)
         return finish_value(J, A::value(v));
     };
 
+    if (PASS2 && J.pending && *J.pending <= (unsigned long long)J.left_cap) {
+        const int64_t left = (int64_t)*J.pending;
+        for (int64_t q = spread_lane(); q < left; q += nth) {
+            int64_t rs, cs;
+            double *out = left_pair(J, q, rs, cs);
+            if (!is_pending(*out)) continue;
+            *out = run(rs, cs);
+            if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = *out;
+        }
+        return;
+    }
     if (J.mode == PM_PAIRED) {
         for (int64_t s = gtid; s < J.rows.count; s += nth)
             if (!PASS2 || !J.pending || is_pending(J.out[s])) J.out[s] = run(s, s);

@@ -79,8 +79,6 @@ namespace {
 constexpr int kThreads = 128;
 constexpr unsigned kCap = 1u << 30;  // saturated value, and out of band
 constexpr int kFixOne = (1 << 29) - 1;  // 1.0 in fixed point
-constexpr int64_t kTailPairs = 2048;  // pairs left that guided_tail_kernel takes (more fill
-                                      // the second pass's warps)
 
 // Smallest and largest value of both series sets.  (The second is passed over
 // only as the very same set: device arrays are used in place, so a set may
@@ -779,17 +777,11 @@ __device__ __forceinline__ unsigned bottom_bits(uint64_t word) {
     return bits;
 }
 
-// Whether the pairs to come go to the full recurrence at once and the costly tiles
-// under way stop: three quarters of `need` or more pairs were left, shared a tile
-// with one left (a warp of the second pass takes as long for one pair as for 32), or
-// had a fourth of a wide band's blocks collected -- values that tie everywhere.
-// `need` is half of the resident pairs, so that a few columns of such series among
-// others decide nothing, and no job that the tail kernel takes.  dtw, length 512
-// (full recurrence / a rule at the start of a tile, by full tiles taken / this one):
-// 0 / 1 values, r = 0.1, 1000 x 800 pairs 237 / 244 / 242 ms, 33 x 3000 55 / 64 / 59;
-// r = 1, 500 x 400, runs of 8 equal values 319 / 358 / 341, one spike each 319 / 347 /
-// 333; 900 against themselves, one spike each, r = 0.1 128 / 141 / 135; four constant
-// series before 796 walks, 1000 walks, r = 0.1 237 / 220 / 42.
+// Whether the pairs to come go to the full recurrence at once: three quarters of
+// `need` or more pairs were left or had a fourth of a wide band's blocks collected
+// (values that tie everywhere).  `need` is half of the resident pairs, so that a few
+// columns of such series among others decide nothing, and no job that the tail kernel
+// takes.
 __device__ __forceinline__ bool ties_everywhere(const GuidedArgs &A) {
     const unsigned long long seen =
         *reinterpret_cast<const volatile unsigned long long *>(&A.prep->seen);
@@ -798,11 +790,18 @@ __device__ __forceinline__ bool ties_everywhere(const GuidedArgs &A) {
     return seen >= A.need && 4 * heavy >= 3 * seen;
 }
 
-// `watch`: a lane ends without a value, count = -1, once ties_everywhere.
+// Whether the second pass comes anyway: pairs with more than a fourth of their blocks
+// then go with it, also from under way.
+__device__ __forceinline__ bool second_pass_comes(const GuidedArgs &A) {
+    return *reinterpret_cast<const volatile unsigned long long *>(&A.prep->heavy) >
+           (unsigned long long)A.tail_cap;
+}
+
+// `large`: the lane ends without a value, count = -1, once second_pass_comes.
 template <int KIND, int S>
 __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__restrict__ X,
                                            const double *__restrict__ Y, int &count, int row0,
-                                           int64_t gt, Stage<S> &St, bool watch) {
+                                           int64_t gt, Stage<S> &St, bool large) {
     constexpr int W64 = S * S / 64;
     constexpr int C = 64 / S;
     constexpr unsigned SM = (1u << S) - 1u;
@@ -838,7 +837,7 @@ __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__
     // the next word, loaded while the current one is worked on
     uint4 next = left > 0 ? list[left - 1] : make_uint4(0u, 0u, 0u, 0u);
     while (__any_sync(0xffffffffu, todo != 0 || left > 0)) {
-        if (watch && todo == 0 && (left & 15) == 15 && ties_everywhere(A)) {
+        if (large && todo == 0 && (left & 15) == 15 && second_pass_comes(A)) {
             left = 0;
             count = -1;
         }
@@ -988,12 +987,23 @@ guided_pairs_kernel(const GuidedArgs A) {
                 if (J.mode == PM_UPPER) J.out[cs * J.out_ld + rs] = res;
             }
         };
+        // the tile's pairs `who` to the second pass
+        auto leave = [&](bool who) {
+            const unsigned mask = __ballot_sync(FULL, who);
+            if (mask == 0) return;
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(&A.prep->pending, (unsigned long long)__popc(mask));
+            at = __shfl_sync(FULL, at, 0) + __popc(mask & ((1u << lane) - 1u));
+            if (!who) return;
+            store(__longlong_as_double(kGuidedPending));
+            if ((int64_t)at < A.left_cap)
+                A.left[at] = J.mode == PM_PAIRED ? rs : rs + J.rows.count * cs;
+        };
         if (__any_sync(FULL, lane == 0 && ties_everywhere(A))) {
-            if (active) {
-                store(__longlong_as_double(kGuidedPending));
-                atomicAdd(&A.prep->pending, 1ull);
-                atomicAdd(&A.prep->heavy, 1ull);
-                atomicAdd(&A.prep->seen, 1ull);
+            leave(active);
+            if (lane == 0) {
+                atomicAdd(&A.prep->heavy, 32ull);
+                atomicAdd(&A.prep->seen, 32ull);
             }
             continue;
         }
@@ -1048,25 +1058,22 @@ guided_pairs_kernel(const GuidedArgs A) {
         if (KIND != K_WDTW && fix) count = collect<KIND, S, KIND != K_WDTW>(A, B, D, e, live, gt, row0);
         else count = collect<KIND, S, false>(A, B, D, e, live, gt, row0);
 
-        const unsigned heavy = __ballot_sync(
-            FULL, active && (count <= 0 || (A.blocks >= 12 && 4 * count > B.ns * A.blocks)));
+        const bool large = 4 * count > B.ns * A.blocks;
+        const unsigned heavy =
+            __ballot_sync(FULL, active && (count <= 0 || (A.blocks >= 12 && large)));
         const int pairs = __popc(__ballot_sync(FULL, active));
-        const int costly = __any_sync(FULL, active && count <= 0) ? pairs : __popc(heavy);
         if (lane == 0) {
-            if (costly) atomicAdd(&A.prep->heavy, (unsigned long long)costly);
+            if (heavy) atomicAdd(&A.prep->heavy, (unsigned long long)__popc(heavy));
             atomicAdd(&A.prep->seen, (unsigned long long)pairs);
         }
-        const bool watch = 4 * costly >= 3 * pairs;
 
         double value = 0.0;
-        if (watch && ties_everywhere(A)) count = -1;
+        if (large && second_pass_comes(A)) count = -1;
         if (__any_sync(FULL, count > 0))
             value = evaluate<KIND, S>(A, A.xd + rs * A.xs + 3, A.yd + cs * A.ys, count, row0, gt,
-                                      stage, watch);
-        if (active) {
-            store(count > 0 ? sqrt(value) : __longlong_as_double(kGuidedPending));
-            if (count <= 0) atomicAdd(&A.prep->pending, 1ull);
-        }
+                                      stage, large);
+        if (active && count > 0) store(sqrt(value));
+        leave(active && count <= 0);
     }
 }
 
@@ -1085,7 +1092,7 @@ __global__ void __launch_bounds__(kThreads) guided_tail_kernel(const GuidedArgs 
     const unsigned FULL = 0xffffffffu;
     const ElasticJob &J = A.J;
     const unsigned long long left = A.prep->pending;
-    if (left == 0 || left > (unsigned long long)kTailPairs) return;
+    if (left == 0 || left > (unsigned long long)A.tail_cap) return;
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
     const int64_t warps = ((int64_t)gridDim.x * kThreads) >> 5;
@@ -1098,105 +1105,97 @@ __global__ void __launch_bounds__(kThreads) guided_tail_kernel(const GuidedArgs 
     // row is written a step before lane 0 reads it
     const int delta = imax(G + 2, imin(m, S + B.mx + B.mn + B.r - 2 - G * S));
     const int steps = (strips - 1) / G * delta + ((strips - 1) & (G - 1)) + m;
-    const int64_t total = J.mode == PM_PAIRED ? J.rows.count : J.rows.count * J.cols.count;
-    for (int64_t base = warp * 32; base < total; base += warps * 32) {
-        const int64_t p = base + lane;
-        int64_t rs = p, cs = p;
+    for (int64_t q = warp; q < (int64_t)left; q += warps) {
+        int64_t r1 = (int64_t)A.left[q], c1 = r1;
         if (J.mode != PM_PAIRED) {
-            rs = p / J.cols.count;
-            cs = p - rs * J.cols.count;
+            c1 = r1 / J.rows.count;
+            r1 -= c1 * J.rows.count;
         }
-        bool mine = p < total && !(J.mode == PM_UPPER && rs >= cs);
-        if (mine) mine = is_pending(J.mode == PM_PAIRED ? J.out[rs] : J.out[rs * J.out_ld + cs]);
-        for (unsigned todo = __ballot_sync(FULL, mine); todo; todo &= todo - 1) {
-            const int src = __ffs(todo) - 1;
-            const int64_t r1 = __shfl_sync(FULL, rs, src), c1 = __shfl_sync(FULL, cs, src);
-            const double *X = J.rows.base + r1 * J.rows.stride;
-            const double *Y = J.cols.base + c1 * J.cols.stride;
-            double P[S], x[S], result = 0.0, acc = 0.0, bot = INF, bdiag = INF, before = INF;
+        const double *X = J.rows.base + r1 * J.rows.stride;
+        const double *Y = J.cols.base + c1 * J.cols.stride;
+        double P[S], x[S], result = 0.0, acc = 0.0, bot = INF, bdiag = INF, before = INF;
 #pragma unroll
-            for (int k = 0; k < S; k++) P[k] = INF, x[k] = 0.0;
-            const double x0 = X[0];
-            int s = lane, c = -lane;
-            for (int t = 0; t < steps; t++) {
-                const double above = __shfl_up_sync(FULL, bot, 1);
-                const bool any = s < strips;
-                const int i0 = 1 + s * S;
-                const int first = any ? B.cs(s, S) : m, end = any ? B.ce(s, S) : m;
-                const int pfirst = any ? B.cs(s - 1, S) : 0, pend = any ? B.ce(s - 1, S) : 0;
-                double up = above;
-                if (lane == 0 && any) {
-                    up = INF;
-                    if (s > 0) {
-                        if (c >= pfirst && c < pend) up = row[c];
-                    } else if (c < lim) {
-                        const double v = x0 - __ldg(Y + c);
-                        double cst = v * v;
-                        if (KIND == K_WDTW) cst = cst * __ldg(J.weights + imax(c - 1, 0));
-                        acc = c == 0 ? cst : acc + cst;
-                        up = acc;
-                    }
+        for (int k = 0; k < S; k++) P[k] = INF, x[k] = 0.0;
+        const double x0 = X[0];
+        int s = lane, c = -lane;
+        for (int t = 0; t < steps; t++) {
+            const double above = __shfl_up_sync(FULL, bot, 1);
+            const bool any = s < strips;
+            const int i0 = 1 + s * S;
+            const int first = any ? B.cs(s, S) : m, end = any ? B.ce(s, S) : m;
+            const int pfirst = any ? B.cs(s - 1, S) : 0, pend = any ? B.ce(s - 1, S) : 0;
+            double up = above;
+            if (lane == 0 && any) {
+                up = INF;
+                if (s > 0) {
+                    if (c >= pfirst && c < pend) up = row[c];
+                } else if (c < lim) {
+                    const double v = x0 - __ldg(Y + c);
+                    double cst = v * v;
+                    if (KIND == K_WDTW) cst = cst * __ldg(J.weights + imax(c - 1, 0));
+                    acc = c == 0 ? cst : acc + cst;
+                    up = acc;
                 }
-                const double raw = up;
-                if (any && c >= first) {
-                    if (c == first) {
-                        bdiag = INF;
-                        if (c > pfirst && c <= pend) {
-                            bdiag = before;
-                            if (lane == 0 && s > 0) bdiag = row[c - 1];
-                        }
-#pragma unroll
-                        for (int k = 0; k < S; k++) {
-                            P[k] = INF;
-                            x[k] = X[imin(i0 + k, n - 1)];
-                        }
+            }
+            const double raw = up;
+            if (any && c >= first) {
+                if (c == first) {
+                    bdiag = INF;
+                    if (c > pfirst && c <= pend) {
+                        bdiag = before;
+                        if (lane == 0 && s > 0) bdiag = row[c - 1];
                     }
-                    if (c >= pend) up = INF;
-                    const double y = __ldg(Y + c), above_cell = up;
-                    double dg = bdiag;
 #pragma unroll
                     for (int k = 0; k < S; k++) {
-                        const int d = c - (i0 + k);
-                        const double lf = P[k], v = x[k] - y;
-                        double cst = v * v;
-                        if (KIND == K_WDTW)
-                            cst = cst * __ldg(J.weights + abs(c - imin(i0 + k, n - 1)));
-                        double mv = nn_min(up, lf);
-                        if (KIND == K_ADTW) mv = mv + J.p;
-                        double nv = nn_min(mv, dg) + cst;
-                        if (d < B.lo || d > B.mx - 1) nv = INF;
-                        dg = lf;
-                        up = nv;
-                        P[k] = nv;
+                        P[k] = INF;
+                        x[k] = X[imin(i0 + k, n - 1)];
                     }
-                    bot = P[S - 1];
-                    bdiag = above_cell;
-                    if (lane == G - 1 && s + 1 < strips) row[c] = bot;
-                    if (s == strips - 1 && c == m - 1) {
+                }
+                if (c >= pend) up = INF;
+                const double y = __ldg(Y + c), above_cell = up;
+                double dg = bdiag;
 #pragma unroll
-                        for (int k = 0; k < S; k++)
-                            if (i0 + k < n) result = P[k];
-                    }
+                for (int k = 0; k < S; k++) {
+                    const int d = c - (i0 + k);
+                    const double lf = P[k], v = x[k] - y;
+                    double cst = v * v;
+                    if (KIND == K_WDTW)
+                        cst = cst * __ldg(J.weights + abs(c - imin(i0 + k, n - 1)));
+                    double mv = nn_min(up, lf);
+                    if (KIND == K_ADTW) mv = mv + J.p;
+                    double nv = nn_min(mv, dg) + cst;
+                    if (d < B.lo || d > B.mx - 1) nv = INF;
+                    dg = lf;
+                    up = nv;
+                    P[k] = nv;
                 }
-                before = raw;
-                c++;
-                if (any && c >= end) {
-                    s += G;
-                    c -= delta;
+                bot = P[S - 1];
+                bdiag = above_cell;
+                if (lane == G - 1 && s + 1 < strips) row[c] = bot;
+                if (s == strips - 1 && c == m - 1) {
+#pragma unroll
+                    for (int k = 0; k < S; k++)
+                        if (i0 + k < n) result = P[k];
                 }
-                __syncwarp();
             }
-            const double v = sqrt(__shfl_sync(FULL, result, (strips - 1) & (G - 1)));
-            if (lane == 0) {
-                if (J.mode == PM_PAIRED) {
-                    J.out[r1] = v;
-                } else {
-                    J.out[r1 * J.out_ld + c1] = v;
-                    if (J.mode == PM_UPPER) J.out[c1 * J.out_ld + r1] = v;
-                }
+            before = raw;
+            c++;
+            if (any && c >= end) {
+                s += G;
+                c -= delta;
             }
             __syncwarp();
         }
+        const double v = sqrt(__shfl_sync(FULL, result, (strips - 1) & (G - 1)));
+        if (lane == 0) {
+            if (J.mode == PM_PAIRED) {
+                J.out[r1] = v;
+            } else {
+                J.out[r1 * J.out_ld + c1] = v;
+                if (J.mode == PM_UPPER) J.out[c1 * J.out_ld + r1] = v;
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -1209,6 +1208,8 @@ struct Plan {
     int groups = 0, blocks = 0, list_cap = 0, brow_cols = 0;
     int64_t xs = 0, ys = 0;
     int woff = 0, wlen = 0;
+    int64_t left_cap = 0;     // entries of the list of pairs left
+    int64_t tail_cap = 0;     // most pairs left that guided_tail_kernel takes
     size_t shared_bytes = 0;  // copies of the series, their extremes, weights, prep
     size_t thread_bytes = 0;  // per resident thread
 };
@@ -1233,6 +1234,20 @@ int64_t round_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 constexpr size_t kGuidedBudget8 = (size_t)8 << 30;
 constexpr size_t kGuidedBudget16 = (size_t)16 << 30;
 
+// Pairs left that guided_tail_kernel takes: as long as its FP64 instructions (24 a
+// step, 21 cycles of an SM each) take no longer than a thread of the second pass
+// takes for its pair (330 cycles a cell), halved.  2200 of 256 x 256, r = 0.1.
+int64_t tail_pairs(int n, int m, int r) {
+    const int64_t width = imin(m, imax(0, m - n) + imax(0, n - m) + 2 * r - 1);
+    const int64_t strips = (n - 1 + kTailRows - 1) / kTailRows;
+    const int64_t delta = imax(34, imin(m, (int)width + r));
+    const int64_t steps = (strips - 1) / 32 * delta + 31 + m;
+    return std::max<int64_t>(256, device_info().sm_count * n * width / 3 / steps);
+}
+
+// More pairs left than this are found by their outputs, tile by tile.
+constexpr int64_t kLeftCap = (int64_t)1 << 25;
+
 // max_pairs > 0: for lists of at most so many pairs
 Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
     Plan p;
@@ -1249,6 +1264,9 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
     int64_t work = (J.mode == PM_PAIRED ? (J.rows.count + 31) / 32
                                         : (J.rows.count + 31) / 32 * J.cols.count) * 32;
     if (max_pairs > 0) work = std::min(work, max_pairs);
+    p.tail_cap = std::min(work, tail_pairs(n, m, r));
+    // (a list's second pass finds its pairs by their outputs)
+    p.left_cap = max_pairs > 0 ? p.tail_cap : std::min<int64_t>(work, kLeftCap);
     // wdtw between very unequal lengths: the path ends on a diagonal whose weight
     // is up to 10^10 times that of the main one, near which cells cost less than
     // the 32-bit resolution and are all collected.  With two warps per SM their
@@ -1264,11 +1282,11 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
         p.S = S;
         p.groups = (imin(m, width + S - 1) + 3) / 4 + 1;
         p.blocks = p.groups / (S / 4) + 2;
-        // a wide band's pairs with more of its blocks are faster in guided_tail_kernel
-        // (a list's pairs have no such pass: half); 600 x 500 pairs of 900, r =
-        // 0.2: 58 to 61 ms, with half of them 64 to 102, waiting for one pair
-        p.list_cap = imax((n + m) / S + 8,
-                          ns * p.blocks / (max_pairs > 0 || p.blocks < 12 ? 2 : 4));
+        // a wide band's pairs with more of its blocks are faster in guided_tail_kernel or
+        // the second pass; 600 x 500 pairs of 900, r = 0.2: 58 to 61 ms, with half of
+        // them 64 to 102, waiting for one pair (narrow bands: 200 x 150 pairs of 256, r =
+        // 0.1, noise 1.6 ms with half, 1.9 with a fourth)
+        p.list_cap = imax((n + m) / S + 8, ns * p.blocks / (p.blocks < 12 ? 2 : 4));
         p.brow_cols = (int)round_up(m, S);
         p.xs = round_up(3 + 1 + (int64_t)ns * S, 4);
         p.ys = round_up(m, 16);
@@ -1282,7 +1300,7 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
                          align256(J.rows.count * sizeof(GuidedRange)) +
                          align256(J.cols.count * sizeof(GuidedRange)) +
                          align256((size_t)imax(p.wlen, 1) * 4) + align256(sizeof(GuidedPrep)) +
-                         4 * 256;
+                         align256((size_t)p.left_cap * 8) + 4 * 256;
         int nb;
         switch (J.kind) {
             case K_DTW: nb = blocks_per_sm<K_DTW>(S); break;
@@ -1312,7 +1330,9 @@ int run_kernel(const GuidedContext &C, cudaStream_t s) {
 }
 
 int run_tail(const GuidedContext &C, cudaStream_t s) {
-    const int grid = imin(C.grid, 4 * device_info().sm_count);
+    // a warp per pair: at most half the rows of `brow`
+    const int grid = (int)std::min<int64_t>(
+        {(C.args.tail_cap + 3) / 4, C.args.nth / 4, (int64_t)16 * device_info().sm_count});
     switch (C.args.J.kind) {
         case K_DTW: guided_tail_kernel<K_DTW><<<grid, kThreads, 0, s>>>(C.args); break;
         case K_WDTW: guided_tail_kernel<K_WDTW><<<grid, kThreads, 0, s>>>(C.args); break;
@@ -1372,7 +1392,8 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     GuidedArgs &A = C.args;
     A.J = J;
     A.nth = nth;
-    A.need = (unsigned)std::max<int64_t>(kTailPairs, nth / 2);
+    A.need = (unsigned)std::max<int64_t>(p.tail_cap, nth / 2);
+    A.tail_cap = p.tail_cap;
     A.groups = p.groups;
     A.blocks = p.blocks;
     A.list_cap = p.list_cap;
@@ -1396,6 +1417,11 @@ int guided_prepare(const ElasticJob &J, Workspace &ws, size_t leave, int64_t max
     WB_TAKE(ckcol, uint4, ws, (size_t)ns * p.blocks * (p.S / 4) * nth);
     WB_TAKE(list, uint4, ws, (size_t)p.list_cap * (p.S * p.S / 64) * nth);
     WB_TAKE(brow, double, ws, (size_t)2 * p.brow_cols * nth);
+    if (p.left_cap > 0) {
+        WB_TAKE(left, unsigned long long, ws, (size_t)p.left_cap);
+        A.left = left;
+        A.left_cap = p.left_cap;
+    }
     A.prep = prep;
     A.xf = xf;
     A.yf = yf;
@@ -1438,23 +1464,24 @@ int guided_run(const GuidedContext &C, cudaStream_t s) {
     GuidedPrep *prep = C.args.prep;
     WB_CUDA(cudaMemsetAsync(&prep->queue, 0, 4 * sizeof(unsigned long long), s));
     switch (C.args.J.kind) {
-        case K_DTW: return run_kernel<K_DTW>(C, s);
-        case K_WDTW: return run_kernel<K_WDTW>(C, s);
-        default: return run_kernel<K_ADTW>(C, s);
+        case K_DTW: WB_TRY(run_kernel<K_DTW>(C, s)); break;
+        case K_WDTW: WB_TRY(run_kernel<K_WDTW>(C, s)); break;
+        default: WB_TRY(run_kernel<K_ADTW>(C, s));
     }
+    return run_tail(C, s);
 }
 
-int launch_guided(const ElasticJob &J, Workspace &ws, size_t leave,
-                  unsigned long long **pending) {
-    *pending = nullptr;
+int launch_guided(ElasticJob &J, Workspace &ws, size_t leave) {
     GuidedContext C;
     WB_TRY(guided_prepare(J, ws, leave, 0, C));
     if (!C.args.prep) return WB_OK;
     timer_begin("guided_pairs_kernel", ws.stream());
     WB_TRY(guided_run(C, ws.stream()));
     timer_end(ws.stream());
-    WB_TRY(run_tail(C, ws.stream()));
-    *pending = &C.args.prep->pending;
+    J.pending = &C.args.prep->pending;
+    J.left = C.args.left;
+    J.left_cap = C.args.left_cap;
+    J.tail_cap = C.args.tail_cap;
     return WB_OK;
 }
 

@@ -24,7 +24,7 @@ struct GuidedPrep {
     unsigned long long queue;    // next tile of 32 pairs
     unsigned long long pending;  // pairs left to the full recurrence
     unsigned long long seen;     // pairs whose blocks were collected, and of them those
-    unsigned long long heavy;    // with a fourth of the blocks or in a tile with one left
+    unsigned long long heavy;    // left or with a fourth of their blocks
 };
 
 // Extremes of a series: fixed point, and the largest float magnitude.
@@ -50,6 +50,8 @@ struct GuidedArgs {
     const uint32_t *items = nullptr;
     const unsigned *n_items = nullptr;
     int64_t n_all = 0, col0 = 0;
+    unsigned long long *left = nullptr;  // the job's pairs left over (ElasticJob)
+    int64_t left_cap = 0, tail_cap = 0;
     unsigned need = 0;  // pairs seen before the kernel gives up
     // per resident thread, interleaved [...][thread]
     int64_t nth = 0;
@@ -76,7 +78,8 @@ struct GuidedSeries {
 int guided_series(const ElasticJob &job, const GuidedSeries &out, GuidedPrep *prep,
                   cudaStream_t s);
 
-// edr / lcss over the full band, bit-parallel (bit_edit.cu); like launch_guided.
+// edr / lcss over the full band, bit-parallel (bit_edit.cu); *pending is null
+// when it does not run, else the device counter of the pairs left.
 bool bit_edit_supported(const ElasticJob &job);
 size_t bit_edit_bytes(const ElasticJob &job);
 int launch_bit_edit(const ElasticJob &job, Workspace &ws, size_t leave,
@@ -101,12 +104,10 @@ int guided_prepare(const ElasticJob &job, Workspace &ws, size_t leave, int64_t m
                    GuidedContext &ctx);
 int guided_run(const GuidedContext &ctx, cudaStream_t s);
 
-// Evaluates the job on what is left of the workspace beyond `leave` bytes;
-// *pending is null when
-// the job is not guided (or too little is left), else the device counter of
-// the pairs whose output is kGuidedPending.
-int launch_guided(const ElasticJob &job, Workspace &ws, size_t leave,
-                  unsigned long long **pending);
+// Evaluates the job on what is left of the workspace beyond `leave` bytes and sets
+// job.pending and job.left for the second pass; they stay null when the job is not
+// guided (or too little is left).
+int launch_guided(ElasticJob &job, Workspace &ws, size_t leave);
 
 // argmin_distance of the dtw family over float32 bounds and guided
 // evaluations (argmin_guided.cu).
@@ -117,8 +118,8 @@ std::vector<int64_t> argmin_guided_chunks(int64_t nq, int64_t ny, int64_t k);
 class GuidedArgmin {
   public:
     int prepare(const ElasticJob &job, Workspace &ws, size_t leave, bool &ok);
-    int launch_chunk(int index, const EaChunk &chunk, cudaStream_t s,
-                     const unsigned long long **pending);
+    // sets job.pending for the second pass
+    int launch_chunk(int index, const EaChunk &chunk, cudaStream_t s, ElasticJob &job);
 
   private:
     struct Impl;
@@ -194,6 +195,22 @@ struct Band {
 
 __device__ __forceinline__ bool is_pending(double v) {
     return __double_as_longlong(v) == kGuidedPending;
+}
+// Pair number q of the list of those left, and its output.
+__device__ __forceinline__ double *left_pair(const ElasticJob &J, int64_t q, int64_t &rs,
+                                             int64_t &cs) {
+    const int64_t id = (int64_t)J.left[q];
+    rs = cs = id;
+    if (J.mode == PM_PAIRED) return J.out + rs;
+    cs = id / J.rows.count;
+    rs = id - cs * J.rows.count;
+    return J.out + rs * J.out_ld + cs;
+}
+// This thread's number where the warps of all blocks come first, so that a few lists'
+// worth of warps spread over the SMs.
+__device__ __forceinline__ int64_t spread_lane() {
+    const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    return warp * 32 + (threadIdx.x & 31);
 }
 #endif
 
