@@ -101,6 +101,9 @@ int launch_elastic_external_ring(const ElasticJob &job, double *ring, size_t rin
 // The shared-memory ring kernels (and the tiled euclidean kernel) without any
 // workspace; WB_EUNSUPPORTED when the band ring does not fit in shared memory.
 int launch_elastic_shared_ring(const ElasticJob &job, cudaStream_t s);
+// Blocks (of 128 threads) of the shared-memory ring kernels that an SM holds, 0 where
+// the band ring does not fit.
+int shared_ring_blocks(const ElasticJob &job);
 // Workspace launch_elastic needs, and what the guided evaluation adds (0: not used).
 size_t elastic_workspace_bytes(const ElasticJob &job);
 size_t guided_workspace_bytes(const ElasticJob &job);

@@ -174,20 +174,24 @@ struct ElasticPlan {
     size_t gring_bytes;
 };
 
+int shared_ring_blocks(const ElasticJob &J) {
+    const DeviceInfo &dev = device_info();
+    const int P = imax(2, ring_len(J.rows.len, J.cols.len, J.band));
+    const size_t per_block = (size_t)P * kThreads * sizeof(double);
+    if (per_block > (size_t)dev.smem_per_sm - 2048 || per_block > (size_t)dev.max_smem_optin)
+        return 0;
+    return (int)std::min<size_t>(4, ((size_t)dev.smem_per_sm - 1024) / (per_block + 1024));
+}
+
 static ElasticPlan plan_elastic(const ElasticJob &J) {
     const DeviceInfo &dev = device_info();
     ElasticPlan pl;
     pl.P = imax(2, ring_len(J.rows.len, J.cols.len, J.band));
-    const size_t per_block = (size_t)pl.P * kThreads * sizeof(double);
     int64_t work_threads;
     if (J.mode == PM_PAIRED) work_threads = J.rows.count;
     else work_threads = ((J.rows.count + 31) / 32) * 32 * J.cols.count;
     int64_t want_blocks = (work_threads + kThreads - 1) / kThreads;
-    int blocks_per_sm = 0;
-    if (per_block <= (size_t)dev.smem_per_sm - 2048 && per_block <= (size_t)dev.max_smem_optin) {
-        blocks_per_sm = (int)(((size_t)dev.smem_per_sm - 1024) / (per_block + 1024));
-        if (blocks_per_sm > 4) blocks_per_sm = 4;
-    }
+    const int blocks_per_sm = shared_ring_blocks(J);
     // a ring that leaves fewer than 4 warps per SM goes to global memory
     if (blocks_per_sm >= 1) {
         pl.gring = false;

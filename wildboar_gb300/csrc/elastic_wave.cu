@@ -22,6 +22,10 @@
 //     |x_{i-1} - y_{j-1}| is the previous diagonal cell's |x_i - y_j|, and the
 //     stiffness of a diagonal moves down a strip instead of being loaded (200 x
 //     150 pairs of 256 34.1 -> 32.4 ms).
+// With one lane per pair the last strip evaluates its own rows only (with G > 1 the
+// lanes of a warp are at different strips, which would run one after the other):
+// erp, 700 x 700 pairs of 57 (8 strips, the last of 1 row) 15.4 -> 13.9 ms, msm, 400
+// x 400 of 60 6.7 -> 5.6.
 // Measured on one GB300 against the strip and ring kernels (one thread per
 // pair, whose busiest SM had 1.27 times the mean): msm, 301 x 290 pairs of 256 x
 // 250 111.7 -> 50.9 ms (44 ms of FP64 instructions), 9 x 10 of 256 26.2 ->
@@ -32,6 +36,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "guided.cuh"
 
@@ -230,33 +235,40 @@ __global__ void __launch_bounds__(32)
                         for (int k = kRows - 1; k > 0; k--) st[k] = st[k - 1];
                         st[0] = s0;
                     }
+                    auto column = [&](auto part) {
+                        constexpr bool SHORT = decltype(part)::value;
 #pragma unroll
-                    for (int k = 0; k < kRows; k++) {
-                        const double lf = P[k];
-                        double nv;
-                        if constexpr (KIND == K_ERP) {
-                            nv = nn_min(dg + fabs(x[k] - y), nn_min(up + rx[k], lf + colv));
-                        } else if constexpr (KIND == K_MSM) {
-                            const float px = k ? xf[k > 0 ? k - 1 : 0] : pxf;
-                            const float fx = fabsf(__fsub_rn(xf[k], yf));
-                            const float dx = fabsf(__fsub_rn(xf[k], px));
-                            const double both = add_nonneg(cf, fx);
-                            double cu = fx < dx ? both : rx[k];
-                            if (between(xf[k], px, yf)) cu = cd;
-                            double cl = dyf < fx ? colv : both;
-                            if (between(yf, xf[k], ypf)) cl = cd;
-                            nv = nn_min(nn_min(dg + fabs(x[k] - y), up + cu), lf + cl);
-                        } else {
-                            const double del = nn_min(up + rx[k], lf + colv) + pen;
-                            const double a = abs_of(x[k] - y);
-                            nv = nn_min(del, ((dg + a) + adg) + st[k]);
-                            adg = ad[k];
-                            ad[k] = a;
+                        for (int k = 0; k < kRows; k++) {
+                            if (SHORT && k >= rows) continue;
+                            const double lf = P[k];
+                            double nv;
+                            if constexpr (KIND == K_ERP) {
+                                nv = nn_min(dg + fabs(x[k] - y), nn_min(up + rx[k], lf + colv));
+                            } else if constexpr (KIND == K_MSM) {
+                                const float px = k ? xf[k > 0 ? k - 1 : 0] : pxf;
+                                const float fx = fabsf(__fsub_rn(xf[k], yf));
+                                const float dx = fabsf(__fsub_rn(xf[k], px));
+                                const double both = add_nonneg(cf, fx);
+                                double cu = fx < dx ? both : rx[k];
+                                if (between(xf[k], px, yf)) cu = cd;
+                                double cl = dyf < fx ? colv : both;
+                                if (between(yf, xf[k], ypf)) cl = cd;
+                                nv = nn_min(nn_min(dg + fabs(x[k] - y), up + cu), lf + cl);
+                            } else {
+                                const double del = nn_min(up + rx[k], lf + colv) + pen;
+                                const double a = abs_of(x[k] - y);
+                                nv = nn_min(del, ((dg + a) + adg) + st[k]);
+                                adg = ad[k];
+                                ad[k] = a;
+                            }
+                            dg = lf;
+                            up = nv;
+                            P[k] = nv;
                         }
-                        dg = lf;
-                        up = nv;
-                        P[k] = nv;
-                    }
+                    };
+                    // (with one lane per pair the warp's strips have the same rows)
+                    if (G == 1 && rows < kRows) column(std::true_type{});
+                    else column(std::false_type{});
                 }
                 bot = P[kRows - 1];
                 bdiag = upper;
@@ -316,9 +328,10 @@ Plan plan_kind(const ElasticJob &J) {
         const int64_t warps = (p.pairs * G + 31) / 32;
         const int64_t turns = (warps + resident - 1) / resident;
         const int64_t grid = (warps + turns - 1) / turns;
-        const int64_t steps =
-            ((strips + G - 1) / G - 1) * (int64_t)imax(m, G + 2) + m + G - 1;
-        const double cost = (double)turns * (double)steps *
+        double steps =
+            (double)(((strips + G - 1) / G - 1) * (int64_t)imax(m, G + 2) + m + G - 1);
+        if (G == 1) steps = (double)m * n / kRows;  // the last strip's own rows
+        const double cost = (double)turns * steps *
                             std::hypot(kAlone, (double)((grid + sms - 1) / sms));
         if (!p.lanes || cost < best) {
             best = cost;
@@ -340,7 +353,8 @@ Plan plan_wave(const ElasticJob &J) {
 
 }  // namespace
 
-// erp, msm and twe without a band edge inside the matrix
+// erp, msm and twe without a band edge inside the matrix, where this is the faster
+// form
 bool wave_supported(const ElasticJob &J) {
     if (J.kind != K_ERP && J.kind != K_MSM && J.kind != K_TWE) return false;
     if (J.key || J.all_zero || J.pending) return false;
@@ -350,7 +364,19 @@ bool wave_supported(const ElasticJob &J) {
     const int least = J.kind == K_MSM ? 2 : 1;
     // a negative (or NaN) c has no place in add_nonneg
     if (n < least || m < least || (J.kind == K_MSM && !(J.c >= 0.0))) return false;
-    return imax(0, n - m) + J.band >= n && imax(0, m - n) + J.band >= m;
+    if (imax(0, n - m) + J.band < n || imax(0, m - n) + J.band < m) return false;
+    // Many pairs of short twe series stay with the ring kernel, whose 32 rows to a
+    // column read the column's tables once: 1.03 to 1.07 times as fast (length 24 to
+    // 111) where it has 6 tiles and more for each of its warps, two blocks' rings fit
+    // an SM and the rows fill the tiles; with one block, or 2 to 4 tiles a warp, or
+    // 100 rows (of 128), it takes 1.07 to 1.38 times as long.
+    if (J.kind == K_TWE && J.mode == PM_ALL) {
+        const int64_t blocks = shared_ring_blocks(J), chunks = (J.rows.count + 31) / 32;
+        if (blocks >= 2 && 20 * J.rows.count >= 19 * 32 * chunks &&
+            chunks * J.cols.count >= 24 * blocks * device_info().sm_count)
+            return false;
+    }
+    return true;
 }
 
 size_t wave_bytes(const ElasticJob &J) { return plan_wave(J).bytes; }
