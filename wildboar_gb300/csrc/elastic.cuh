@@ -139,6 +139,8 @@ struct SubseqElasticJob {
     // with kept[pair] <= 0, *redo of them
     const int *kept = nullptr;
     const unsigned long long *redo = nullptr;
+    // [pair] what the minimum's sum is known not to exceed (above 1e300: nothing)
+    const double *start = nullptr;
 };
 size_t elastic_subseq_ring_bytes(const SubseqElasticJob &J, int max_len, int max_band,
                                  int *P_out, int *grid_out);

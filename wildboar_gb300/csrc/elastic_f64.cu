@@ -440,7 +440,8 @@ elastic_subseq_kernel(const SubseqElasticJob J, double *gring, int P) {
         double gx_sum = 0.0;
         if (KIND == K_ERP)
             for (int k = 0; k < L; k++) gx_sum = gx_sum + fabs(S[k] - J.g);
-        double min_dist = INF;
+        double min_dist = INF, start = INF;
+        if (KIND == K_DTW && J.start && J.start[oidx] < 1e300) start = J.start[oidx];
         int best = 0;
         for (int base = 0; base < nwin; base += 32) {
             const int w = base + lane;
@@ -451,10 +452,12 @@ elastic_subseq_kernel(const SubseqElasticJob J, double *gring, int P) {
             // abandoned window's partial key already exceeds the threshold its
             // replay compares it with.  Adjacent windows overlap, so a round
             // far from every good match abandons in all its lanes together.
-            const double bound =
+            double bound =
                 (J.prof_raw || KIND == K_LCSS) ? INF
                                                : subseq_threshold(J.metric, min_dist, L,
                                                                   J.t_len_thr);
+            // (a window above it is not the minimum)
+            if (KIND == K_DTW) bound = start < bound ? start : bound;
             if (w < nwin) {
                 const double *Y = T + w;
                 double raw;

@@ -58,6 +58,7 @@ struct FilterArgs {
     uint32_t *windows = nullptr;  // [pair][kKeep]
     double *sums = nullptr;       // [pair][kKeep] their FP64 sums
     int *kept = nullptr;          // [pair]
+    double *start = nullptr;      // [pair] bound of the smallest sum, for the FP64 scan
     uint32_t *extra = nullptr;    // pair kKeep + q of the kept windows q >= 1
     unsigned *n_extra = nullptr;
     int per_block = 1;            // shapelets per block
@@ -301,6 +302,8 @@ __global__ void __launch_bounds__(kThreads) subseq_filter_kernel(const FilterArg
             // 0: the FP64 scan takes the pair
             if (full || count > kKeep) count = 0;
             if (lane == 0) {
+                // (`bound` is one of the smallest FP64 sum too, in scaled values)
+                if (bound < FLT_MAX) A.start[pair] = (double)bound * 1.000001 / (scale * scale);
                 A.kept[pair] = count;
                 if (count > 1) {
                     const unsigned at = atomicAdd(A.n_extra, (unsigned)(count - 1));
@@ -387,6 +390,7 @@ size_t subseq_filter_bytes(const SubseqElasticJob &J, int64_t total) {
            align256(J.x.count * 4) + align256(J.m * 4) + align256(total * 8) +
            align256(pairs * kKeep * 4) + align256(pairs * kKeep * 8) +
            align256(pairs * (kKeep - 1) * 4) + 2 * align256(pairs * 4 + 4) +
+           align256(pairs * 8) +
            align256(sizeof(GuidedPrep)) + 4096;
 }
 
@@ -405,6 +409,7 @@ int launch_subseq_filter(SubseqElasticJob &J, int64_t total, double *gring, int 
     WB_TAKE(sums, double, ws, pairs * kKeep);
     WB_TAKE(extra, uint32_t, ws, pairs * (kKeep - 1));
     WB_TAKE(n_extra, unsigned, ws, 1);
+    WB_TAKE(start, double, ws, pairs);
     A.J = J;
     A.prep = prep;
     A.xf = xf;
@@ -417,12 +422,14 @@ int launch_subseq_filter(SubseqElasticJob &J, int64_t total, double *gring, int 
     A.sums = sums;
     A.extra = extra;
     A.n_extra = n_extra;
+    A.start = start;
     const DeviceInfo &dev = device_info();
     const int64_t cap = (int64_t)dev.sm_count * 4;
     WB_CUDA(cudaMemsetAsync(&prep->lo, 0x7f, sizeof(prep->lo), s));
     WB_CUDA(cudaMemsetAsync(&prep->hi, 0x80, sizeof(prep->hi), s));
     WB_CUDA(cudaMemsetAsync(&prep->queue, 0, sizeof(prep->queue) + sizeof(prep->pending), s));
     WB_CUDA(cudaMemsetAsync(kept, 0, pairs * sizeof(int), s));
+    WB_CUDA(cudaMemsetAsync(start, 0x7f, pairs * sizeof(double), s));  // 1.4e306
     WB_CUDA(cudaMemsetAsync(n_extra, 0, sizeof(unsigned), s));
     const int prep_grid = (int)std::min(cap, (J.x.count + J.m + 7) / 8);
     filter_range_kernel<<<prep_grid, 256, 0, s>>>(J, prep);
@@ -451,6 +458,7 @@ int launch_subseq_filter(SubseqElasticJob &J, int64_t total, double *gring, int 
     WB_LAUNCH_CHECK("subseq_select_kernel");
     J.kept = kept;
     J.redo = &prep->pending;
+    J.start = start;
     return WB_OK;
 }
 
