@@ -194,7 +194,7 @@ def test_a_shared_memory_limit_is_never_lowered(ws):
     assert ws.t_limit(1) >= 100_000
     assert ws.t_allow(1, 224_256) == 0 and ws.t_sets() == 1  # set once, to all there is
     assert ws.t_allow(1, 224_257) != 0  # more than the device has
-    assert ws.t_allow(2, 40_000) == 0 and ws.t_sets() == 2  # within the default
+    assert ws.t_allow(2, 40_000) == 0 and ws.t_allow(2, 200_000) == 0 and ws.t_sets() == 2
 
 
 def test_no_call_sets_a_limit_by_itself():

@@ -844,7 +844,7 @@ static int subseq_elastic(const double *shapelets, const int64_t *offsets,
                   (metric == WB_ERP ? align256((size_t)x->n * T * 8) + align256(x->n * 8) : 0) +
                   (metric == WB_TWE ? align256((size_t)max_orig * 8 + 8) : 0) +
                   (out_on_device ? 0 : 2 * align256(n_out * 8));
-    const bool filter = !profile && subseq_filter_supported(J, kind, max_band);
+    const bool filter = !profile && subseq_filter_supported(J, kind, max_band, total);
     const size_t filter_bytes = filter ? subseq_filter_bytes(J, total) : 0;
     WB_TRY(ws.reserve(need + filter_bytes, need));
     WB_TAKE(gring, double, ws, ring / sizeof(double));
@@ -1119,7 +1119,7 @@ static int subseq_entry(const double *shapelets, const int64_t *offsets, const i
     J.x.len = (int)x->n_timestep;
     need += subseq_workspace_bytes(J, scaled);
     const size_t filter_bytes =
-        !profile && subseq_dot_supported(J) ? subseq_dot_bytes(J, scaled) : 0;
+        !profile && subseq_dot_supported(J, scaled) ? subseq_dot_bytes(J, scaled) : 0;
     WB_TRY(ws.reserve(need + filter_bytes, need));
     WB_TRY(stage(x, dim, ws, J.x));
     if (stop_sq) {

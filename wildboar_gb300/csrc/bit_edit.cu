@@ -206,6 +206,7 @@ Plan plan_bits(const ElasticJob &J) {
 bool bit_edit_supported(const ElasticJob &J) {
     if (J.kind != K_EDR && J.kind != K_LCSS) return false;
     if (J.key || J.all_zero || J.pending) return false;
+    if (J.mode == PM_UPPER && J.rows.count < 2) return false;  // no pairs
     const char *e = getenv("WB_GPU_ELASTIC");
     if (e && (strcmp(e, "ring") == 0 || strcmp(e, "strip") == 0)) return false;
     const int n = J.rows.len, m = J.cols.len;

@@ -125,11 +125,11 @@ struct DeviceInfo {
 };
 const DeviceInfo &device_info();
 
-// Raises a kernel's limit of dynamic shared memory to all that the device has
-// beside its static part, where `bytes` is above the present one.  The limit
-// belongs to the kernel, not to a launch: set to what a call needs, it could be
-// lowered by another thread's call of the same kernel before this one launches,
-// which then fails.
+// Sets a kernel's limit of dynamic shared memory, once, to all that the device has
+// beside its static part; fails where `bytes` is more than that.  The limit belongs
+// to the kernel, not to a launch: set to what a call needs, it could be lowered by
+// another thread's call of the same kernel before this one launches, which then
+// fails.
 cudaError_t allow_shared(const void *kernel, size_t bytes);
 template <class K>
 cudaError_t allow_shared(K *kernel, size_t bytes) {

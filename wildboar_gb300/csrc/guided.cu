@@ -1254,6 +1254,7 @@ Plan plan_guided(const ElasticJob &J, size_t avail, int64_t max_pairs = 0) {
     const int n = J.rows.len, m = J.cols.len, r = J.band;
     if (J.kind != K_DTW && J.kind != K_WDTW && J.kind != K_ADTW) return p;
     if ((J.key && max_pairs == 0) || J.all_zero || J.pending) return p;
+    if (J.mode == PM_UPPER && J.rows.count < 2) return p;  // no pairs
     const char *e = getenv("WB_GPU_ELASTIC");
     if (e && (strcmp(e, "ring") == 0 || strcmp(e, "strip") == 0)) return p;
     const int mx = imax(0, m - n) + r, mn = imax(0, n - m);

@@ -581,7 +581,7 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
             return fail(WB_ENOMEM, "workspace reservation exceeded");
         shapelet_norm_kernel<<<(int)(J.m < 65535 ? J.m : 65535), 128, 0, s>>>(J, norm);
         WB_LAUNCH_CHECK("shapelet_norm_kernel");
-        if (subseq_dot_supported(J) &&
+        if (subseq_dot_supported(J, true) &&
             ws.remaining() >= subseq_dot_bytes(J, true) + scan_bytes(J)) {
             WB_TRY(launch_subseq_dot(J, true, norm, mean_tab, std_tab, host.order, host.lengths,
                                      host.group_of, host.uploads, ws));
@@ -624,7 +624,7 @@ int launch_subseq(const SubseqJob &job, bool scaled, Workspace &ws, SubseqHost &
         timer_end(s);
         WB_LAUNCH_CHECK("subseq_paired_kernel");
     } else {
-        if (subseq_dot_supported(J) &&
+        if (subseq_dot_supported(J, false) &&
             ws.remaining() >= subseq_dot_bytes(J, false) + scan_bytes(J))
             WB_TRY(launch_subseq_dot(J, false, nullptr, nullptr, nullptr, host.order, host.lengths,
                                      host.group_of, host.uploads, ws));

@@ -75,7 +75,7 @@ int launch_subseq(const SubseqJob &J, bool scaled, Workspace &ws, SubseqHost &ho
 // and sets J.kept / J.redo for the scan of the others.  Scaled: `norm` holds
 // the normalised shapelets; ex / ex2 receive the windows' running sums and, if
 // pairs are left, their means and standard deviations.
-bool subseq_dot_supported(const SubseqJob &J);
+bool subseq_dot_supported(const SubseqJob &J, bool scaled);
 size_t subseq_dot_bytes(const SubseqJob &J, bool scaled);
 int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex, double *ex2,
                       const std::vector<int64_t> &order, const std::vector<int64_t> &hlen,

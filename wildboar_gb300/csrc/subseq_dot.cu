@@ -599,8 +599,22 @@ static void plan_quads(const std::vector<int64_t> &order, const std::vector<int6
     }
 }
 
-bool subseq_dot_supported(const SubseqJob &J) {
+bool subseq_dot_supported(const SubseqJob &J, bool scaled) {
     const int64_t pairs = J.x.count * J.m;
+    // The filter's launches take 50 us more than the scan's where that has little to
+    // do.  A scan's warp takes about 1 us for a value of a shapelet in its first
+    // windows (FP64) and 12 ns in every further 32 (float, abandoned early): 20 x 100
+    // of 30 x 300 values, 165 us so, 0.50 ms in all and 0.42 with the filter, 5 x 400,
+    // 66 us, 0.42 and 0.42, 1 x 10 of 10 x 100, 10 us, 0.32 and 0.36.  (Scaled windows:
+    // from the first on, 5 x 400 1.3 and 0.7 ms.)
+    if (!scaled) {
+        const double len = (double)J.total_values / (double)std::max<int64_t>(J.m, 1);
+        const int64_t chunks = (J.m + J.chunk - 1) / J.chunk;
+        const int64_t turns = 1 + J.x.count * chunks / (8 * device_info().sm_count);
+        const double us = (double)((std::min<int64_t>(J.m, J.chunk) + 3) / 4 * turns) * len *
+                          (1.0 + 0.012 * (J.x.len - len) / 32.0);
+        if (us < 70.0) return false;
+    }
     return !J.paired && J.x.len <= kMaxSeries && pairs < ((int64_t)1 << 31) / kKeep &&
            pairs * kKeep * 16 <= (int64_t)2 << 30;
 }

@@ -378,7 +378,14 @@ int64_t pairs_of(const SubseqElasticJob &J) { return J.paired ? J.x.count : J.x.
 
 }  // namespace
 
-bool subseq_filter_supported(const SubseqElasticJob &J, int kind, int max_band) {
+bool subseq_filter_supported(const SubseqElasticJob &J, int kind, int max_band, int64_t total) {
+    // The filter's launches take 35 us more than the scan's where that has little to
+    // do: band cells of 32 windows that a scan's warp evaluates, 330 cycles each (1 x
+    // 10 of 10 and 100 values, 40 cells, 0.33 ms, with the filter 0.36; 5 x 400 of 30 and
+    // 300, 1350 cells, 0.89 and 0.46).
+    const int64_t len = total / std::max<int64_t>(J.m, 1);
+    const int64_t turns = 1 + pairs_of(J) / (16 * device_info().sm_count);
+    if ((J.x.len - len) / 32 * len * (2 * max_band - 1) * turns < 200) return false;
     return kind == K_DTW && !J.prof_raw && J.x.len <= kMaxSeries &&
            2 * max_band - 1 <= 8 * kMaxBlocks && pairs_of(J) < ((int64_t)1 << 31) / kKeep &&
            pairs_of(J) * kKeep * 16 <= (int64_t)2 << 30;

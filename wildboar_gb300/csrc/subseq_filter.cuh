@@ -8,7 +8,7 @@ namespace wb {
 
 // The filter takes the job (max_band: its widest half-band); `total` packed
 // shapelet values.
-bool subseq_filter_supported(const SubseqElasticJob &J, int kind, int max_band);
+bool subseq_filter_supported(const SubseqElasticJob &J, int kind, int max_band, int64_t total);
 size_t subseq_filter_bytes(const SubseqElasticJob &J, int64_t total);
 // Writes the results of the pairs it settles and sets J.kept / J.redo, so that
 // launch_elastic_subseq(J) scans the others.  gring, P, grid: that kernel's.

@@ -115,13 +115,23 @@ int Workspace::reserve(size_t bytes, size_t least) {
     return WB_OK;
 }
 
+// (asking the runtime takes some 20 us a call, so what was set is kept)
 cudaError_t allow_shared(const void *kernel, size_t bytes) {
-    cudaFuncAttributes at;
-    cudaError_t e = cudaFuncGetAttributes(&at, kernel);
-    if (e != cudaSuccess || (size_t)at.maxDynamicSharedSizeBytes >= bytes) return e;
-    const int most = device_info().max_smem_optin - (int)at.sharedSizeBytes;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                bytes > (size_t)imax(most, 0) ? (int)bytes : most);
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limits;
+    const DeviceInfo &dev = device_info();
+    std::lock_guard<std::mutex> g(mu);
+    size_t &limit = limits[std::make_pair(dev.device, kernel)];
+    if (limit == 0) {
+        cudaFuncAttributes at;
+        cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+        if (e != cudaSuccess) return e;
+        const int most = dev.max_smem_optin - (int)at.sharedSizeBytes;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return e;
+        limit = (size_t)imax(most, 0);
+    }
+    return bytes <= limit ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 }  // namespace wb
