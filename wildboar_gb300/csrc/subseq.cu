@@ -181,6 +181,12 @@ subseq_scan_kernel(const SubseqJob J, const double *norm, const double *mean_tab
             const float *Sf = filt ? J.shp_f32 + J.offsets[idx] : nullptr;
             const float e = filt ? filter_e(MT, J.shp_absmax[idx]) : 0.0f;
             float thr32 = __int_as_float(0x7f800000);
+            const bool known = !SCALED && J.start && J.start[si * J.m + idx] < 1e300;
+            if (known) {  // only windows below it are taken
+                best = J.start[si * J.m + idx];
+                bidx = -1;
+                if (filt) thr32 = filter_threshold(__double2float_ru(best), e, L);
+            }
             // Windows that pass the filter wait in a FIFO (ascending window
             // order) and are summed in FP64 32 at a time, so the FP64 pipe
             // works on full warps.  The order of evaluation stays ascending,
@@ -253,6 +259,10 @@ subseq_scan_kernel(const SubseqJob J, const double *norm, const double *mean_tab
                 if (qn >= 32) eval_batch(32);
             }
             if (qn > 0) eval_batch(qn);
+            if (bidx < 0) {  // no finite sum
+                best = INF;
+                bidx = 0;
+            }
             if (lane == 0) {
                 J.out_dist[si * J.m + idx] = sqrt(best);
                 J.out_idx[si * J.m + idx] = bidx;

@@ -47,6 +47,8 @@ struct SubseqJob {
     const int *kept = nullptr;
     const unsigned long long *redo = nullptr;
     const unsigned char *redo_rows = nullptr;
+    // euclidean: [pair] what the minimum's sum is below (above 1e300: nothing)
+    const double *start = nullptr;
     double *out_dist = nullptr;          // (x.count, m)
     int64_t *out_idx = nullptr;          // (x.count, m)
 };

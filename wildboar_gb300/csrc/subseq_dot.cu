@@ -89,6 +89,7 @@ struct DotArgs {
     uint32_t *windows = nullptr;            // [pair][kKeep]
     double *sums = nullptr;
     int *kept = nullptr;
+    double *start = nullptr;                // euclidean: [pair] bound of the smallest sum
     uint32_t *extra = nullptr;
     unsigned *n_extra = nullptr;
 };
@@ -472,6 +473,8 @@ __global__ void __launch_bounds__(kThreads, 5) dot_filter_kernel(const DotArgs A
                 }
                 if (n > kCand || kept > kKeep) kept = 0;
                 if (lane == 0) {
+                    if (!SCALED && limit < FLT_MAX)
+                        A.start[pair] = (double)limit * 1.000001 / (scale * scale);
                     A.kept[pair] = kept;
                     if (kept > 1) {
                         const unsigned at = atomicAdd(A.n_extra, (unsigned)(kept - 1));
@@ -625,7 +628,7 @@ size_t subseq_dot_bytes(const SubseqJob &J, bool scaled) {
     return align256(J.m * sizeof(Quad)) + align256(J.m * sizeof(Unit)) +
            align256((J.total_values + 8 * J.m) * 16) + align256(J.m * 4 * sizeof(float2)) +
            align256(J.x.count * (int64_t)J.x.len * 4) + align256(J.x.count * 4) +
-           (scaled ? 0 : align256(J.x.count * ((int64_t)J.x.len + 1) * 8)) +
+           (scaled ? 0 : align256(J.x.count * ((int64_t)J.x.len + 1) * 8) + align256(pairs * 8)) +
            align256(sizeof(GuidedPrep)) + align256((scaled ? J.x.count : 1) * sizeof(Range)) +
            align256(pairs * kKeep * 4) +
            align256(pairs * kKeep * 8) + align256(pairs * 4) +
@@ -650,10 +653,12 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     WB_TAKE(sn, float2, ws, nq * 4);
     WB_TAKE(xf, float, ws, J.x.count * (int64_t)J.x.len);
     WB_TAKE(xmax2, float, ws, J.x.count);
-    double *prefix = nullptr;
+    double *prefix = nullptr, *start = nullptr;
     if (!scaled) {
         prefix = ws.take<double>(J.x.count * ((int64_t)J.x.len + 1));
-        if (!prefix) return fail(WB_ENOMEM, "workspace reservation exceeded");
+        start = ws.take<double>(pairs);
+        if (!prefix || !start) return fail(WB_ENOMEM, "workspace reservation exceeded");
+        WB_CUDA(cudaMemsetAsync(start, 0x7f, pairs * sizeof(double), s));  // 1.4e306
     }
     WB_TAKE(windows, uint32_t, ws, pairs * kKeep);
     WB_TAKE(sums, double, ws, pairs * kKeep);
@@ -689,6 +694,7 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     A.windows = windows;
     A.sums = sums;
     A.kept = kept;
+    A.start = start;
     A.extra = extra;
     A.n_extra = n_extra;
     const DeviceInfo &dev = device_info();
@@ -736,6 +742,7 @@ int launch_subseq_dot(SubseqJob &J, bool scaled, const double *norm, double *ex,
     J.kept = kept;
     J.redo = &prep->pending;
     J.redo_rows = redo_rows;
+    J.start = start;
     return WB_OK;
 }
 
