@@ -952,7 +952,7 @@ __device__ __forceinline__ void keep_region(const DirKeep &D, int64_t base, int 
 
 // The sweep with directions of every item into its batch region, and the
 // distance sqrt(hi + lo) of the same sweep (compensated predecessor choice).
-// Bound: issue and ALU of the 18 instructions of a cell.  Columns go in pairs,
+// Bound: issue and ALU of the 19.8 instructions of a cell.  Columns go in pairs,
 // those with rows out of band too (32 of 117 at r = 0.2, length 256: one at a time
 // they waited on the chain of their rows): 131072 items of 256, r = 0.2, 2.92 ->
 // 2.63 ms.  Packed differences and selections under predicates (14 instructions)

@@ -28,7 +28,7 @@
 // x 400 of 60 6.7 -> 5.6.
 // Measured on one GB300 against the strip and ring kernels (one thread per
 // pair, whose busiest SM had 1.27 times the mean): msm, 301 x 290 pairs of 256 x
-// 250 111.7 -> 50.9 ms (44 ms of FP64 instructions), 9 x 10 of 256 26.2 ->
+// 250 111.7 -> 48.6 ms (44 ms of FP64 instructions), 9 x 10 of 256 26.2 ->
 // 0.94 ms; twe, 20 x 20 of 500 95.8 -> 3.0 ms; erp, 200 x 150 of 256 20.9 -> 16.9
 // ms.
 
@@ -305,7 +305,8 @@ struct Plan {
 // A warp that has an SM to itself takes 525 cycles for a cell of msm, one of
 // many 93: their ratio.  Measured (msm, length 256, lanes 1 .. 32, ms): 9 x 10
 // pairs 16.3, 8.4, 4.4, 2.4, 1.43, 0.94; 60 x 50 16.3, 8.5, 4.5, 2.6, 2.2, 2.5;
-// 301 x 290 51.8, 49.4, 52.0, 50.9, 53.5, 60.8; length 60, 900 x 800: 24.7,
+// 301 x 290 51.8, 49.4, 52.0, 50.9, 53.5, 60.8 (1 lane 48.5 since the last strip has its
+// own rows only); length 60, 900 x 800: 24.7,
 // 25.9, 27.1, 30.4, 60.0, 118.8.
 constexpr double kAlone = 5.5;
 

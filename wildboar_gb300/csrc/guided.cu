@@ -54,14 +54,14 @@
 // and in fixed point too 2^-23 + 2^-24 of A_max on either side, since the penalty
 // is a float before it is in units.)
 //
-// Pairs whose collected cells do not fit the thread's list (a fourth to half of
-// the band's blocks: long runs of equal values tie everywhere) or whose inputs
-// are not finite are left to the full recurrence: their output holds
-// kGuidedPending until guided_tail_kernel (few pairs) or launch_elastic's second
-// pass over exactly those pairs.
+// Pairs whose collected cells do not fit the thread's list (a fourth of the band's
+// blocks, half of a narrow band's: long runs of equal values tie everywhere) or whose
+// inputs are not finite are left to the full recurrence: their output holds
+// kGuidedPending, and a list of them goes to guided_tail_kernel (few pairs) or to
+// launch_elastic's second pass.
 //
 // Measured on one GB300 (full recurrence -> guided): dtw r = 0.1, 1000 x 1000,
-// length 512: 292 -> 36 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 9.3
+// length 512: 292 -> 36 ms; r = 1, 310 x 301, lengths 400 and 361: 96 -> 8.9
 // ms; wdtw r = 1, 500 x 403, length 256: 107 -> 9.0 ms.  Of the first, the
 // sweep takes a third, the walk a fourth and the FP64 part two fifths (2100
 // iterations for the 890 cells of a pair: lanes wait for the turn's longest
@@ -1228,8 +1228,8 @@ int64_t round_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
 // Budget of the kept rows and columns of all resident pairs, for blocks of 8
 // cells and of 16.  Where 8 cells need more, their rows and columns bound the
-// kernel by DRAM writes (310 x 301 pairs of 400 x 361, r = 1: 10.3 ms with 12 GB,
-// 8.1 with blocks of 16); blocks of 16 are worth every resident warp (600 x 500
+// kernel by DRAM writes (310 x 301 pairs of 400 x 361, r = 1: 2.2 ms more with 12 GB
+// than the 8.1 to 9.3 of blocks of 16); blocks of 16 are worth every resident warp (600 x 500
 // pairs of 900, r = 0.2, 14 GB: 84 -> 71 ms against the 62 % that 8 GB hold).
 constexpr size_t kGuidedBudget8 = (size_t)8 << 30;
 constexpr size_t kGuidedBudget16 = (size_t)16 << 30;

@@ -37,7 +37,7 @@
 //
 // Measured on one GB300: 2000 z-normalised shapelets of 16 to 128 values x 400
 // series of 1024: 158.5 ms (FP64 divisions per window tile and a float scan
-// per shapelet) -> 10.0 ms, of which the filter takes 4.0, the running sums 1.0
+// per shapelet) -> 9.9 ms, of which the filter takes 4.0, the running sums 1.0
 // and the FP64 sums 1.4 ms; 10 000 shapelets x 1 000 series: 1.27 s -> 87 ms
 // (with the shapelet values read through L1 instead of staged in shared memory
 // the filter takes 4.8 ms).
