@@ -797,8 +797,10 @@ __device__ __forceinline__ bool second_pass_comes(const GuidedArgs &A) {
            (unsigned long long)A.tail_cap;
 }
 
-// `large`: the lane ends without a value, count = -1, once second_pass_comes.
-template <int KIND, int S>
+// WATCH: a lane that is `large` ends without a value, count = -1, once
+// second_pass_comes.  (Its own form: the test in the loop takes the others 0.7 % of the
+// kernel's time.)
+template <int KIND, int S, bool WATCH>
 __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__restrict__ X,
                                            const double *__restrict__ Y, int &count, int row0,
                                            int64_t gt, Stage<S> &St, bool large) {
@@ -837,12 +839,13 @@ __device__ __forceinline__ double evaluate(const GuidedArgs &A, const double *__
     // the next word, loaded while the current one is worked on
     uint4 next = left > 0 ? list[left - 1] : make_uint4(0u, 0u, 0u, 0u);
     while (__any_sync(0xffffffffu, todo != 0 || left > 0)) {
-        if (large && todo == 0 && (left & 15) == 15 && second_pass_comes(A)) {
-            left = 0;
-            count = -1;
-        }
         if (todo == 0 && left > 0) {
             left--;
+            if (WATCH && large && (left & 15) == 15 && second_pass_comes(A)) {
+                left = 0;
+                count = -1;
+                continue;
+            }
             const uint4 E = next;
             if (left > 0) next = list[left - 1];
             const int w = W64 - 1 - left % W64;
@@ -961,7 +964,11 @@ guided_pairs_kernel(const GuidedArgs A) {
 
     for (;;) {
         unsigned long long t64 = 0;
-        if (lane == 0) t64 = atomicAdd(&A.prep->queue, 1ull);
+        bool give_up = false;
+        if (lane == 0) {
+            t64 = atomicAdd(&A.prep->queue, 1ull);
+            give_up = ties_everywhere(A);
+        }
         const int64_t t = (int64_t)__shfl_sync(FULL, t64, 0);
         if (t >= ntiles) break;
         int64_t cs = t / chunks;
@@ -999,7 +1006,7 @@ guided_pairs_kernel(const GuidedArgs A) {
             if ((int64_t)at < A.left_cap)
                 A.left[at] = J.mode == PM_PAIRED ? rs : rs + J.rows.count * cs;
         };
-        if (__any_sync(FULL, lane == 0 && ties_everywhere(A))) {
+        if (__any_sync(FULL, give_up)) {
             leave(active);
             if (lane == 0) {
                 atomicAdd(&A.prep->heavy, 32ull);
@@ -1069,9 +1076,11 @@ guided_pairs_kernel(const GuidedArgs A) {
 
         double value = 0.0;
         if (large && second_pass_comes(A)) count = -1;
-        if (__any_sync(FULL, count > 0))
-            value = evaluate<KIND, S>(A, A.xd + rs * A.xs + 3, A.yd + cs * A.ys, count, row0, gt,
-                                      stage, large);
+        const double *X = A.xd + rs * A.xs + 3, *Y = A.yd + cs * A.ys;
+        if (__any_sync(FULL, large && count > 0))
+            value = evaluate<KIND, S, true>(A, X, Y, count, row0, gt, stage, large);
+        else if (__any_sync(FULL, count > 0))
+            value = evaluate<KIND, S, false>(A, X, Y, count, row0, gt, stage, false);
         if (active && count > 0) store(sqrt(value));
         leave(active && count <= 0);
     }
